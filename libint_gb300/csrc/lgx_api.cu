@@ -188,7 +188,7 @@ struct lgx_context {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
   std::string err;
-  DBuf boys, boys_tay, boys32, sph_off, sph_c, sph_cd, sph_cf, Df, inv_odd;
+  DBuf boys, boys_tay, boys32, boys_split, sph_off, sph_c, sph_cd, sph_cf, Df, inv_odd;
   std::map<int, std::unique_ptr<ProgDev>> progs;
   bool use_rk = true;  // register kernels for the small classes
   bool use_post = true;  // generated post stages for the large J/K classes
@@ -684,6 +684,7 @@ void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
   a.boys = ctx->boys.as<double>();
   a.boys_tay = ctx->boys_tay.as<double>();
   a.boys32 = ctx->boys32.as<float>();
+  a.boys_split = ctx->boys_split.as<float>();
   a.inv_odd = ctx->inv_odd.as<double>();
   a.sph_off = ctx->sph_off.as<int>();
   a.sph_c = ctx->sph_c.as<int>();
@@ -1281,14 +1282,12 @@ lgx_status build_bins(lgx_context* ctx, BasisDev& B, double thresh, int mode, do
 //   W - P, W - Q (eta / (zeta + eta), zeta / (zeta + eta), 6 products) 8
 //   P - A, Q - C                                                      6
 //   1/2zeta, 1/2eta, 1/2(zeta + eta), rho/zeta, rho/eta               5
-// = 50 + 4 mmax.  The mixed scheme's FP32 kernels with the Boys function in
-// FP64 form rho, P - Q, T and F_m(T) again in FP64 (27 + 3 mmax on the FP64
-// pipe) besides the FP32 quantities the VRR uses; prologue_flops64 is that
-// FP64 share.
+// = 50 + 4 mmax.  The mixed scheme's FP32 kernels form rho, P - Q and T a
+// second time (13), in double-float arithmetic counted as one operation each;
+// they have no FP64 share.
 double prologue_flops(int mmax, bool b64) {
   return 50.0 + 4.0 * mmax + (b64 ? 13.0 : 0.0);
 }
-double prologue_flops64(int mmax, bool b64) { return b64 ? 27.0 + 3.0 * mmax : 0.0; }
 
 // FP operations of the Cartesian -> solid-harmonic transform of one set.
 double sph_flops(int la, int lb, int lc, int ld, const int* pure) {
@@ -1592,14 +1591,13 @@ lgx_status finish_bins(lgx_context* ctx, BasisDev& B, int deriv, bool allow_fp32
     const int lq[4] = {bin.la, bin.lb, bin.lc, bin.ld};
     for (int k = 0; k < 4; ++k) nsph *= pure[k] ? 2 * lq[k] + 1 : ncart(lq[k]);
     // VRR + post stage + transform, then the prologue and the digestion,
-    // which run in the launch's precision too (the FP64 Boys share of the
-    // mixed scheme's FP32 kernels on the FP64 pipe)
+    // which run in the launch's precision too
     const bool b64 = mode_b64(r.mode);
     const double flops =
         double(np) * (double(P->host.vrr_flops) + prologue_flops(P->host.mmax, b64)) +
         q * (double(P->host.post_flops) + nsets * sph_flops(bin.la, bin.lb, bin.lc, bin.ld, pure) +
              nsets * 12.0 * nsph);
-    const double flops_on64 = r.fp32 ? double(np) * prologue_flops64(P->host.mmax, b64) : flops;
+    const double flops_on64 = r.fp32 ? 0.0 : flops;
     f64 += flops_on64;
     f32 += flops - flops_on64;
     lgx_launch_stats ls{};
@@ -2127,6 +2125,30 @@ lgx_status lgx_create(lgx_context** out, int device) {
     std::vector<float> boysf(boys.begin(), boys.end());
     CK(c->boys32.ensure(boysf.size() * sizeof(float)));
     CK(cudaMemcpy(c->boys32.p, boysf.data(), boysf.size() * sizeof(float), cudaMemcpyHostToDevice));
+    {
+      // split FP32 tables: packed rows per mmax, then the general rows
+      std::vector<float> sp(kBoysSplitSize, 0.0f);
+      auto hi = [&](int k, int m) { return float(boys[size_t(k) * kBoysCols + m]); };
+      auto lo = [&](int k, int m) {
+        const double f = boys[size_t(k) * kBoysCols + m];
+        return float(f - double(float(f)));
+      };
+      for (int k = 0; k < kBoysRows; ++k) {
+        for (int M = 0; M <= kBoysSplitM; ++M) {
+          float* row = &sp[boys_split_off(M) + size_t(k) * boys_split_cols(M)];
+          for (int m = 0; m <= M + 4; ++m) row[m] = hi(k, m);
+          for (int m = 0; m <= M; ++m) row[M + 5 + m] = lo(k, m);
+        }
+        float* row = &sp[kBoysGenOff + size_t(k) * kBoysGenCols];
+        for (int m = 0; m < kBoysGenCols / 2; ++m) {
+          row[2 * m] = hi(k, m);
+          row[2 * m + 1] = lo(k, m);
+        }
+      }
+      CK(c->boys_split.ensure(sp.size() * sizeof(float)));
+      CK(cudaMemcpy(c->boys_split.p, sp.data(), sp.size() * sizeof(float),
+                    cudaMemcpyHostToDevice));
+    }
     if (const char* e = getenv("LGX_DISABLE_RK")) c->use_rk = (e[0] == '0');
     if (const char* e = getenv("LGX_DISABLE_POST")) c->use_post = (e[0] == '0');
     if (const char* e = getenv("LGX_TUNE")) c->tune = (e[0] != '0');

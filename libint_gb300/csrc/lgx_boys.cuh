@@ -93,7 +93,7 @@ __device__ __forceinline__ void rk_boys(const double* __restrict__ tay, double T
   rk_boys_core<MMAX>(tay, T, T > kBoysTmax, k, md, pfac, F);
 }
 
-// The mixed scheme's FP64 Boys function of an FP32 quartet, given its
+// The mixed scheme's FP64 Boys function of an FP32 quartet (store kernels), given its
 // argument T = T.hi + T.lo in double-float (ds_boys_arg): the branch and the
 // grid point come from T.hi; the offset md = T_k - T = (T_k - T.hi) - T.lo,
 // where T_k - T.hi is exact in FP32 (T_k = k/64 and T.hi are within a
@@ -116,6 +116,62 @@ __device__ __forceinline__ void rk_boys_b64(const double* __restrict__ tay, dsf 
   }
   const double T64 = f2d_int(T.hi) + f2d_int(T.lo);
   rk_boys_core<MMAX, false, 4, true>(tay, T64, asym, k, md, 1.0, F);
+}
+
+// The Boys function of the mixed scheme's J/K kernels times the FP32
+// prefactor, F_m(T) pfac for T = T.hi + T.lo in double-float (ds_boys_arg),
+// with no FP64 instruction: every value is a leading FP32 part plus an FP32
+// correction, rounded once in the product by pfac.
+//  T <= 50: F_m(T) = hi_m + [lo_m + md F_{m+1} + md^2/2 (F_{m+2} + md/3
+//   (F_{m+3} + md/4 F_{m+4}))] of the split table, for every m directly; md = T_k - T =
+//   (T_k - T.hi) - T.lo, whose first difference is exact (Sterbenz) and whose
+//   two parts multiply F_{m+1} one by one: with |md| <= 1/128 the bracket is
+//   right to 2^-31 of F_m, 1/128 of the FP32 half-ulp; the series stops at
+//   2.5e-13.
+//  T > 50: r = T^{-1/2} and u = 1/(2T) as hi + lo (boys_asym), F_0 =
+//   sqrt(pi)/2 r, F_{m+1} = (2m+1) u F_m without the e^{-T} terms.
+// The store kernels keep rk_boys_b64: they hand out the integrals one by one,
+// and this evaluation, although as close to the exact values, rounds about
+// one F_m in a thousand (and every product by pfac) the other way.
+// What bounds it: the gathers (2 LDG.128 for m <= 1, 5 for m = 6) and FP32
+// issue, about 7 instructions per m; evaluated on the FP64 pipe (2 lanes per
+// cycle and SM) the same values made that pipe the bound of these kernels
+// ((H2O)32 cc-pVDZ mixed pass 218 ms, with this 163 ms).
+template <int MMAX>
+__device__ __forceinline__ void rk_boys_split(const float* __restrict__ tab, dsf T, float pfac,
+                                              float* F) {
+  static_assert(MMAX <= kBoysSplitM, "packed split tables end at kBoysSplitM");
+  if (T.hi > float(kBoysTmax)) {
+    const BoysAsym b = boys_asym(T);
+    dsf f = boys_asym_first(b.r);
+#pragma unroll
+    for (int m = 0; m <= MMAX; ++m) {
+      F[m] = boys_asym_out(f, pfac);
+      if (m < MMAX) f = boys_asym_step(f, b.u, float(2 * m + 1));
+    }
+    return;
+  }
+  constexpr int kCols = boys_split_cols(MMAX);
+  const int k = __float2int_rn(T.hi * float(kBoysInvDT));
+  const float dh = __fadd_rn(__fmul_rn(float(k), float(kBoysDT)), -T.hi);
+  const float md = __fadd_rn(dh, -T.lo);
+  const float4* row = reinterpret_cast<const float4*>(tab + boys_split_off(MMAX) + k * kCols);
+  float w[kCols];
+#pragma unroll
+  for (int i = 0; i < kCols / 4; ++i) {
+    const float4 v = __ldg(row + i);
+    w[4 * i] = v.x;
+    w[4 * i + 1] = v.y;
+    w[4 * i + 2] = v.z;
+    w[4 * i + 3] = v.w;
+  }
+  const float m2 = 0.5f * md * md, m3 = md * (1.0f / 3.0f), m4 = 0.25f * md;
+#pragma unroll
+  for (int m = 0; m <= MMAX; ++m) {
+    float c = fmaf(m2, fmaf(m3, fmaf(m4, w[m + 4], w[m + 3]), w[m + 2]), w[MMAX + 5 + m]);
+    c = fmaf(dh, w[m + 1], fmaf(-T.lo, w[m + 1], c));
+    F[m] = fmaf(w[m], pfac, c * pfac);
+  }
 }
 
 template <int MMAX>

@@ -30,6 +30,25 @@ constexpr int kBoysRows = int(kBoysTmax * 64.0) + 2;  // 3202 grid points
 // entry 7 of the m = 0 row holds e^{-T_k}.
 constexpr int kBoysTaylorStride = 8;
 
+// Split FP32 tables of the mixed scheme's J/K kernels: the grid values
+// F_m(T_k) as hi = float(F), lo = float(F - hi).
+//  packed, one per mmax <= kBoysSplitM (the register kernels' compile-time
+//   mmax): a row holds hi of m = 0..mmax+4, then lo of m = 0..mmax, padded to
+//   whole float4; 32 B for mmax <= 1 (100 KB for the whole grid, so a launch's
+//   table stays in L1), 80 B for mmax = 6;
+//  general (the program kernels' run-time mmax): hi, lo interleaved,
+//   m = 0..kBoysMaxM+4.
+constexpr int kBoysSplitM = 6;
+__host__ __device__ constexpr int boys_split_cols(int mmax) { return (2 * mmax + 9) & ~3; }
+__host__ __device__ constexpr int boys_split_off(int mmax) {
+  int o = 0;
+  for (int m = 0; m < mmax; ++m) o += kBoysRows * boys_split_cols(m);
+  return o;
+}
+constexpr int kBoysGenCols = 2 * (kBoysMaxM + 5);
+constexpr int kBoysGenOff = boys_split_off(kBoysSplitM + 1);
+constexpr int kBoysSplitSize = kBoysGenOff + kBoysRows * kBoysGenCols;
+
 // ------------------------------------------------------------ basis data
 struct DevBasis {
   int nshell;
@@ -187,6 +206,50 @@ __device__ __forceinline__ dsf ds_boys_arg(const float4& bh, const float4& bl, c
   const dsf dy = ds_sub({bh.y, bl.y}, {kh.y, kl.y});
   const dsf dz = ds_sub({bh.z, bl.z}, {kh.z, kl.z});
   return ds_mul(rho, ds_add(ds_add(ds_sqr(dx), ds_sqr(dy)), ds_sqr(dz)));
+}
+
+// T^{-1/2} and 1/(2T) of a double-float T (normal, positive) as hi + lo, from
+// the FP32 estimate r0: e = 1 - T r0^2 (|e| <= ~3e-7) is formed exactly enough
+// by three FMAs on the rounded product q = T.hi r0, and r = r0 + r0 e/2 leaves
+// 3/8 e^2 <= 4e-14.
+struct BoysAsym {
+  dsf r, u;
+};
+__device__ __forceinline__ BoysAsym boys_asym(dsf T) {
+  BoysAsym b;
+  const float r0 = rsqrtf(T.hi);
+  const float q = __fmul_rn(T.hi, r0);
+  float e = fmaf(-q, r0, 1.0f);
+  e = fmaf(-fmaf(T.hi, r0, -q), r0, e);
+  e = fmaf(-__fmul_rn(T.lo, r0), r0, e);
+  b.r.hi = r0;
+  b.r.lo = 0.5f * r0 * e;
+  const float rr = __fmul_rn(r0, r0);
+  b.u.hi = 0.5f * rr;
+  b.u.lo = fmaf(r0, b.r.lo, 0.5f * fmaf(r0, r0, -rr));
+  return b;
+}
+// x (2m + 1) u, unnormalised (|lo| stays a few ulp of hi over <= 16 steps).
+__device__ __forceinline__ dsf boys_asym_step(dsf x, dsf u, float odd) {
+  const float c = __fmul_rn(odd, u.hi);
+  const float cl = fmaf(odd, u.lo, fmaf(odd, u.hi, -c));
+  const float p = __fmul_rn(x.hi, c);
+  return {p, fmaf(x.hi, cl, fmaf(x.lo, c, fmaf(x.hi, c, -p)))};
+}
+// sqrt(pi)/2 2^60 r: the upward recursion runs scaled by 2^60, so that the lo
+// parts of the smallest normal values stay normal.
+constexpr float kBoysScale = 1152921504606846976.0f;
+__device__ __forceinline__ dsf boys_asym_first(dsf r) {
+  constexpr double c = 0.88622692545275801365 * double(kBoysScale);
+  constexpr float ch = float(c), cl = float(c - double(ch));
+  const float h = __fmul_rn(ch, r.hi);
+  return {h, fmaf(ch, r.lo, fmaf(cl, r.hi, fmaf(ch, r.hi, -h)))};
+}
+// The recursion's value times pfac without the scale; zero when subnormal.
+__device__ __forceinline__ float boys_asym_out(dsf f, float pfac) {
+  float r;
+  asm("mul.ftz.f32 %0, %1, 0f21800000;" : "=f"(r) : "f"(fmaf(f.hi, pfac, f.lo * pfac)));
+  return r;
 }
 
 // A shell pair with its primitive-pair range (pair list, shell.h:1079-1329).

@@ -10,10 +10,10 @@ enum KernelMode : int {
   kModeSchwarz = 1,  // K(pair) = sqrt(max |(ab|ab)|)
   kModeJK = 2,       // digest into J/K accumulators (deriv 0)
   kModeGrad = 3,     // digest first derivatives into gJ/gK (deriv 1)
-  // FP32 kernels of the mixed scheme with the Boys function in FP64: the
-  // argument T = rho |P - Q|^2, F_m(T) (Taylor / asymptotic branch, e^{-T}
-  // and the downward recursion) in FP64 from the FP64 pair data, then the
-  // VRR / HRR / contraction in FP32; otherwise as kModeJK / kModeStore
+  // FP32 kernels of the mixed scheme: the Boys argument T = rho |P - Q|^2 in
+  // double-float arithmetic and F_m(T) to FP32 rounding (J/K: split FP32
+  // tables; store: FP64 evaluation), then the VRR / HRR / contraction in
+  // FP32; otherwise as kModeJK / kModeStore
   kModeJKB64 = 4,
   kModeStoreB64 = 5
 };
@@ -23,6 +23,10 @@ __host__ __device__ constexpr bool mode_store(int m) {
 }
 __host__ __device__ constexpr bool mode_b64(int m) {
   return m == kModeJKB64 || m == kModeStoreB64;
+}
+// Boys evaluator of an FP32 kernel: 0 FP32, 1 FP64 rounded, 2 split tables.
+__host__ __device__ constexpr int mode_boys(int m) {
+  return m == kModeJKB64 ? 2 : (m == kModeStoreB64 ? 1 : 0);
 }
 
 // Explicit work item: one shell quartet in canonical orientation.
@@ -107,6 +111,7 @@ struct EriArgs {
   const double* boys;     // [kBoysRows][kBoysCols] F_m(T_k)
   const double* boys_tay; // pre-divided Taylor table (kBoysTaylorStride)
   const float* boys32;    // FP32 copy of the Boys table
+  const float* boys_split;  // split FP32 tables (boys_split_off, kBoysGenOff)
   const double* inv_odd;  // 1/(2m+1), m < 40
   // Cartesian -> solid harmonics, sparse: nonzeros of row (l, p) are
   // [sph_off[l*9+p], sph_off[l*9+p+1]) with Cartesian index sph_c[] and

@@ -215,17 +215,19 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<float>
   return true;
 }
 
-// One primitive quartet into acc (FP32 VRR) with the Boys function in FP64
-// (the kModeJKB64 / kModeStoreB64 kernels of the mixed scheme).  The
-// screening, prefactor and VRR geometry are the FP32 ones of rk_prim above;
-// the Boys argument T = rho |P - Q|^2 is formed in double-float arithmetic
-// from the bins' double-float records bds / kds, or for explicit quartet
-// lists (null bds / kds) from those of the primitive pairs bidx / kidx
-// (ds_boys_arg: FP32 operations, relative error ~1e-13); F_m(T) comes from
-// the FP64 evaluator (Taylor with the
-// downward recursion and e^{-T}, or the asymptotic branch, rk_boys_b64) and
-// is rounded to FP32 with integer operations before the FP32 pfac.
-template <class C>
+// One primitive quartet into acc (FP32 VRR) with the Boys function to full
+// FP32 accuracy (the kModeJKB64 / kModeStoreB64 kernels of the mixed
+// scheme).  The screening, prefactor and VRR geometry are the FP32 ones of
+// rk_prim above; the Boys argument T = rho |P - Q|^2 is formed in
+// double-float arithmetic from the bins' double-float records bds / kds, or
+// for explicit quartet lists (null bds / kds) from those of the primitive
+// pairs bidx / kidx (ds_boys_arg: FP32 operations, relative error ~1e-13).
+// BOYS 2 (J/K): F_m(T) from the split tables (rk_boys_split), no FP64
+// instruction; evaluated in FP64 that pipe was 65% busy and bound the s/p
+// classes ((H2O)32 cc-pVDZ mixed pass 218 -> 163 ms, (H2O)20 cc-pVTZ 828 ->
+// 746 ms).  BOYS 1 (store): the FP64 evaluator, rounded to FP32 with integer
+// operations before the FP32 pfac.
+template <class C, int BOYS>
 __device__ __forceinline__ bool rk_prim_b64(const EriArgs& a, const RkQuartet<float>& q,
                                             const PrimF32& bp, const PrimF32& kp,
                                             const PrimPairJKds* bds, const PrimPairJKds* kds,
@@ -249,11 +251,15 @@ __device__ __forceinline__ bool rk_prim_b64(const EriArgs& a, const RkQuartet<fl
   }
   const dsf T =
       ds_boys_arg(__ldg(&bds->hi), __ldg(&bds->lo), __ldg(&kds->hi), __ldg(&kds->lo), rho, oogpq);
-  double F64[C::kMmax + 1];
-  rk_boys_b64<C::kMmax>(a.boys_tay, T, F64);
   float F[C::kMmax + 1];
+  if constexpr (BOYS == 2) {
+    rk_boys_split<C::kMmax>(a.boys_split, T, pfac, F);
+  } else {
+    double F64[C::kMmax + 1];
+    rk_boys_b64<C::kMmax>(a.boys_tay, T, F64);
 #pragma unroll
-  for (int m = 0; m <= C::kMmax; ++m) F[m] = d2f_int(F64[m]) * pfac;
+    for (int m = 0; m <= C::kMmax; ++m) F[m] = d2f_int(F64[m]) * pfac;
+  }
   rk::Geo<float> g;
   const float ez = eta * oogpq, zz = zeta * oogpq;
   g.PAx = PA[0]; g.PAy = PA[1]; g.PAz = PA[2];
@@ -381,7 +387,7 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
         if constexpr (mode_b64(MODE)) {
           const PrimPairJKds* bds = rec ? a.jkds + brec.x + ib * brec.y : nullptr;
           const PrimPairJKds* kds = rec ? a.jkds + krec.x + ik * krec.y : nullptr;
-          kept += rk_prim_b64<C>(a, q, bp, kp, bds, kds, q.bra_pp + ib, q.ket_pp + ik, scr, acc)
+          kept += rk_prim_b64<C, mode_boys(MODE)>(a, q, bp, kp, bds, kds, q.bra_pp + ib, q.ket_pp + ik, scr, acc)
                       ? 1
                       : 0;
         } else {

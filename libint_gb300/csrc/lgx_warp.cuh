@@ -138,6 +138,39 @@ __device__ __forceinline__ void boys_b64_stage(const double* __restrict__ tay,
   }
 }
 
+// The same for the J/K program kernels (runtime mmax <= kBoysMaxM): rk_boys_split's evaluation from the general
+// split table, and beyond T = 50 with the e^{-T} terms of the upward
+// recursion (they reach ~3e-8 of F_16 at T = 50).
+__device__ __forceinline__ void boys_split_stage(const float* __restrict__ tab, dsf T, int mmax,
+                                                 float pfac, float* __restrict__ F) {
+  if (T.hi > float(kBoysTmax)) {
+    const BoysAsym b = boys_asym(T);
+    const float eu = __expf(-T.hi) * kBoysScale * b.u.hi;
+    dsf f = boys_asym_first(b.r);
+    for (int m = 0; m <= mmax; ++m) {
+      F[m] = boys_asym_out(f, pfac);
+      f = boys_asym_step(f, b.u, float(2 * m + 1));
+      f.lo -= eu;
+    }
+    return;
+  }
+  const int k = __float2int_rn(T.hi * float(kBoysInvDT));
+  const float dh = __fadd_rn(__fmul_rn(float(k), float(kBoysDT)), -T.hi);
+  const float md = __fadd_rn(dh, -T.lo);
+  const float2* row = reinterpret_cast<const float2*>(tab + kBoysGenOff + k * kBoysGenCols);
+  const float m2 = 0.5f * md * md, m3 = md * (1.0f / 3.0f), m4 = 0.25f * md;
+  float2 f0 = __ldg(row), f1 = __ldg(row + 1), f2 = __ldg(row + 2), f3 = __ldg(row + 3);
+  for (int m = 0; m <= mmax; ++m) {
+    const float2 f4 = __ldg(row + m + 4);
+    const float c = fmaf(m2, fmaf(m3, fmaf(m4, f4.x, f3.x), f2.x), f0.y);
+    F[m] = fmaf(f0.x, pfac, fmaf(dh, f1.x, fmaf(-T.lo, f1.x, c)) * pfac);
+    f0 = f1;
+    f1 = f2;
+    f2 = f3;
+    f3 = f4;
+  }
+}
+
 // FP32 Boys (4-term Taylor on the same grid, FP32 recursion).
 __device__ __forceinline__ void boys_to_stage(const float* __restrict__ tab, float T, int mmax,
                                               float pfac, float* __restrict__ F) {
@@ -276,7 +309,7 @@ __device__ __forceinline__ T sel3(int d, T x, T y, T z) {
 // of T).  Returns false if screened out.
 // ATT: instantiation for the attenuated operators (a.op = erf / erfc); the
 // Coulomb instantiations carry none of that code.
-template <bool ATT, bool B64 = false>
+template <bool ATT, int B64 = 0>
 __device__ __forceinline__ bool prologue(const EriArgs& a, const QuartetGeom<double>& g, int idx,
                                          double npbraket, double* st) {
   const int ib = idx / g.nkpp, ik = idx - ib * g.nkpp;
@@ -324,12 +357,12 @@ __device__ __forceinline__ bool prologue(const EriArgs& a, const QuartetGeom<dou
   return true;
 }
 
-// B64: the mixed scheme's Boys function in FP64 (kModeJKB64 /
-// kModeStoreB64): T = rho |P - Q|^2 in double-float arithmetic from the
-// primitive pairs' double-float records (ds_boys_arg, relative error
-// ~1e-13) and F_m(T) from the FP64 evaluator (boys_b64_stage), rounded to
-// FP32.
-template <bool ATT, bool B64 = false>
+// B64: the mixed scheme's Boys function: T = rho |P - Q|^2 in double-float
+// arithmetic from the primitive pairs' double-float records (ds_boys_arg,
+// relative error ~1e-13) and F_m(T) rounded to FP32, for kModeStoreB64 (1)
+// from the FP64 evaluator (boys_b64_stage), for kModeJKB64 (2) from the split
+// tables (boys_split_stage).
+template <bool ATT, int B64 = 0>
 __device__ __forceinline__ bool prologue(const EriArgs& a, const QuartetGeom<float>& g, int idx,
                                          double npbraket, float* st) {
   const int ib = idx / g.nkpp, ik = idx - ib * g.nkpp;
@@ -351,12 +384,15 @@ __device__ __forceinline__ bool prologue(const EriArgs& a, const QuartetGeom<flo
               PQz = PA[2] - QC[2] + g.AC[2];
   const float rho = zeta * eta * oogpq;
   const float T = rho * fmaf(PQx, PQx, fmaf(PQy, PQy, PQz * PQz));
-  if constexpr (B64) {
+  if constexpr (B64 != 0) {
     const PrimPairJKds* bd = a.ppds + g.bra_pp + ib;
     const PrimPairJKds* kd = a.ppds + g.ket_pp + ik;
-    const dsf T64 = ds_boys_arg(__ldg(&bd->hi), __ldg(&bd->lo), __ldg(&kd->hi), __ldg(&kd->lo),
+    const dsf Td = ds_boys_arg(__ldg(&bd->hi), __ldg(&bd->lo), __ldg(&kd->hi), __ldg(&kd->lo),
                                 rho, oogpq);
-    boys_b64_stage(a.boys_tay, a.inv_odd, T64, a.prog.mmax, pfac, st + kStF);
+    if constexpr (B64 == 2)
+      boys_split_stage(a.boys_split, Td, a.prog.mmax, pfac, st + kStF);
+    else
+      boys_b64_stage(a.boys_tay, a.inv_odd, Td, a.prog.mmax, pfac, st + kStF);
   } else if constexpr (ATT) {
     if (a.op != 1) boys_to_stage(a.boys32, T, a.prog.mmax, pfac, st + kStF);
     attenuate<float>(a, T, rho, a.prog.mmax, pfac, st + kStF);
@@ -514,7 +550,7 @@ __device__ __forceinline__ void vrr_consume(const DevProg& P, const T* __restric
 
 // Steps 1-2: contracted (e0|f0) accumulators in slots[0, nacc).  Returns the
 // number of primitive quartets that survived screening.
-template <typename T, bool ATT = false, bool B64 = false>
+template <typename T, bool ATT = false, int B64 = 0>
 __device__ int contract_quartet(const EriArgs& a, const QuartetGeom<T>& g, T* __restrict__ slots,
                                 T* __restrict__ stage, int lane) {
   const DevProg& P = a.prog;
@@ -867,7 +903,7 @@ __global__ void __launch_bounds__(128) eri_warp_kernel(EriArgs a) {
       load_geom<T>(a, bpair, kpair, flags & 1, (flags >> 1) & 1, g);
       if (mode_jk(MODE) && !quartet_screen(a, g.sh, bpair, kpair, g.scr)) continue;
       const int kept =
-          contract_quartet<T, PostAtten<Post>::value, mode_b64(MODE)>(a, g, slots, stage, lane);
+          contract_quartet<T, PostAtten<Post>::value, mode_boys(MODE)>(a, g, slots, stage, lane);
       my_prims += kept;
       if (mode_store(MODE) && a.is_null && lane == 0) a.is_null[orig] = kept == 0 ? 1 : 0;
       if (kept == 0) {
