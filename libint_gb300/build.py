@@ -34,9 +34,10 @@ def _generate() -> list:
     their content changes); returns the generated CUDA units (csrc/gen)."""
     sys.path.insert(0, os.path.join(PKG_DIR, "codegen"))
     try:
-        import gen_rk
+        import gen_grad
         import gen_post
-        units = gen_rk.main() + gen_post.main()
+        import gen_rk
+        units = gen_rk.main() + gen_post.main() + gen_grad.main()
     finally:
         sys.path.pop(0)
     return [os.path.join("gen", u) for u in units]

@@ -1,0 +1,14 @@
+// GENERATED by libint_gb300/codegen/gen_grad.py -- do not edit.
+#include "../lgx_rkgrad.cuh"
+
+namespace lgx {
+cudaError_t rk_grad_launch_1022(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<1, 0, 2, 2>(a, work, nsm, st);
+}
+cudaError_t rk_grad_launch_1021(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<1, 0, 2, 1>(a, work, nsm, st);
+}
+cudaError_t rk_grad_launch_1011(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<1, 0, 1, 1>(a, work, nsm, st);
+}
+}  // namespace lgx

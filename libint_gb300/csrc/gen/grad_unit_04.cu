@@ -1,0 +1,14 @@
+// GENERATED by libint_gb300/codegen/gen_grad.py -- do not edit.
+#include "../lgx_rkgrad.cuh"
+
+namespace lgx {
+cudaError_t rk_grad_launch_1130(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<1, 1, 3, 0>(a, work, nsm, st);
+}
+cudaError_t rk_grad_launch_1120(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<1, 1, 2, 0>(a, work, nsm, st);
+}
+cudaError_t rk_grad_launch_0020(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<0, 0, 2, 0>(a, work, nsm, st);
+}
+}  // namespace lgx

@@ -1,0 +1,14 @@
+// GENERATED by libint_gb300/codegen/gen_grad.py -- do not edit.
+#include "../lgx_rkgrad.cuh"
+
+namespace lgx {
+cudaError_t rk_grad_launch_2030(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<2, 0, 3, 0>(a, work, nsm, st);
+}
+cudaError_t rk_grad_launch_2020(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<2, 0, 2, 0>(a, work, nsm, st);
+}
+cudaError_t rk_grad_launch_0010(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<0, 0, 1, 0>(a, work, nsm, st);
+}
+}  // namespace lgx

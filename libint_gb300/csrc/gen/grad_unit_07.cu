@@ -1,0 +1,14 @@
+// GENERATED by libint_gb300/codegen/gen_grad.py -- do not edit.
+#include "../lgx_rkgrad.cuh"
+
+namespace lgx {
+cudaError_t rk_grad_launch_0022(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<0, 0, 2, 2>(a, work, nsm, st);
+}
+cudaError_t rk_grad_launch_0021(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<0, 0, 2, 1>(a, work, nsm, st);
+}
+cudaError_t rk_grad_launch_0000(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<0, 0, 0, 0>(a, work, nsm, st);
+}
+}  // namespace lgx

@@ -41,6 +41,11 @@ cudaError_t launch_eri_block_store(const EriArgs& a, int grid, size_t smem, cuda
 cudaError_t rk_launch(bool fp32, int mode, bool att, int la, int lb, int lc, int ld, const EriArgs& a,
                       long long work, int nsm, cudaStream_t st);
 bool rk_available(bool fp32, int mode, bool att, int la, int lb, int lc, int ld);
+cudaError_t rk_grad_launch(int la, int lb, int lc, int ld, const EriArgs& a, long long work,
+                           int nsm, cudaStream_t st);
+bool rk_grad_available(int la, int lb, int lc, int ld);
+cudaError_t launch_grad_sum(const double* copies, int ncopies, long long stride, int n, double* g,
+                            cudaStream_t st);
 cudaError_t launch_jk_records(const PrimPairRec* pp, const int* src, long long n,
                               PrimPairJK32* out, PrimPairJKds* outds, cudaStream_t st);
 cudaError_t post_launch(bool fp32, int mode, int la, int lb, int lc, int ld, const EriArgs& a,
@@ -255,7 +260,7 @@ struct lgx_context {
   BasisDev basis, small;
   DBuf gscratch, counter, errflag, primcount;
   DBuf items, out, isnull;
-  DBuf Jacc, Kacc, Dd, Jd, Kd, gJ, gK;
+  DBuf Jacc, Kacc, Dd, Jd, Kd, gsum, gcopies;  // gradients: sum and per-SM copies
   DBuf prim_rows, prim_slots;  // lgx_compute_primitive_set
   DBuf boysT, boysF;           // lgx_boys
   DBuf xcounters;              // explicit lists: one work counter per class launch
@@ -699,8 +704,11 @@ void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
 
 bool rk_eligible(const lgx_context* ctx, const BasisDev& B, const ProgDev& P, int mode,
                  bool fp32) {
-  if (!ctx->use_rk || !B.std_pure || P.host.deriv != 0) return false;
+  if (!ctx->use_rk || !B.std_pure) return false;
   const bool att = ctx->op != LGX_OP_COULOMB;  // attenuated: J/K register kernels only
+  if (mode == kModeGrad)
+    return !att && rk_grad_available(P.host.la, P.host.lb, P.host.lc, P.host.ld);
+  if (P.host.deriv != 0) return false;
   return rk_available(fp32, mode, att, P.host.la, P.host.lb, P.host.lc, P.host.ld);
 }
 
@@ -734,6 +742,11 @@ lgx_status run_rk(lgx_context* ctx, BasisDev& B, const ProgDev& P, int mode, boo
                   EriArgs a, long long nwork, int group) {
   fill_common(ctx, B, a);
   a.group = group;
+  if (mode == kModeGrad) {
+    CK(rk_grad_launch(P.host.la, P.host.lb, P.host.lc, P.host.ld, a, nwork, ctx->nsm,
+                      ctx->launch_stream ? ctx->launch_stream : ctx->stream));
+    return LGX_OK;
+  }
   CK(rk_launch(fp32, mode, a.op != LGX_OP_COULOMB, P.host.la, P.host.lb, P.host.lc, P.host.ld, a,
                nwork, ctx->nsm,
                ctx->launch_stream ? ctx->launch_stream : ctx->stream));
@@ -1386,6 +1399,7 @@ lgx_status tune_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int mod
       } else {
         a.gJ = ctx->tuneJ.as<double>();
         a.gK = ctx->tuneK.as<double>();
+        a.gcopies = 1;
       }
       float best = 0;
       Variant bestv = d;
@@ -2843,26 +2857,34 @@ lgx_status lgx_jk_grad(lgx_context* ctx, const double* D, double* gJ, double* gK
   if (s != LGX_OK) return s;
   const size_t nn = size_t(B.nbf) * B.nbf;
   CK(ctx->Dd.ensure(nn * sizeof(double)));
-  CK(ctx->gJ.ensure(3 * natoms * sizeof(double)));
-  CK(ctx->gK.ensure(3 * natoms * sizeof(double)));
+  // one copy per SM, 16 MB of copies at most
+  const long long n3 = 3LL * natoms;
+  const int ncopies =
+      int(std::max(1LL, std::min<long long>(ctx->nsm, (16LL << 20) / (2 * n3 * (long long)sizeof(double)))));
+  const size_t gbytes = size_t(2 * n3) * sizeof(double);
+  CK(ctx->gsum.ensure(gbytes));
+  CK(ctx->gcopies.ensure(gbytes * ncopies));
   CK(cudaMemcpyAsync(ctx->Dd.p, D, nn * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemsetAsync(ctx->gJ.p, 0, 3 * natoms * sizeof(double), ctx->stream));
-  CK(cudaMemsetAsync(ctx->gK.p, 0, 3 * natoms * sizeof(double), ctx->stream));
+  CK(cudaMemsetAsync(ctx->gcopies.p, 0, gbytes * ncopies, ctx->stream));
   EriArgs a{};
   a.precision = eps;
   a.ln_prec = std::log(eps);
   a.D = ctx->Dd.as<double>();
-  a.gJ = ctx->gJ.as<double>();
-  a.gK = ctx->gK.as<double>();
+  a.gJ = ctx->gcopies.as<double>();
+  a.gK = a.gJ + n3;
+  a.gcopies = ncopies;
+  a.gstride = 2 * n3;
   a.nbf = B.nbf;
   s = tune_bins(ctx, B, kModeGrad, 1, -1, a);
   if (s != LGX_OK) return s;
   s = run_bins(ctx, B, kModeGrad, 1, -1, a, stats);
   if (s != LGX_OK) return s;
-  CK(cudaMemcpyAsync(gJ, ctx->gJ.p, 3 * natoms * sizeof(double), cudaMemcpyDeviceToHost,
+  CK(launch_grad_sum(ctx->gcopies.as<double>(), ncopies, 2 * n3, int(2 * n3), ctx->gsum.as<double>(),
                      ctx->stream));
-  CK(cudaMemcpyAsync(gK, ctx->gK.p, 3 * natoms * sizeof(double), cudaMemcpyDeviceToHost,
+  CK(cudaMemcpyAsync(gJ, ctx->gsum.p, 3 * natoms * sizeof(double), cudaMemcpyDeviceToHost,
                      ctx->stream));
+  CK(cudaMemcpyAsync(gK, ctx->gsum.as<double>() + n3, 3 * natoms * sizeof(double),
+                     cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   return check_errflag(ctx);
 }

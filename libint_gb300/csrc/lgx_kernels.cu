@@ -145,6 +145,23 @@ __global__ void jk_finalize_kernel(const double* Jacc, const double* Kacc, doubl
   K[t] = 0.125 * (Kacc[(size_t)i * nbf + j] + Kacc[(size_t)j * nbf + i]);
 }
 
+// Sum of the gradient copies: g[i] = sum over c of copies[c * stride + i].
+__global__ void grad_sum_kernel(const double* copies, int ncopies, long long stride, int n,
+                                double* g) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double s = 0.0;
+  for (int c = 0; c < ncopies; ++c) s += copies[c * stride + i];
+  g[i] = s;
+}
+
+cudaError_t launch_grad_sum(const double* copies, int ncopies, long long stride, int n, double* g,
+                            cudaStream_t st) {
+  const int block = 64;
+  grad_sum_kernel<<<(n + block - 1) / block, block, 0, st>>>(copies, ncopies, stride, n, g);
+  return cudaGetLastError();
+}
+
 // ----------------------------------------------------------- launchers
 
 cudaError_t launch_eri(const EriArgs& a, int mode, bool fp32, int grid, int block, size_t smem,

@@ -151,8 +151,13 @@ struct EriArgs {
   const float* Df;     // FP32 copy of D (FP32 register kernels)
   double* Jacc;
   double* Kacc;
+  // gradients: gcopies copies of both 3 natoms arrays, gstride doubles apart;
+  // a block adds to copy blockIdx % gcopies, which keeps the atomics of the
+  // few addresses apart
   double* gJ;
   double* gK;
+  int gcopies;
+  long long gstride;
   int nbf;
   // density-weighted screening of the J/K passes (fock_prec > 0): shell-
   // block infinity norms of D (nshell x nshell), Schwarz factor per pair

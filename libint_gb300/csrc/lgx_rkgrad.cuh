@@ -1,0 +1,224 @@
+// Register-resident gradient kernel: G lanes (1, 2, ..., 32) per contracted
+// shell quartet, the primitive quartets split between them as in rk_kernel.
+// The density is applied first (gen_grad.py): once per quartet the two
+// two-particle densities become weights W over the (e0|f0) set, every
+// primitive quartet contracts its VRR values with them, and seven sums per
+// density, weighted by the exponents, give the three independent centres;
+// no derivative set is formed, transformed or digested.
+//
+// What bounds it: the FP64 pipe (2 lanes per cycle and SM).  The program
+// kernel it replaces runs a class's VRR levels across a warp's lanes, most of
+// them idle in the s/p classes, and digests nine derivative sets.  (H2O)12
+// cc-pVDZ, serial launches, before -> after: (ss|ss) 352 -> 21 ms, (ss|ps) 321
+// -> 52 ms, (ps|ps) 165 -> 30 ms, (pp|dp) 31 -> 10 ms, all classes 1417 -> 285
+// ms.  The weights of the larger classes (2 x 144 doubles for (pp|dp)) live in
+// local memory, which costs less than the FP64 work they feed.  It ends at
+// L = 5: the derivative raises the Boys order to L + 1, and rk_boys is exact
+// to m = 6; the classes above take 14 ms of the 285.
+#pragma once
+#include <algorithm>
+
+#include "gen/grad_classes.cuh"
+#include "lgx_rk.cuh"
+
+namespace lgx {
+
+// Sums of one primitive or contracted quartet for one density:
+// 2a_A V, 2a_B V, 2a_B S, 2a_D U, 2a_D S.
+constexpr int kGradSums = 11;
+
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
+  using C = rk::GradCls<LA, LB, LC, LD>;
+  constexpr int N0 = C::kN0, N1 = C::kN1, N2 = C::kN2, N3 = C::kN3;
+  constexpr int kNsph = N0 * N1 * N2 * N3;
+  // (ss|ss): both densities weight the same integrals, so one unweighted set
+  constexpr int kSets = C::kNacc == 1 ? 1 : 2;
+  const int G = a.group;
+  const int lane = threadIdx.x & 31;
+  const int g = lane & (G - 1);
+  const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
+  const int per_warp = 32 / G;
+  const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long total = a.bin.total;
+  const size_t copy = size_t(blockIdx.x % a.gcopies) * a.gstride;
+  unsigned long long my_prims = 0;
+  PrimScreen scr;
+  scr.prec = a.precision;
+  scr.ln_prec = a.ln_prec;
+  scr.fprec = a.fprecision;
+  scr.fln_prec = a.fln_prec;
+  for (long long c = warp_id; c * per_warp < total; c += nwarps) {
+    const long long c0 = c * per_warp;
+    const long long qi = c0 + (lane / G);
+    // segment of each quartet of the chunk (see rk_kernel)
+    const int seg0 = bin_segment(a.bin, c0);
+    const int kseg = seg0 + 1 + lane;
+    const long long mseg = (kseg <= a.bin.nseg ? a.bin.seg_start[kseg] : total + 64) - c0;
+    const unsigned starts = __reduce_or_sync(0xffffffffu, mseg < per_warp ? 1u << mseg : 0u);
+    const int seg = seg0 + __popc(starts & ((2u << (lane / G)) - 1u));
+    if (qi >= total) continue;
+    const int bpair = a.bin.bra_pairs[a.bin.seg_bra[seg]];
+    const int kpair = a.bin.ket_pairs[int(qi - a.bin.seg_start[seg]) + a.bin.seg_j0[seg]];
+    RkQuartet<double> q;
+    rk_load<double>(a, bpair, kpair, a.pair_swap[bpair] != 0, a.pair_swap[kpair] != 0, q);
+    const int nbf = a.nbf;
+    const size_t o0 = a.basis.bf_off[q.sh[0]], o1 = a.basis.bf_off[q.sh[1]];
+    const size_t o2 = a.basis.bf_off[q.sh[2]], o3 = a.basis.bf_off[q.sh[3]];
+    const double* D = a.D;
+    // the two-particle densities of the quartet
+    auto gamma = [&](double* GJ, double* GK) {
+#pragma unroll
+      for (int i = 0; i < N0; ++i)
+#pragma unroll
+        for (int j = 0; j < N1; ++j)
+#pragma unroll
+          for (int k = 0; k < N2; ++k)
+#pragma unroll
+            for (int l = 0; l < N3; ++l) {
+              const int e = ((i * N1 + j) * N2 + k) * N3 + l;
+              GJ[e] = __ldg(D + (o0 + i) * nbf + o1 + j) * __ldg(D + (o2 + k) * nbf + o3 + l);
+              GK[e] = 0.5 * fma(__ldg(D + (o0 + i) * nbf + o2 + k),
+                                __ldg(D + (o1 + j) * nbf + o3 + l),
+                                __ldg(D + (o0 + i) * nbf + o3 + l) *
+                                    __ldg(D + (o1 + j) * nbf + o2 + k));
+            }
+    };
+    double WJ[C::kNacc], WK[C::kNacc];
+    if constexpr (kSets == 1) {
+      WJ[0] = WK[0] = 1.0;
+    } else {
+      double GJ[kNsph], GK[kNsph];
+      gamma(GJ, GK);
+      C::template weights<double>(GJ, q.AB, q.CD, WJ);
+      C::template weights<double>(GK, q.AB, q.CD, WK);
+    }
+    double acc[kSets][kGradSums];
+#pragma unroll
+    for (int x = 0; x < kSets; ++x)
+#pragma unroll
+      for (int i = 0; i < kGradSums; ++i) acc[x][i] = 0.0;
+    double I[C::kNI];
+#pragma unroll
+    for (int i = 0; i < C::kNI; ++i) I[i] = 0.0;
+    const int nq = q.nbpp * q.nkpp;
+    int kept = 0;
+    int ib = g / q.nkpp, ik = g - ib * q.nkpp;
+    const int gb = G / q.nkpp, gk = G - gb * q.nkpp;
+    for (int p = g; p < nq; p += G) {
+      const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
+      const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
+      bool keep = ln_kept(a, bp.fln_scr + kp.fln_scr, q.bra_pp + ib, q.ket_pp + ik, scr);
+      if (keep) {
+        const double zeta = bp.zeta, eta = kp.zeta;
+        const double rs = rsqrt(zeta + eta);
+        const double pfac = bp.Kc * kp.Kc * rs;
+        keep = (__double_as_longlong(pfac) & 0x7fffffffffffffffll) >=
+               __double_as_longlong(scr.prec);
+        if (keep) {
+          const double oogpq = rs * rs;
+          const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1],
+                       PQz = bp.P[2] - kp.P[2];
+          const double ez = eta * oogpq, zz = zeta * oogpq;
+          const double T = zeta * ez * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
+          double F[C::kMmax + 1];
+          rk_boys<C::kMmax>(a.boys_tay, T, pfac, F);
+          rk::Geo<double> geo;
+          geo.PAx = bp.P[0] - q.A[0]; geo.PAy = bp.P[1] - q.A[1]; geo.PAz = bp.P[2] - q.A[2];
+          geo.QCx = kp.P[0] - q.C[0]; geo.QCy = kp.P[1] - q.C[1]; geo.QCz = kp.P[2] - q.C[2];
+          geo.WPx = -ez * PQx; geo.WPy = -ez * PQy; geo.WPz = -ez * PQz;
+          geo.WQx = zz * PQx; geo.WQy = zz * PQy; geo.WQz = zz * PQz;
+          geo.oo2z = 0.5 * bp.oog;
+          geo.roz = ez;
+          geo.oo2e = 0.5 * kp.oog;
+          geo.roe = zz;
+          geo.oo2ze = 0.5 * oogpq;
+          double s[14];
+          C::template prim<double>(F, geo, WJ, WK, s, I);
+          const double wa = 2.0 * (q.bsw ? bp.a2 : bp.a1), wb = 2.0 * (q.bsw ? bp.a1 : bp.a2);
+          const double wd = 2.0 * (q.ksw ? kp.a1 : kp.a2);
+#pragma unroll
+          for (int x = 0; x < kSets; ++x) {
+            const double* sx = s + 7 * x;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              acc[x][i] = fma(wa, sx[1 + i], acc[x][i]);
+              acc[x][3 + i] = fma(wb, sx[1 + i], acc[x][3 + i]);
+              acc[x][7 + i] = fma(wd, sx[4 + i], acc[x][7 + i]);
+            }
+            acc[x][6] = fma(wb, sx[0], acc[x][6]);
+            acc[x][10] = fma(wd, sx[0], acc[x][10]);
+          }
+        }
+      }
+      kept += keep ? 1 : 0;
+      ib += gb;
+      ik += gk;
+      if (ik >= q.nkpp) {
+        ik -= q.nkpp;
+        ++ib;
+      }
+    }
+    for (int o = G >> 1; o > 0; o >>= 1) {
+#pragma unroll
+      for (int x = 0; x < kSets; ++x)
+#pragma unroll
+        for (int i = 0; i < kGradSums; ++i)
+          acc[x][i] += rk_shfl_xor<double>(gmask, acc[x][i], o, G);
+      if constexpr (C::kTail)
+#pragma unroll
+        for (int i = 0; i < C::kNI; ++i) I[i] += rk_shfl_xor<double>(gmask, I[i], o, G);
+      kept += __shfl_xor_sync(gmask, kept, o, G);
+    }
+    if (g == 0) my_prims += (unsigned long long)kept;
+    if (kept == 0) continue;
+    double GJ[kNsph], GK[kNsph];
+    if constexpr (kSets == 1 || C::kTail) gamma(GJ, GK);
+    const double deg = double((q.sh[0] == q.sh[1] ? 1 : 2) * (q.sh[2] == q.sh[3] ? 1 : 2) *
+                              (bpair == kpair ? 1 : 2));
+    const int at[4] = {a.basis.atom[q.sh[0]], a.basis.atom[q.sh[1]], a.basis.atom[q.sh[2]],
+                       a.basis.atom[q.sh[3]]};
+    int slot = 0;
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const double* sx = acc[kSets == 1 ? 0 : x];
+      const double f = (x == 0 ? 0.5 : -0.25) * deg * (kSets == 1 ? (x == 0 ? GJ[0] : GK[0]) : 1.0);
+      double lo[3] = {0, 0, 0}, dab[3] = {0, 0, 0}, dcd[3] = {0, 0, 0};
+      if constexpr (C::kTail)
+        C::template tail<double>(I, x == 0 ? GJ : GK, x == 0 ? WJ : WK, q.AB, q.CD, lo, dab, dcd);
+      double* out = (x == 0 ? a.gJ : a.gK) + copy;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        double gA = sx[i], gB = fma(q.AB[i], sx[6], sx[3 + i]), gD = fma(q.CD[i], sx[10], sx[7 + i]);
+        if constexpr (LA > 0) gA -= lo[i];
+        if constexpr (C::kBraHrr) {
+          gA += dab[i];
+          gB -= dab[i];
+        }
+        if constexpr (C::kKetHrr) gD -= dcd[i];
+        const double gC = -(gA + gB + gD);
+        const double gv[4] = {gA, gB, gC, gD};
+#pragma unroll
+        for (int t = 0; t < 4; ++t, ++slot)
+          if ((slot & (G - 1)) == g) atomicAdd(out + 3 * at[t] + i, f * gv[t]);
+      }
+    }
+  }
+  if (a.prim_count && my_prims) atomicAdd(a.prim_count, my_prims);
+}
+
+template <int LA, int LB, int LC, int LD>
+cudaError_t rk_grad_launch_one(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  const int block = 128;
+  auto k = rk_grad_kernel<LA, LB, LC, LD>;
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, block, 0) != cudaSuccess || occ < 1)
+    occ = 1;
+  const long long need = (work * a.group + block - 1) / block;
+  const long long grid = std::max(1LL, std::min((long long)nsm * occ, need));
+  k<<<(unsigned)grid, block, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+}  // namespace lgx

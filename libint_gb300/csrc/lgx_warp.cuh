@@ -953,8 +953,9 @@ __global__ void __launch_bounds__(128) eri_warp_kernel(EriArgs a) {
             ck[s] -= sk;
             if (lane == 0) {
               const int at = a.basis.atom[g.sh[ctr]];
-              atomicAdd(a.gJ + 3 * at + s, 0.5 * degi * sj);
-              atomicAdd(a.gK + 3 * at + s, -0.25 * degi * sk);
+              const size_t cp = size_t(blockIdx.x % a.gcopies) * a.gstride;
+              atomicAdd(a.gJ + cp + 3 * at + s, 0.5 * degi * sj);
+              atomicAdd(a.gK + cp + 3 * at + s, -0.25 * degi * sk);
             }
           } else {  // kModeStore
             const int fl = flags >> 2;
@@ -1005,9 +1006,10 @@ __global__ void __launch_bounds__(128) eri_warp_kernel(EriArgs a) {
       }
       if (MODE == kModeGrad && lane == 0) {
         const int at = a.basis.atom[g.sh[2]];
+        const size_t cp = size_t(blockIdx.x % a.gcopies) * a.gstride;
         for (int s = 0; s < 3; ++s) {
-          atomicAdd(a.gJ + 3 * at + s, 0.5 * degi * cj[s]);
-          atomicAdd(a.gK + 3 * at + s, -0.25 * degi * ck[s]);
+          atomicAdd(a.gJ + cp + 3 * at + s, 0.5 * degi * cj[s]);
+          atomicAdd(a.gK + cp + 3 * at + s, -0.25 * degi * ck[s]);
         }
       }
       __syncwarp();
