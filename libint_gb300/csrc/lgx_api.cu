@@ -725,13 +725,24 @@ bool post_gen_ok(const lgx_context* ctx, const BasisDev& B, const ProgDev& P, in
          post_info(P.host.la, P.host.lb, P.host.lc, P.host.ld, &nacc, &slots);
 }
 
+// Lanes per quartet of a J/K or gradient bin: 1 when the bin's quartets fill
+// the GPU (256 lanes per SM; every lane repeats the stages after the primitive
+// loop), else as many as fill it, up to one lane per primitive quartet.  A
+// lone water in 6-31G has 406 (ss|ss) quartets of up to 1296 primitive
+// quartets: with one lane each its pass took 2.7 ms.
+int fill_group(const lgx_context* ctx, long long nwork, double nq_avg) {
+  int g = 1;
+  while (g < 32 && g < nq_avg && nwork * g < 256LL * ctx->nsm) g *= 2;
+  return g;
+}
+
 // Default variant of a class bin (before or without tuning).
 Variant default_variant(const lgx_context* ctx, const BasisDev& B, const ProgDev& P, int mode,
-                        bool fp32, bool implicit, double nq_avg) {
+                        bool fp32, bool implicit, long long nwork, double nq_avg) {
   Variant v;
   if (rk_eligible(ctx, B, P, mode, fp32)) {
     v.kind = 0;
-    v.group = implicit ? 1 : choose_group(nq_avg);
+    v.group = implicit ? fill_group(ctx, nwork, nq_avg) : choose_group(nq_avg);
   } else {
     v.kind = post_gen_ok(ctx, B, P, mode) ? 2 : 1;
   }
@@ -796,7 +807,7 @@ lgx_status run_block_store(lgx_context* ctx, BasisDev& B, const ProgDev& P, EriA
 lgx_status run_eri(lgx_context* ctx, BasisDev& B, const ProgDev& P, int mode, bool fp32,
                    EriArgs a, long long nwork, double nq_avg = 1.0,
                    const Variant* var = nullptr) {
-  const Variant v = var ? *var : default_variant(ctx, B, P, mode, fp32, a.implicit, nq_avg);
+  const Variant v = var ? *var : default_variant(ctx, B, P, mode, fp32, a.implicit, nwork, nq_avg);
   if (v.kind == 0) return run_rk(ctx, B, P, mode, fp32, a, nwork, v.group);
   if (v.kind == 1 && mode == kModeStore && !fp32 && !a.implicit && nwork <= ctx->nsm)
     return run_block_store(ctx, B, P, a, nwork);
@@ -1343,9 +1354,13 @@ void bin_args(const BinCache& C, const BinHost& bin, int sp, EriArgs& a) {
 // Per-class launch-shape autotuner: for every (class, precision) of the
 // pass without a tuned variant, times the candidate variants (register
 // kernel lanes per quartet; program kernel with interpreted or generated
-// post stage and its staging rows) on a leading sample of the bin's
-// quartets, into scratch accumulators, and keeps the fastest.  Runs once per
-// basis; later passes reuse the choice.
+// post stage and its staging rows) on a sample from the middle of the bin
+// (its ends hold the shallowest and the deepest contractions), into scratch
+// accumulators, and keeps the fastest if it beats the default by 4%, more
+// than two runs of one shape differ.  Runs once per basis; later passes reuse
+// the choice.  The sample is what fills the GPU a few times over, 2^18
+// quartets for the register and 2^14 for the program kernels: with 2^22 and
+// 2^17 the tuning of (H2O)32 cc-pVDZ took five passes' time.
 // mode32: kernel mode of the FP32 precision space (kModeJK, or kModeJKB64
 // for the mixed scheme with the Boys function in FP64), or -1 when the pass
 // runs every quartet in FP64.
@@ -1367,17 +1382,18 @@ lgx_status tune_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int mod
       const int key = tune_key(bin, deriv, kmode, fp32, ctx->op);
       if (ctx->tuned.count(key)) continue;
       std::vector<Variant> cand;
-      const Variant d = default_variant(ctx, B, *P, kmode, fp32, true, bin.nq_avg);
+      const Variant d = default_variant(ctx, B, *P, kmode, fp32, true, bin.total[sp], bin.nq_avg);
       cand.push_back(d);
       if (d.kind == 0) {
-        for (int g = 2; g <= 8 && g <= 2 * bin.nq_avg; g *= 2) cand.push_back({0, g, 0});
+        for (int g = 1; g <= 8 && g <= 2 * bin.nq_avg; g *= 2)
+          if (g != d.group) cand.push_back({0, g, 0});
       } else {
         for (int kind = 1; kind <= d.kind; ++kind) {
           cand.push_back({kind, 1, 8});
           if (bin.nq_avg > 4) cand.push_back({kind, 1, 32});
         }
       }
-      const long long cap = d.kind == 0 ? (1LL << 22) : (1LL << 17);
+      const long long cap = d.kind == 0 ? (1LL << 18) : (1LL << 14);
       const long long sample = std::min<long long>(bin.total[sp], cap);
       if (cand.size() < 2 || sample < ctx->tune_min) {
         ctx->tuned[key] = d;
@@ -1391,6 +1407,7 @@ lgx_status tune_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int mod
       }
       EriArgs a = base;
       bin_args(C, bin, sp, a);
+      a.bin.first = (bin.total[sp] - sample) / 2;
       a.bin.total = sample;
       a.prim_count = nullptr;
       if (mode == kModeJK) {
@@ -1413,7 +1430,9 @@ lgx_status tune_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int mod
         }
         CK(cudaEventSynchronize(ctx->ev1));
         CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-        if (ci == 0 || ms < best) {
+        if (ci == 0 || ms < (bestv.group == d.group && bestv.kind == d.kind && bestv.rows == d.rows
+                                 ? 0.96f * best
+                                 : best)) {
           best = ms;
           bestv = cand[ci];
         }
@@ -1539,7 +1558,8 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
     const auto tv = ctx->tuned.find(tune_key(bin, deriv, kmode, fp32, ctx->op));
     const Variant v = tv != ctx->tuned.end()
                           ? tv->second
-                          : default_variant(ctx, B, *P, kmode, fp32, true, bin.nq_avg);
+                          : default_variant(ctx, B, *P, kmode, fp32, true, bin.total[sp],
+                                            bin.nq_avg);
     cudaStream_t st = ctx->stream;
     if (split) {
       const int b = j.branch;

@@ -51,7 +51,7 @@ struct BinWork {
   const int* seg_j0;           // first ket index (into ket_pairs)
   int nseg;
   int pad;
-  long long total;
+  long long first, total;      // quartets [first, first + total) of the bin
   // FP32 records (EriArgs::jk32) of list position i: jk32[rec[i].x + ip * rec[i].y]
   const int2* bra_rec;
   const int2* ket_rec;

@@ -320,12 +320,13 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
   const int per_warp = 32 / G;  // quartets per warp chunk
   const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long first = a.implicit ? a.bin.first : 0;
   const long long total = a.implicit ? a.bin.total : a.nitems;
   unsigned long long my_prims = 0;
   // Warp chunks of per_warp consecutive quartets, strided over the grid:
   // consecutive quartets share a bin segment (same bra pair, same depth).
   for (long long c = warp_id; c * per_warp < total; c += nwarps) {
-    const long long c0 = c * per_warp;
+    const long long c0 = first + c * per_warp;
     const long long qi = c0 + (lane / G);
     int seg = 0;
     if (a.implicit) {
@@ -336,11 +337,11 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
       // at or before its offset.
       const int seg0 = bin_segment(a.bin, c0);
       const int k = seg0 + 1 + lane;
-      const long long m = (k <= a.bin.nseg ? a.bin.seg_start[k] : total + 64) - c0;  // >= 1
+      const long long m = (k <= a.bin.nseg ? a.bin.seg_start[k] : c0 + 64) - c0;  // >= 1
       const unsigned starts = __reduce_or_sync(0xffffffffu, m < per_warp ? 1u << m : 0u);
       seg = seg0 + __popc(starts & ((2u << (lane / G)) - 1u));
     }
-    if (qi >= total) continue;
+    if (qi >= first + total) continue;
     int bpair, kpair, flags, orig = 0;
     long long outoff = 0;
     int2 brec = make_int2(0, 0), krec = make_int2(0, 0);

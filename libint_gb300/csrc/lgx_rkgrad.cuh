@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
   const int per_warp = 32 / G;
   const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const long long total = a.bin.total;
+  const long long first = a.bin.first, total = a.bin.total;
   const size_t copy = size_t(blockIdx.x % a.gcopies) * a.gstride;
   unsigned long long my_prims = 0;
   PrimScreen scr;
@@ -50,15 +50,15 @@ __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
   scr.fprec = a.fprecision;
   scr.fln_prec = a.fln_prec;
   for (long long c = warp_id; c * per_warp < total; c += nwarps) {
-    const long long c0 = c * per_warp;
+    const long long c0 = first + c * per_warp;
     const long long qi = c0 + (lane / G);
     // segment of each quartet of the chunk (see rk_kernel)
     const int seg0 = bin_segment(a.bin, c0);
     const int kseg = seg0 + 1 + lane;
-    const long long mseg = (kseg <= a.bin.nseg ? a.bin.seg_start[kseg] : total + 64) - c0;
+    const long long mseg = (kseg <= a.bin.nseg ? a.bin.seg_start[kseg] : c0 + 64) - c0;
     const unsigned starts = __reduce_or_sync(0xffffffffu, mseg < per_warp ? 1u << mseg : 0u);
     const int seg = seg0 + __popc(starts & ((2u << (lane / G)) - 1u));
-    if (qi >= total) continue;
+    if (qi >= first + total) continue;
     const int bpair = a.bin.bra_pairs[a.bin.seg_bra[seg]];
     const int kpair = a.bin.ket_pairs[int(qi - a.bin.seg_start[seg]) + a.bin.seg_j0[seg]];
     RkQuartet<double> q;

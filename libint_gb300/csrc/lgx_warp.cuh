@@ -867,6 +867,7 @@ __global__ void __launch_bounds__(128) eri_warp_kernel(EriArgs a) {
     T* base = reinterpret_cast<T*>(smem_d) + wpb * stage_per_warp;
     slots = base + size_t(wib) * a.slot_stride;
   }
+  const long long first = a.implicit ? a.bin.first : 0;
   const long long total = a.implicit ? a.bin.total : a.nitems;
   long long nchunks = 0;
   unsigned long long my_prims = 0;
@@ -879,7 +880,8 @@ __global__ void __launch_bounds__(128) eri_warp_kernel(EriArgs a) {
       if (lane == 0) atomicExch(a.error_flag, 1);
       break;
     }
-    const long long end = min(total, start + (long long)a.chunk);
+    const long long end = first + min(total, start + (long long)a.chunk);
+    start += first;
     int seg = 0;
     if (a.implicit) seg = bin_segment(a.bin, start);
     for (long long q = start; q < end; ++q) {
