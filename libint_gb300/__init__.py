@@ -444,9 +444,9 @@ class Context:
         int32.  Returns the offsets (computed as in compute_batch when not
         given)."""
         q = np.ascontiguousarray(quartets, dtype=np.int32).reshape(-1, 4)
-        if q.size and (q.min() < 0 or q.max() >= len(self.basis)):
-            raise LgxError(_lgx.LGX_ERR_INVALID_ARG, "quartet shell index out of range")
         if offsets is None:
+            if q.size and (q.min() < 0 or q.max() >= len(self.basis)):
+                raise LgxError(_lgx.LGX_ERR_INVALID_ARG, "quartet shell index out of range")
             sizes = np.array([s.size() for s in self.basis], np.int64)
             nv = (sizes[q[:, 0]] * sizes[q[:, 1]] * sizes[q[:, 2]] * sizes[q[:, 3]] *
                   (12 if deriv else 1))

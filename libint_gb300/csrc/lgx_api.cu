@@ -12,7 +12,6 @@
 #include <mutex>
 #include <numeric>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/lgx.h"
@@ -30,6 +29,8 @@ cudaError_t launch_jk_finalize(const double* Jacc, const double* Kacc, double* J
 cudaError_t launch_drop_pairs(PrimPairRec* pp, int n, double ln_prec, cudaStream_t st);
 size_t stage_bytes_per_warp(bool fp32, int rows);
 int eri_blocks_per_sm(int mode, bool fp32, int block, size_t smem);
+cudaError_t launch_list_count(const ListArgs& a, int nsm, cudaStream_t st);
+cudaError_t launch_list_scatter(const ListArgs& a, cudaStream_t st);
 cudaError_t launch_d2f(const double* src, float* dst, long long n, cudaStream_t st);
 cudaError_t launch_shell_block_norm(const DevBasis& b, const double* D, int nbf, double* out,
                                     cudaStream_t st);
@@ -260,6 +261,7 @@ struct lgx_context {
   BasisDev basis, small;
   DBuf gscratch, counter, errflag, primcount;
   DBuf items, out, isnull;
+  DBuf list_in, list_keys, list_cnt, list_tab;  // explicit lists classified on the GPU
   DBuf Jacc, Kacc, Dd, Jd, Kd, gsum, gcopies;  // gradients: sum and per-SM copies
   DBuf prim_rows, prim_slots;  // lgx_compute_primitive_set
   DBuf boysT, boysF;           // lgx_boys
@@ -877,24 +879,33 @@ Canon canonicalize(const BasisDev& B, const int* s) {
   return q;
 }
 
-// Explicit quartet list -> grouped launches (store mode).
-// mode32: kernel mode of the FP32 items (quartets with K12 K34 <
-// mixed_thresh; kModeStore or kModeStoreB64), used when mixed_thresh > 0.
-lgx_status run_explicit(lgx_context* ctx, BasisDev& B, const int32_t* quartets, long long n,
-                        int deriv, int mode, double mixed_thresh, const int64_t* offsets,
-                        double* d_out, int* d_isnull, double precision, int screening,
-                        double* d_kschwarz, int mode32 = kModeStore) {
-  // class key of each quartet from a (la, lb, lc, ld) table, counting
-  // passes, and a stable scatter of the work items into one array grouped by
-  // key (ascending key order, as the launches below go); long lists split
-  // both passes over the host threads (per-thread counts merged so that the
-  // items of a class keep the list order, packed offsets fixed up by the
-  // chunks' prefix sums)
+// One launch of an explicit list: items [begin, begin + count) of one class
+// and precision; group > 0 fixes the register kernel's lanes per quartet.
+struct ListSeg {
+  int la, lb, lc, ld;
+  bool fp32;
+  size_t begin, count;
+  double nq;  // mean primitive quartets per quartet
+  int group;
+};
+struct ListPlan {
+  std::vector<ListSeg> segs;
+  size_t need = 0;  // end of the furthest set (doubles)
+};
+
+// Lists from this length on are classified on the GPU: below, the host loop
+// (about 8 ns a quartet) is shorter than the extra launches and the wait for
+// their counts (about 50 us).
+constexpr long long kListDeviceMin = 8192;
+
+// class key of (la, lb, lc, ld) and back
+struct ClassTables {
+  std::vector<int> key;                   // (la, lb, lc, ld) -> class index
+  std::vector<std::array<int, 4>> shape;  // class index -> (la, lb, lc, ld)
+};
+const ClassTables& class_tables() {
   constexpr int LK = kMaxLInternal + 1;
-  struct ClassTables {
-    std::vector<int> key;          // (la, lb, lc, ld) -> class index
-    std::vector<std::array<int, 4>> shape;  // class index -> (la, lb, lc, ld)
-  };
+  static_assert(LK == kListLK, "class table of lgx_list.cu");
   static const ClassTables kTab = [] {
     ClassTables t;
     t.key.assign(LK * LK * LK * LK, -1);
@@ -909,126 +920,205 @@ lgx_status run_explicit(lgx_context* ctx, BasisDev& B, const int32_t* quartets, 
           }
     return t;
   }();
-  const int nkeys = 2 * num_classes();
-  struct G {
-    size_t count = 0, begin = 0;
-    double nq = 0;
-    int la = 0, lb = 0, lc = 0, ld = 0;
-    bool fp32 = false;
-  };
+  return kTab;
+}
+
+// The class launches of counts per key (depth of a key as in lgx_list.cu).
+// FP64 register-kernel classes are cut where the lanes per quartet change;
+// everything else is one launch per class and precision.  Lanes per quartet:
+// one per 8 primitive quartets (the chain of one lane stays short beside the
+// stages that every lane repeats), more where the class's quartets alone do
+// not fill the GPU.  Fewer than 4096 lanes' worth of a depth joins the deeper
+// one's launch.
+void list_segments(const lgx_context* ctx, const BasisDev& B, int deriv, int mode,
+                   const unsigned* hist, const unsigned long long* nqsum, ListPlan& plan) {
+  const ClassTables& tab = class_tables();
+  size_t at = 0;
+  for (int k = 0; k < 2 * num_classes(); ++k) {
+    const unsigned* h = hist + size_t(k) * kListDepth;
+    size_t count = 0;
+    for (int d = 0; d < kListDepth; ++d) count += h[d];
+    if (!count) continue;
+    const auto& sh = tab.shape[k / 2];
+    ListSeg seg{sh[0], sh[1], sh[2], sh[3], (k & 1) != 0, at, count,
+                double(nqsum[k]) / double(count), 0};
+    const bool cut = ctx->use_rk && B.std_pure && deriv == 0 && mode == kModeStore && !seg.fp32 &&
+                     rk_available(false, mode, ctx->op != LGX_OP_COULOMB, seg.la, seg.lb, seg.lc,
+                                  seg.ld);
+    if (!cut) {
+      plan.segs.push_back(seg);
+    } else {
+      seg.count = 0;
+      seg.group = 0;
+      for (int d = 0; d < kListDepth; ++d) {
+        if (!h[d]) continue;
+        const double nq = std::ldexp(1.0, kListDepth - 1 - d);
+        int g = 1;
+        while (g < 32 && (8 * g <= nq || (2 * g <= nq && double(count) * g < 256.0 * ctx->nsm)))
+          g *= 2;
+        if (seg.count && g != seg.group && size_t(h[d]) * g >= 4096) {
+          plan.segs.push_back(seg);
+          seg.begin += seg.count;
+          seg.count = 0;
+        }
+        if (seg.count == 0) seg.group = g;
+        seg.count += h[d];
+      }
+      plan.segs.push_back(seg);
+    }
+    at += count;
+  }
+}
+
+// Work items of a list in ctx->items, grouped by class, and their launches.
+// Fails on a shell index out of range before anything is written.
+lgx_status plan_list(lgx_context* ctx, BasisDev& B, const int32_t* quartets, long long n,
+                     int deriv, int mode, double mixed_thresh, const int64_t* offsets,
+                     ListPlan& plan) {
+  constexpr int LK = kMaxLInternal + 1;
+  const ClassTables& tab = class_tables();
   const size_t nn = size_t(std::max<long long>(n, 0));
+  const long long nsets = deriv ? 12 : 1;
+  const bool split = mode == kModeStore && mixed_thresh > 0 && B.schwarz_ok;
+  const int nkeys = 2 * num_classes() * kListDepth;
+  auto values = [&](const int* s) {
+    long long nv = nsets;
+    for (int k = 0; k < 4; ++k) nv *= nfunc(B.l[s[k]], B.pure[s[k]]);
+    return nv;
+  };
+  CK(ctx->items.ensure(std::max<size_t>(nn, 1) * sizeof(QuartetItem)));
+  if (n >= kListDeviceMin) {
+    std::vector<int64_t> packed;
+    if (!offsets && mode != kModeSchwarz) {
+      packed.resize(nn);
+      long long run = 0;
+      for (size_t q = 0; q < nn; ++q) {
+        const int* s = quartets + 4 * q;
+        for (int k = 0; k < 4; ++k)
+          if (s[k] < 0 || s[k] >= B.nshell)
+            return fail(ctx, LGX_ERR_INVALID_ARG, "quartet shell index out of range");
+        packed[q] = run;
+        run += values(s);
+      }
+      offsets = packed.data();
+    }
+    // [statistics][sums][counts], read back together
+    const size_t nsum = 2 * size_t(num_classes()), head = (2 + nsum) * sizeof(unsigned long long);
+    const size_t cbytes = head + size_t(nkeys) * sizeof(unsigned);
+    const size_t obytes = offsets ? nn * sizeof(int64_t) : 0;
+    CK(ctx->list_in.ensure(nn * sizeof(int4) + obytes));
+    CK(ctx->list_keys.ensure(nn * sizeof(unsigned short)));
+    CK(ctx->list_cnt.ensure(cbytes));
+    if (!ctx->list_tab.p) {
+      CK(ctx->list_tab.ensure(tab.key.size() * sizeof(int)));
+      CK(cudaMemcpyAsync(ctx->list_tab.p, tab.key.data(), tab.key.size() * sizeof(int),
+                         cudaMemcpyHostToDevice, ctx->stream));
+    }
+    ListArgs a{};
+    a.b = B.dev;
+    a.q = ctx->list_in.as<int4>();
+    a.off = offsets ? reinterpret_cast<const long long*>(a.q + nn) : nullptr;
+    a.n = n;
+    a.nsets = int(nsets);
+    a.nkeys = nkeys;
+    a.kpair = split ? B.Kd.as<double>() : nullptr;
+    a.mixed = mixed_thresh;
+    a.tab = ctx->list_tab.as<int>();
+    a.keys = ctx->list_keys.as<unsigned short>();
+    a.stat = ctx->list_cnt.as<unsigned long long>();
+    a.nqsum = a.stat + 2;
+    a.hist = reinterpret_cast<unsigned*>(a.nqsum + nsum);
+    a.items = ctx->items.as<QuartetItem>();
+    CK(cudaMemcpyAsync(ctx->list_in.p, quartets, nn * sizeof(int4), cudaMemcpyHostToDevice,
+                       ctx->stream));
+    if (offsets)
+      CK(cudaMemcpyAsync(ctx->list_in.as<int4>() + nn, offsets, obytes, cudaMemcpyHostToDevice,
+                         ctx->stream));
+    CK(cudaMemsetAsync(ctx->list_cnt.p, 0, cbytes, ctx->stream));
+    CK(launch_list_count(a, ctx->nsm, ctx->stream));
+    std::vector<unsigned long long> cnt((cbytes + 7) / 8);
+    CK(cudaMemcpyAsync(cnt.data(), ctx->list_cnt.p, cbytes, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (cnt[1]) return fail(ctx, LGX_ERR_INVALID_ARG, "quartet shell index out of range");
+    plan.need = size_t(cnt[0]);
+    unsigned* hist = reinterpret_cast<unsigned*>(cnt.data() + 2 + nsum);
+    list_segments(ctx, B, deriv, mode, hist, cnt.data() + 2, plan);
+    unsigned run = 0;  // counts -> first place of each key
+    for (int k = 0; k < nkeys; ++k) {
+      const unsigned c = hist[k];
+      hist[k] = run;
+      run += c;
+    }
+    CK(cudaMemcpyAsync(a.hist, hist, size_t(nkeys) * sizeof(unsigned), cudaMemcpyHostToDevice,
+                       ctx->stream));
+    CK(launch_list_scatter(a, ctx->stream));
+    return LGX_OK;
+  }
+  // class key of each quartet, then a stable scatter of the work items into
+  // one array grouped by key (ascending, as the launches go)
+  const int ncls = 2 * num_classes();
   std::vector<QuartetItem> items(nn);
   std::vector<int> keys(nn);
-  const int nthr = nn >= 65536 ? int(std::max(1u, std::min(16u, std::thread::hardware_concurrency())))
-                               : 1;
-  const size_t chunk = (nn + nthr - 1) / std::max(1, nthr);
-  std::vector<std::vector<size_t>> cnt(nthr, std::vector<size_t>(nkeys, 0));
-  std::vector<std::vector<double>> nqs(nthr, std::vector<double>(nkeys, 0.0));
-  std::vector<long long> span(nthr, 0);  // packed output length of each chunk
-  std::vector<int> bad(nthr, 0);          // 1: shell index out of range, 2: l beyond the build
-  const long long nsets = deriv ? 12 : 1;
-  auto pass1 = [&](int t) {
-    const size_t q0 = std::min(nn, size_t(t) * chunk), q1 = std::min(nn, q0 + chunk);
-    long long run_off = 0;
-    for (size_t q = q0; q < q1; ++q) {
-      const int* s = quartets + 4 * q;
-      for (int k = 0; k < 4; ++k)
-        if (s[k] < 0 || s[k] >= B.nshell) {
-          bad[t] = 1;
-          return;
-        }
-      const Canon c = canonicalize(B, s);
-      QuartetItem& it = items[q];
-      it.bra_pair = int(pidx(std::max(c.c[0], c.c[1]), std::min(c.c[0], c.c[1])));
-      it.ket_pair = int(pidx(std::max(c.c[2], c.c[3]), std::min(c.c[2], c.c[3])));
-      it.flags = c.flags;
-      it.pad = int(q);
-      if (mode == kModeSchwarz) {
-        it.out = offsets ? offsets[q] : (long long)q;
-      } else if (offsets) {
-        it.out = offsets[q];
-      } else {
-        long long nv = 1;
-        for (int k = 0; k < 4; ++k) nv *= nfunc(B.l[s[k]], B.pure[s[k]]);
-        it.out = run_off;  // chunk-relative; the chunk's base is added in the scatter
-        run_off += nv * nsets;
-      }
-      bool fp32 = false;
-      if (mode == kModeStore && mixed_thresh > 0 && B.schwarz_ok) {
-        const double bound = B.Kpair[it.bra_pair] * B.Kpair[it.ket_pair];
-        fp32 = bound < mixed_thresh;
-      }
-      const int ci = kTab.key[((c.la * LK + c.lb) * LK + c.lc) * LK + c.ld];
-      if (ci < 0) {
-        bad[t] = 2;
-        return;
-      }
-      const int key = ci * 2 + (fp32 ? 1 : 0);
-      keys[q] = key;
-      ++cnt[t][key];
-      nqs[t][key] += double(B.hpairs[it.bra_pair].npp) * double(B.hpairs[it.ket_pair].npp);
+  std::vector<size_t> pos(ncls, 0);
+  std::vector<double> nqs(ncls, 0.0);
+  long long run = 0;
+  for (size_t q = 0; q < nn; ++q) {
+    const int* s = quartets + 4 * q;
+    for (int k = 0; k < 4; ++k)
+      if (s[k] < 0 || s[k] >= B.nshell)
+        return fail(ctx, LGX_ERR_INVALID_ARG, "quartet shell index out of range");
+    const Canon c = canonicalize(B, s);
+    QuartetItem& it = items[q];
+    it.bra_pair = int(pidx(std::max(c.c[0], c.c[1]), std::min(c.c[0], c.c[1])));
+    it.ket_pair = int(pidx(std::max(c.c[2], c.c[3]), std::min(c.c[2], c.c[3])));
+    it.flags = c.flags;
+    it.pad = int(q);
+    const long long nv = values(s);
+    if (mode == kModeSchwarz) {
+      it.out = offsets ? offsets[q] : (long long)q;
+    } else {
+      it.out = offsets ? offsets[q] : run;
+      run += nv;
+      plan.need = std::max(plan.need, size_t(it.out + nv));
     }
-    span[t] = run_off;
-  };
-  auto run_threads = [&](auto&& fn) {
-    if (nthr == 1) {
-      fn(0);
-      return;
-    }
-    std::vector<std::thread> th;
-    th.reserve(nthr);
-    for (int t = 0; t < nthr; ++t) th.emplace_back(fn, t);
-    for (auto& x : th) x.join();
-  };
-  run_threads(pass1);
-  for (int t = 0; t < nthr; ++t) {
-    if (bad[t] == 1) return fail(ctx, LGX_ERR_INVALID_ARG, "quartet shell index out of range");
-    if (bad[t] == 2) return fail(ctx, LGX_ERR_LMAX_EXCEEDED, "angular momentum beyond LGX_MAX_L");
+    bool fp32 = false;
+    if (split) fp32 = B.Kpair[it.bra_pair] * B.Kpair[it.ket_pair] < mixed_thresh;
+    const int ci = tab.key[((c.la * LK + c.lb) * LK + c.lc) * LK + c.ld];
+    if (ci < 0) return fail(ctx, LGX_ERR_LMAX_EXCEEDED, "angular momentum beyond LGX_MAX_L");
+    keys[q] = ci * 2 + (fp32 ? 1 : 0);
+    ++pos[keys[q]];
+    nqs[keys[q]] += double(B.hpairs[it.bra_pair].npp) * double(B.hpairs[it.ket_pair].npp);
   }
-  std::vector<long long> base(nthr, 0);  // packed output offset of each chunk
-  for (int t = 1; t < nthr; ++t) base[t] = base[t - 1] + span[t - 1];
-  // class order ascending; within a class, chunk order (= list order)
-  std::vector<G> gk(nkeys);
-  std::vector<std::vector<size_t>> pos(nthr, std::vector<size_t>(nkeys, 0));
   size_t total = 0;
-  std::vector<int> order;  // keys with work, ascending
-  for (int k = 0; k < nkeys; ++k) {
-    G& g = gk[k];
-    g.begin = total;
-    for (int t = 0; t < nthr; ++t) {
-      pos[t][k] = total;
-      total += cnt[t][k];
-      g.nq += nqs[t][k];
+  for (int k = 0; k < ncls; ++k) {
+    const size_t count = pos[k];
+    pos[k] = total;
+    if (count) {
+      const auto& sh = tab.shape[k / 2];
+      plan.segs.push_back({sh[0], sh[1], sh[2], sh[3], (k & 1) != 0, total, count,
+                           nqs[k] / double(count), 0});
     }
-    g.count = total - g.begin;
-    if (g.count) {
-      const auto& sh = kTab.shape[k / 2];
-      g.la = sh[0]; g.lb = sh[1]; g.lc = sh[2]; g.ld = sh[3];
-      g.fp32 = (k & 1) != 0;
-      order.push_back(k);
-    }
+    total += count;
   }
-  CK(ctx->items.ensure(std::max<size_t>(total, 1) * sizeof(QuartetItem)));
   std::vector<QuartetItem> all(total);
-  const bool packed = !offsets && mode != kModeSchwarz;
-  auto scatter = [&](int t) {
-    const size_t q0 = std::min(nn, size_t(t) * chunk), q1 = std::min(nn, q0 + chunk);
-    std::vector<size_t>& p = pos[t];
-    for (size_t q = q0; q < q1; ++q) {
-      QuartetItem it = items[q];
-      if (packed) it.out += base[t];
-      all[p[keys[q]]++] = it;
-    }
-  };
-  run_threads(scatter);
+  for (size_t q = 0; q < nn; ++q) all[pos[keys[q]]++] = items[q];
   CK(cudaMemcpyAsync(ctx->items.p, all.data(), total * sizeof(QuartetItem),
                      cudaMemcpyHostToDevice, ctx->stream));
+  return LGX_OK;
+}
+
+// The launches of a planned list.
+// mode32: kernel mode of the FP32 items (quartets with K12 K34 <
+// mixed_thresh; kModeStore or kModeStoreB64).
+lgx_status run_list(lgx_context* ctx, BasisDev& B, const ListPlan& plan, int deriv, int mode,
+                    double* d_out, int* d_isnull, double precision, int screening,
+                    double* d_kschwarz, int mode32) {
   // the class launches run on parallel branches (streams forked from and
   // joined back into ctx->stream, one work counter and one program-kernel
   // slot scratch per launch / branch): a short list, such as the raised and
   // lowered quartets of a second-derivative set, then costs its slowest
   // class rather than the sum of its classes
-  const int ng = int(order.size());
+  const int ng = int(plan.segs.size());
   const int nbr = std::min(ng, lgx_context::kMaxBranches);
   const bool split = ctx->overlap && nbr > 1;
   CK(ctx->xcounters.ensure(size_t(ng) * sizeof(unsigned long long)));
@@ -1049,12 +1139,11 @@ lgx_status run_explicit(lgx_context* ctx, BasisDev& B, const int32_t* quartets, 
   } restore{ctx};
   size_t gi = 0;
   lgx_status s = LGX_OK;
-  for (const int key : order) {
-    const G& grp = gk[key];
+  for (const ListSeg& seg : plan.segs) {
     ProgDev* P = nullptr;
-    s = get_prog(ctx, grp.la, grp.lb, grp.lc, grp.ld, deriv, &P);
+    s = get_prog(ctx, seg.la, seg.lb, seg.lc, seg.ld, deriv, &P);
     if (s != LGX_OK) break;
-    const bool fp32 = grp.fp32;
+    const bool fp32 = seg.fp32;
     if (split) {
       const int b = int(gi) % nbr;
       ctx->launch_stream = fp32 ? ctx->s32[b] : ctx->s64[b];
@@ -1065,14 +1154,15 @@ lgx_status run_explicit(lgx_context* ctx, BasisDev& B, const int32_t* quartets, 
     a.precision = precision;
     a.ln_prec = precision > 0 ? std::log(precision) : -std::numeric_limits<double>::max();
     a.screening = screening;
-    a.items = ctx->items.as<QuartetItem>() + grp.begin;
-    a.nitems = (long long)grp.count;
+    a.items = ctx->items.as<QuartetItem>() + seg.begin;
+    a.nitems = (long long)seg.count;
     a.implicit = 0;
     a.out = d_out;
     a.is_null = d_isnull;
     a.kschwarz = d_kschwarz;
-    const double nq = grp.nq / double(std::max<size_t>(1, grp.count));
-    s = run_eri(ctx, B, *P, fp32 ? mode32 : mode, fp32, a, a.nitems, nq);
+    const Variant v{0, seg.group, 0};
+    s = run_eri(ctx, B, *P, fp32 ? mode32 : mode, fp32, a, a.nitems, seg.nq,
+                seg.group > 0 ? &v : nullptr);
     if (s != LGX_OK) break;
     ++gi;
   }
@@ -1085,6 +1175,17 @@ lgx_status run_explicit(lgx_context* ctx, BasisDev& B, const int32_t* quartets, 
     }
   }
   return s;
+}
+
+// Explicit FP64 quartet list -> grouped launches.
+lgx_status run_explicit(lgx_context* ctx, BasisDev& B, const int32_t* quartets, long long n,
+                        int deriv, int mode, const int64_t* offsets, double* d_out,
+                        int* d_isnull, double precision, int screening, double* d_kschwarz) {
+  ListPlan plan;
+  lgx_status s = plan_list(ctx, B, quartets, n, deriv, mode, 0.0, offsets, plan);
+  if (s != LGX_OK) return s;
+  return run_list(ctx, B, plan, deriv, mode, d_out, d_isnull, precision, screening, d_kschwarz,
+                  kModeStore);
 }
 
 lgx_status ensure_schwarz(lgx_context* ctx, BasisDev& B) {
@@ -1101,8 +1202,8 @@ lgx_status ensure_schwarz(lgx_context* ctx, BasisDev& B) {
   }
   // kept on the device too: the density-weighted J/K screening reads it
   CK(B.Kd.ensure(npairs * sizeof(double)));
-  s = run_explicit(ctx, B, q.data(), npairs, 0, kModeSchwarz, 0.0, nullptr, nullptr, nullptr,
-                   0.0, 0, B.Kd.as<double>());
+  s = run_explicit(ctx, B, q.data(), npairs, 0, kModeSchwarz, nullptr, nullptr, nullptr, 0.0, 0,
+                   B.Kd.as<double>());
   if (s != LGX_OK) return s;
   B.Kpair.resize(npairs);
   CK(cudaMemcpyAsync(B.Kpair.data(), B.Kd.p, npairs * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1859,7 +1960,7 @@ lgx_status shellset_deriv2(lgx_context* ctx, const lgx_shell shells[4], double p
   CK(ctx->out.ensure(std::max<size_t>(total, 1) * sizeof(double)));
   CK(ctx->isnull.ensure(size_t(nq) * sizeof(int)));
   CK(cudaMemsetAsync(ctx->out.p, 0, total * sizeof(double), ctx->stream));
-  s = run_explicit(ctx, ctx->small, q.data(), nq, 1, kModeStore, 0.0, off.data(),
+  s = run_explicit(ctx, ctx->small, q.data(), nq, 1, kModeStore, off.data(),
                    ctx->out.as<double>(), ctx->isnull.as<int>(), precision, screening, nullptr);
   if (s != LGX_OK) return s;
   std::vector<double> d1(total);
@@ -2293,7 +2394,7 @@ lgx_status shellset_locked(lgx_context* ctx, const lgx_shell shells[4], int deri
   CK(ctx->out.ensure(size_t(nv * ns) * sizeof(double)));
   CK(ctx->isnull.ensure(sizeof(int)));
   const int32_t q[4] = {0, 1, 2, 3};
-  s = run_explicit(ctx, ctx->small, q, 1, deriv, kModeStore, 0.0, nullptr, ctx->out.as<double>(),
+  s = run_explicit(ctx, ctx->small, q, 1, deriv, kModeStore, nullptr, ctx->out.as<double>(),
                    ctx->isnull.as<int>(), precision, screening, nullptr);
   if (s != LGX_OK) return s;
   int nul = 0;
@@ -2437,19 +2538,6 @@ static lgx_status compute_batch(lgx_context* ctx, const int32_t* quartets, int64
   if (mixed_mode(mode) && deriv) return fail(ctx, LGX_ERR_INVALID_ARG, "mixed mode is deriv 0");
   CK(cudaSetDevice(ctx->device));
   BasisDev& B = ctx->basis;
-  size_t need = 0;
-  for (int64_t q = 0; q < n; ++q) {
-    long long nv = 1;
-    for (int k = 0; k < 4; ++k) {
-      const int s = quartets[4 * q + k];
-      if (s < 0 || s >= B.nshell) return fail(ctx, LGX_ERR_INVALID_ARG, "shell index out of range");
-      nv *= nfunc(B.l[s], B.pure[s]);
-    }
-    nv *= deriv ? 12 : 1;
-    const size_t end = size_t((offsets ? offsets[q] : (int64_t)need) + nv);
-    need = offsets ? std::max(need, end) : end;
-  }
-  if (need > out_capacity) return fail(ctx, LGX_ERR_TOO_LARGE, "output buffer too small");
   lgx_status s;
   if (mixed_mode(mode)) {
     s = ensure_schwarz(ctx, B);
@@ -2458,6 +2546,12 @@ static lgx_status compute_batch(lgx_context* ctx, const int32_t* quartets, int64
   const double eps = std::numeric_limits<double>::epsilon();
   s = ensure_pairs(ctx, B, std::log(eps), 0);
   if (s != LGX_OK) return s;
+  ListPlan plan;
+  s = plan_list(ctx, B, quartets, n, deriv, kModeStore, mixed_mode(mode) ? mixed_thresh : 0.0,
+                offsets, plan);
+  if (s != LGX_OK) return s;
+  const size_t need = plan.need;
+  if (need > out_capacity) return fail(ctx, LGX_ERR_TOO_LARGE, "output buffer too small");
   double* d_out = out;
   int* d_isnull = reinterpret_cast<int*>(is_null);
   if (!device_out) {
@@ -2469,9 +2563,8 @@ static lgx_status compute_batch(lgx_context* ctx, const int32_t* quartets, int64
     d_isnull = ctx->isnull.as<int>();
   }
   CK(cudaMemsetAsync(d_out, 0, std::max<size_t>(need, 1) * sizeof(double), ctx->stream));
-  s = run_explicit(ctx, B, quartets, n, deriv, kModeStore,
-                   mixed_mode(mode) ? mixed_thresh : 0.0, offsets, d_out, d_isnull, eps, 0,
-                   nullptr, mixed_mode(mode) ? fp32_kernel_mode(ctx, mode, kModeStore) : kModeStore);
+  s = run_list(ctx, B, plan, deriv, kModeStore, d_out, d_isnull, eps, 0, nullptr,
+               mixed_mode(mode) ? fp32_kernel_mode(ctx, mode, kModeStore) : kModeStore);
   if (s != LGX_OK) return s;
   if (!device_out) {
     CK(cudaMemcpyAsync(out, d_out, need * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

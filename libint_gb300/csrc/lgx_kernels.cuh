@@ -38,6 +38,28 @@ struct QuartetItem {
   long long out;           // output offset (doubles) or K index (Schwarz)
 };
 
+// Explicit quartet list in device memory and its grouping (lgx_list.cu).
+// A key is (class * 2 + FP32) * kListDepth + depth, depth counted from the
+// deepest contraction (kListDepth - 1 - log2 of the primitive quartets).
+constexpr int kListDepth = 17;  // up to 16^4 primitive quartets
+constexpr int kListLK = 5;      // angular momenta of the class table
+struct ListArgs {
+  DevBasis b;
+  const int4* q;
+  const long long* off;  // output offset per quartet; null: its index
+  long long n;
+  int nsets;             // sets per quartet (1 or 12)
+  int nkeys;
+  const double* kpair;   // Schwarz factors when the list is split by precision, else null
+  double mixed;
+  const int* tab;        // (l1, l2, l3, l4) -> class index
+  unsigned short* keys;
+  unsigned* hist;        // counts per key, then the next free place per key
+  unsigned long long* nqsum;  // primitive quartets per class and precision
+  unsigned long long* stat;   // [0] end of the furthest set, [1] bad shell index
+  QuartetItem* items;
+};
+
 // Implicit work: one class bin of the screened J/K quartet space as a list
 // of segments.  A segment is one bra pair with a contiguous run of ket
 // pairs of one contraction-depth group; segments are ordered by (bra depth
