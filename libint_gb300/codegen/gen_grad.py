@@ -23,6 +23,13 @@ Per class:
       (kSums values), I += contracted (e0|f0), e from la-1;
   tail<T>(I, G, W, AB, CD, lo, dab, dcd): the terms without an exponent.
 
+First-derivative shell sets of explicit lists (DerivCls): contracted (e0|f0)
+accumulators, unweighted and weighted by 2a of A, B and D, then per centre and
+direction the HRR of the raised and lowered sets (master_rrs_list.h:52-55) and
+the solid-harmonic transform; centre C by translational invariance.
+  prim<T>(F, g, w, I): w = 2a of A, B, D;
+  sets<T>(I, AB, CD, v): v[ctr * 3 + dir][kNsph] of A, B, D.
+
 usage: python libint_gb300/codegen/gen_grad.py
 """
 from __future__ import annotations
@@ -39,6 +46,8 @@ from gen_rk import (Emitter, _write_if_changed, comps, first_dir, lit, ncart,  #
 GEN_DIR = os.path.join(os.path.dirname(HERE), "csrc", "gen")
 # total angular momentum of the classes (see rk_grad_kernel for where it ends)
 GRAD_MAX_L = 5
+# classes of the derivative store kernels (see rk_deriv_kernel)
+DERIV_MAX_L = 3
 N_UNITS = 8
 XYZ = "xyz"
 
@@ -282,6 +291,109 @@ def gen_class(la, lb, lc, ld):
     return "\n".join(s)
 
 
+def gen_deriv_class(la, lb, lc, ld):
+    ls = [la, lb, lc, ld]
+    acc = {}      # (weight, e, f) -> accumulator
+    memo = {}
+    em = Emitter()
+
+    def leaf(w, e, f):
+        k = acc.setdefault((w, e, f), len(acc))
+        return "I[%d]" % k
+
+    def bra(w, a, b, f):
+        if sum(b) == 0:
+            return leaf(w, a, f)
+        key = (w, "b", a, b, f)
+        if key not in memo:
+            i = first_dir(b)
+            memo[key] = em.tmp("fma(AB[%d], %s, %s)" % (i, bra(w, a, sh(b, i, -1), f),
+                                                       bra(w, sh(a, i, 1), sh(b, i, -1), f)))
+        return memo[key]
+
+    def ket(w, a, b, c, d):
+        if sum(d) == 0:
+            return bra(w, a, b, c)
+        key = (w, "k", a, b, c, d)
+        if key not in memo:
+            j = first_dir(d)
+            memo[key] = em.tmp("fma(CD[%d], %s, %s)" % (j, ket(w, a, b, c, sh(d, j, -1)),
+                                                       ket(w, a, b, sh(c, j, 1), sh(d, j, -1))))
+        return memo[key]
+
+    nsph = None
+    for x, pos in enumerate((0, 1, 3)):  # A, B, D
+        for i in range(3):
+            vals = []
+            for a in comps(la):
+                for b in comps(lb):
+                    for c in comps(lc):
+                        for d in comps(ld):
+                            q = [a, b, c, d]
+                            up = list(q)
+                            up[pos] = sh(q[pos], i, 1)
+                            expr = ket(x + 1, *up)
+                            if q[pos][i] > 0:
+                                dn = list(q)
+                                dn[pos] = sh(q[pos], i, -1)
+                                n = q[pos][i]
+                                low = ket(0, *dn)
+                                expr = em.tmp("%s - %s" % (expr, low) if n == 1 else
+                                              "fma(T(-%d), %s, %s)" % (n, low, expr))
+                            vals.append(expr)
+            dims = [ncart(l) for l in ls]
+            for k in range(4):
+                if ls[k] < 2:
+                    continue
+                M = sph_matrix(ls[k])
+                npure = 2 * ls[k] + 1
+                outer, inner = math.prod(dims[:k]), math.prod(dims[k + 1:])
+                nxt = []
+                for oo in range(outer):
+                    for p in range(npure):
+                        for ii in range(inner):
+                            expr = None
+                            for c in range(dims[k]):
+                                if M[p][c] != 0.0:
+                                    src = vals[(oo * dims[k] + c) * inner + ii]
+                                    expr = "%s * %s" % (lit(M[p][c]), src) if expr is None else \
+                                        "fma(%s, %s, %s)" % (lit(M[p][c]), src, expr)
+                            nxt.append(em.tmp(expr))
+                vals = nxt
+                dims[k] = npure
+            nsph = len(vals)
+            for k, v in enumerate(vals):
+                em.lines.append("    v[%d] = %s;" % ((3 * x + i) * nsph + k, v))
+    sets_body = em.lines
+
+    pem = Emitter()
+    vrr = Vrr(pem)
+    by = {}
+    for (w, e, f), k in acc.items():
+        by.setdefault((e, f), []).append((w, k))
+    for e, f in sorted(by, key=lambda t: (sum(t[0]), sum(t[1]), t)):
+        v = vrr.node(e, f, 0)
+        for w, k in sorted(by[(e, f)]):
+            if w == 0:
+                pem.lines.append("    I[%d] += %s;" % (k, v))
+            else:
+                pem.lines.append("    I[%d] = fma(w[%d], %s, I[%d]);" % (k, w - 1, v, k))
+    prim_body = vrr.factors() + pem.lines
+
+    s = ["template <>\nstruct DerivCls<%d, %d, %d, %d> {" % (la, lb, lc, ld),
+         "  static constexpr int kMmax = %d, kNacc = %d, kNsph = %d;" % (sum(ls) + 1, len(acc), nsph),
+         "  static constexpr int kN0 = %d, kN1 = %d, kN2 = %d, kN3 = %d;" %
+         tuple(2 * l + 1 if l >= 2 else ncart(l) for l in ls),
+         "  template <typename T>\n  static __device__ __forceinline__ void prim(const T* F, "
+         "const Geo<T>& g, const T* w, T* I) {"]
+    s += prim_body
+    s += ["  }", "  template <typename T>\n  static __device__ __forceinline__ void sets(const T* I, "
+          "const T* AB, const T* CD, T* v) {"]
+    s += sets_body
+    s += ["  }", "};"]
+    return "\n".join(s)
+
+
 def main():
     os.makedirs(GEN_DIR, exist_ok=True)
     classes = rk_classes(GRAD_MAX_L)
@@ -289,42 +401,51 @@ def main():
              "// Unrolled density weights, primitive stage and tail of the",
              "// register-resident gradient kernels (see gen_grad.py).",
              "#pragma once", '#include "../lgx_rk_common.cuh"', "", "namespace lgx {",
-             "namespace rk {", "", "template <int LA, int LB, int LC, int LD>", "struct GradCls;", ""]
+             "namespace rk {", "", "template <int LA, int LB, int LC, int LD>", "struct GradCls;",
+             "template <int LA, int LB, int LC, int LD>", "struct DerivCls;", ""]
     for c in classes:
         parts += [gen_class(*c), ""]
+    for c in rk_classes(DERIV_MAX_L):
+        parts += [gen_deriv_class(*c), ""]
     parts += ["}  // namespace rk", "}  // namespace lgx"]
     _write_if_changed(os.path.join(GEN_DIR, "grad_classes.cuh"), "\n".join(parts) + "\n")
 
     classes = sorted(classes, key=lambda c: -sum(c))
     names, decls = [], []
+    items = [("grad", c) for c in classes] + [("deriv", c) for c in rk_classes(DERIV_MAX_L)]
+    items.sort(key=lambda t: -sum(t[1]))
     for k in range(N_UNITS):
         name = "grad_unit_%02d.cu" % k
         names.append(name)
         lines = ["// GENERATED by libint_gb300/codegen/gen_grad.py -- do not edit.",
                  '#include "../lgx_rkgrad.cuh"', "", "namespace lgx {"]
-        for c in classes[k::N_UNITS]:
-            fn = "rk_grad_launch_%d%d%d%d" % c
-            decls.append((c, fn))
+        for kind, c in items[k::N_UNITS]:
+            fn = "rk_%s_launch_%d%d%d%d" % ((kind,) + c)
+            decls.append((kind, c, fn))
             lines.append("cudaError_t %s(const EriArgs& a, long long work, int nsm, "
                          "cudaStream_t st) {" % fn)
-            lines.append("  return rk_grad_launch_one<%d, %d, %d, %d>(a, work, nsm, st);" % c)
+            lines.append("  return rk_%s_launch_one<%d, %d, %d, %d>(a, work, nsm, st);" %
+                         ((kind,) + c))
             lines.append("}")
         lines.append("}  // namespace lgx")
         _write_if_changed(os.path.join(GEN_DIR, name), "\n".join(lines) + "\n")
     d = ["// GENERATED by libint_gb300/codegen/gen_grad.py -- do not edit.",
-         "// Run-time dispatch of the register-resident gradient kernels.",
+         "// Run-time dispatch of the register-resident derivative kernels.",
          '#include "../lgx_kernels.cuh"', "", "namespace lgx {"]
-    for _, fn in sorted(decls):
+    for _, _, fn in sorted(decls):
         d.append("cudaError_t %s(const EriArgs& a, long long work, int nsm, cudaStream_t st);" % fn)
-    d += ["", "cudaError_t rk_grad_launch(int la, int lb, int lc, int ld, const EriArgs& a, "
-          "long long work, int nsm,", "                           cudaStream_t st) {",
-          "  switch (((la * 8 + lb) * 8 + lc) * 8 + ld) {"]
-    for c, fn in sorted(decls):
-        d.append("    case %d: return %s(a, work, nsm, st);" %
-                 (((c[0] * 8 + c[1]) * 8 + c[2]) * 8 + c[3], fn))
-    d += ["  }", "  return cudaErrorNotSupported;", "}", "",
-          "bool rk_grad_available(int la, int lb, int lc, int ld) {",
-          "  return la + lb + lc + ld <= %d;" % GRAD_MAX_L, "}", "}  // namespace lgx"]
+    for name, lmax in (("grad", GRAD_MAX_L), ("deriv", DERIV_MAX_L)):
+        d += ["", "cudaError_t rk_%s_launch(int la, int lb, int lc, int ld, const EriArgs& a, "
+              "long long work, int nsm," % name, "                           cudaStream_t st) {",
+              "  switch (((la * 8 + lb) * 8 + lc) * 8 + ld) {"]
+        for kind, c, fn in sorted(decls):
+            if kind == name:
+                d.append("    case %d: return %s(a, work, nsm, st);" %
+                         (((c[0] * 8 + c[1]) * 8 + c[2]) * 8 + c[3], fn))
+        d += ["  }", "  return cudaErrorNotSupported;", "}", "",
+              "bool rk_%s_available(int la, int lb, int lc, int ld) {" % name,
+              "  return la <= 3 && lc <= 3 && la + lb + lc + ld <= %d;" % lmax, "}"]
+    d += ["}  // namespace lgx"]
     _write_if_changed(os.path.join(GEN_DIR, "grad_dispatch.cu"), "\n".join(d) + "\n")
     return names + ["grad_dispatch.cu"]
 

@@ -1,8 +1,17 @@
 // GENERATED by libint_gb300/codegen/gen_grad.py -- do not edit.
-// Run-time dispatch of the register-resident gradient kernels.
+// Run-time dispatch of the register-resident derivative kernels.
 #include "../lgx_kernels.cuh"
 
 namespace lgx {
+cudaError_t rk_deriv_launch_0000(const EriArgs& a, long long work, int nsm, cudaStream_t st);
+cudaError_t rk_deriv_launch_0010(const EriArgs& a, long long work, int nsm, cudaStream_t st);
+cudaError_t rk_deriv_launch_0011(const EriArgs& a, long long work, int nsm, cudaStream_t st);
+cudaError_t rk_deriv_launch_0020(const EriArgs& a, long long work, int nsm, cudaStream_t st);
+cudaError_t rk_deriv_launch_0021(const EriArgs& a, long long work, int nsm, cudaStream_t st);
+cudaError_t rk_deriv_launch_0030(const EriArgs& a, long long work, int nsm, cudaStream_t st);
+cudaError_t rk_deriv_launch_1010(const EriArgs& a, long long work, int nsm, cudaStream_t st);
+cudaError_t rk_deriv_launch_1011(const EriArgs& a, long long work, int nsm, cudaStream_t st);
+cudaError_t rk_deriv_launch_1020(const EriArgs& a, long long work, int nsm, cudaStream_t st);
 cudaError_t rk_grad_launch_0000(const EriArgs& a, long long work, int nsm, cudaStream_t st);
 cudaError_t rk_grad_launch_0010(const EriArgs& a, long long work, int nsm, cudaStream_t st);
 cudaError_t rk_grad_launch_0011(const EriArgs& a, long long work, int nsm, cudaStream_t st);
@@ -60,6 +69,26 @@ cudaError_t rk_grad_launch(int la, int lb, int lc, int ld, const EriArgs& a, lon
 }
 
 bool rk_grad_available(int la, int lb, int lc, int ld) {
-  return la + lb + lc + ld <= 5;
+  return la <= 3 && lc <= 3 && la + lb + lc + ld <= 5;
+}
+
+cudaError_t rk_deriv_launch(int la, int lb, int lc, int ld, const EriArgs& a, long long work, int nsm,
+                           cudaStream_t st) {
+  switch (((la * 8 + lb) * 8 + lc) * 8 + ld) {
+    case 0: return rk_deriv_launch_0000(a, work, nsm, st);
+    case 8: return rk_deriv_launch_0010(a, work, nsm, st);
+    case 9: return rk_deriv_launch_0011(a, work, nsm, st);
+    case 16: return rk_deriv_launch_0020(a, work, nsm, st);
+    case 17: return rk_deriv_launch_0021(a, work, nsm, st);
+    case 24: return rk_deriv_launch_0030(a, work, nsm, st);
+    case 520: return rk_deriv_launch_1010(a, work, nsm, st);
+    case 521: return rk_deriv_launch_1011(a, work, nsm, st);
+    case 528: return rk_deriv_launch_1020(a, work, nsm, st);
+  }
+  return cudaErrorNotSupported;
+}
+
+bool rk_deriv_available(int la, int lb, int lc, int ld) {
+  return la <= 3 && lc <= 3 && la + lb + lc + ld <= 3;
 }
 }  // namespace lgx

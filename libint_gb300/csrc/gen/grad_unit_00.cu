@@ -11,4 +11,10 @@ cudaError_t rk_grad_launch_0031(const EriArgs& a, long long work, int nsm, cudaS
 cudaError_t rk_grad_launch_0030(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<0, 0, 3, 0>(a, work, nsm, st);
 }
+cudaError_t rk_grad_launch_0020(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<0, 0, 2, 0>(a, work, nsm, st);
+}
+cudaError_t rk_deriv_launch_0000(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_deriv_launch_one<0, 0, 0, 0>(a, work, nsm, st);
+}
 }  // namespace lgx

@@ -11,4 +11,7 @@ cudaError_t rk_grad_launch_1030(const EriArgs& a, long long work, int nsm, cudaS
 cudaError_t rk_grad_launch_1020(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<1, 0, 2, 0>(a, work, nsm, st);
 }
+cudaError_t rk_deriv_launch_0011(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_deriv_launch_one<0, 0, 1, 1>(a, work, nsm, st);
+}
 }  // namespace lgx

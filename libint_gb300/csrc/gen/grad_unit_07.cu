@@ -8,6 +8,9 @@ cudaError_t rk_grad_launch_0022(const EriArgs& a, long long work, int nsm, cudaS
 cudaError_t rk_grad_launch_0021(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<0, 0, 2, 1>(a, work, nsm, st);
 }
+cudaError_t rk_grad_launch_0011(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_grad_launch_one<0, 0, 1, 1>(a, work, nsm, st);
+}
 cudaError_t rk_grad_launch_0000(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<0, 0, 0, 0>(a, work, nsm, st);
 }

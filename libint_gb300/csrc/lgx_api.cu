@@ -45,6 +45,9 @@ bool rk_available(bool fp32, int mode, bool att, int la, int lb, int lc, int ld)
 cudaError_t rk_grad_launch(int la, int lb, int lc, int ld, const EriArgs& a, long long work,
                            int nsm, cudaStream_t st);
 bool rk_grad_available(int la, int lb, int lc, int ld);
+cudaError_t rk_deriv_launch(int la, int lb, int lc, int ld, const EriArgs& a, long long work,
+                            int nsm, cudaStream_t st);
+bool rk_deriv_available(int la, int lb, int lc, int ld);
 cudaError_t launch_grad_sum(const double* copies, int ncopies, long long stride, int n, double* g,
                             cudaStream_t st);
 cudaError_t launch_jk_records(const PrimPairRec* pp, const int* src, long long n,
@@ -710,7 +713,9 @@ bool rk_eligible(const lgx_context* ctx, const BasisDev& B, const ProgDev& P, in
   const bool att = ctx->op != LGX_OP_COULOMB;  // attenuated: J/K register kernels only
   if (mode == kModeGrad)
     return !att && rk_grad_available(P.host.la, P.host.lb, P.host.lc, P.host.ld);
-  if (P.host.deriv != 0) return false;
+  if (P.host.deriv != 0)
+    return mode == kModeStore && !fp32 && !att &&
+           rk_deriv_available(P.host.la, P.host.lb, P.host.lc, P.host.ld);
   return rk_available(fp32, mode, att, P.host.la, P.host.lb, P.host.lc, P.host.ld);
 }
 
@@ -758,6 +763,11 @@ lgx_status run_rk(lgx_context* ctx, BasisDev& B, const ProgDev& P, int mode, boo
   if (mode == kModeGrad) {
     CK(rk_grad_launch(P.host.la, P.host.lb, P.host.lc, P.host.ld, a, nwork, ctx->nsm,
                       ctx->launch_stream ? ctx->launch_stream : ctx->stream));
+    return LGX_OK;
+  }
+  if (P.host.deriv != 0) {
+    CK(rk_deriv_launch(P.host.la, P.host.lb, P.host.lc, P.host.ld, a, nwork, ctx->nsm,
+                       ctx->launch_stream ? ctx->launch_stream : ctx->stream));
     return LGX_OK;
   }
   CK(rk_launch(fp32, mode, a.op != LGX_OP_COULOMB, P.host.la, P.host.lb, P.host.lc, P.host.ld, a,
@@ -942,9 +952,11 @@ void list_segments(const lgx_context* ctx, const BasisDev& B, int deriv, int mod
     const auto& sh = tab.shape[k / 2];
     ListSeg seg{sh[0], sh[1], sh[2], sh[3], (k & 1) != 0, at, count,
                 double(nqsum[k]) / double(count), 0};
-    const bool cut = ctx->use_rk && B.std_pure && deriv == 0 && mode == kModeStore && !seg.fp32 &&
-                     rk_available(false, mode, ctx->op != LGX_OP_COULOMB, seg.la, seg.lb, seg.lc,
-                                  seg.ld);
+    const bool att = ctx->op != LGX_OP_COULOMB;
+    const bool cut =
+        ctx->use_rk && B.std_pure && mode == kModeStore && !seg.fp32 &&
+        (deriv ? !att && rk_deriv_available(seg.la, seg.lb, seg.lc, seg.ld)
+               : rk_available(false, mode, att, seg.la, seg.lb, seg.lc, seg.ld));
     if (!cut) {
       plan.segs.push_back(seg);
     } else {

@@ -27,6 +27,44 @@ namespace lgx {
 // 2a_A V, 2a_B V, 2a_B S, 2a_D U, 2a_D S.
 constexpr int kGradSums = 11;
 
+// Prologue of one FP64 primitive quartet (the screening, Boys values and VRR
+// factors of rk_prim); false when screened out.
+template <int MMAX>
+__device__ __forceinline__ bool rk_prologue(const EriArgs& a, const RkQuartet<double>& q, int ib,
+                                            int ik, const PrimScreen& scr, double* F,
+                                            rk::Geo<double>& geo) {
+  const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
+  const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
+  if (!ln_kept(a, bp.fln_scr + kp.fln_scr, q.bra_pp + ib, q.ket_pp + ik, scr)) return false;
+  const double zeta = bp.zeta, eta = kp.zeta;
+  const double rs = rsqrt(zeta + eta);
+  const double pfac = bp.Kc * kp.Kc * rs;
+  // |pfac|, with the Conservative factor where the list is screened by it
+  if (a.screening == 1) {
+    const double mag = fabs(pfac) * fmax(1.0, double(bp.fnonsph) * double(kp.fnonsph)) *
+                       double(q.nbpp * q.nkpp);
+    if (mag < scr.prec) return false;
+  } else if ((__double_as_longlong(pfac) & 0x7fffffffffffffffll) <
+             __double_as_longlong(scr.prec)) {
+    return false;
+  }
+  const double oogpq = rs * rs;
+  const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1], PQz = bp.P[2] - kp.P[2];
+  const double ez = eta * oogpq, zz = zeta * oogpq;
+  const double T = zeta * ez * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
+  rk_boys<MMAX>(a.boys_tay, T, pfac, F);
+  geo.PAx = bp.P[0] - q.A[0]; geo.PAy = bp.P[1] - q.A[1]; geo.PAz = bp.P[2] - q.A[2];
+  geo.QCx = kp.P[0] - q.C[0]; geo.QCy = kp.P[1] - q.C[1]; geo.QCz = kp.P[2] - q.C[2];
+  geo.WPx = -ez * PQx; geo.WPy = -ez * PQy; geo.WPz = -ez * PQz;
+  geo.WQx = zz * PQx; geo.WQy = zz * PQy; geo.WQz = zz * PQz;
+  geo.oo2z = 0.5 * bp.oog;
+  geo.roz = ez;
+  geo.oo2e = 0.5 * kp.oog;
+  geo.roe = zz;
+  geo.oo2ze = 0.5 * oogpq;
+  return true;
+}
+
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
   using C = rk::GradCls<LA, LB, LC, LD>;
@@ -107,52 +145,29 @@ __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
     int ib = g / q.nkpp, ik = g - ib * q.nkpp;
     const int gb = G / q.nkpp, gk = G - gb * q.nkpp;
     for (int p = g; p < nq; p += G) {
-      const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
-      const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
-      bool keep = ln_kept(a, bp.fln_scr + kp.fln_scr, q.bra_pp + ib, q.ket_pp + ik, scr);
-      if (keep) {
-        const double zeta = bp.zeta, eta = kp.zeta;
-        const double rs = rsqrt(zeta + eta);
-        const double pfac = bp.Kc * kp.Kc * rs;
-        keep = (__double_as_longlong(pfac) & 0x7fffffffffffffffll) >=
-               __double_as_longlong(scr.prec);
-        if (keep) {
-          const double oogpq = rs * rs;
-          const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1],
-                       PQz = bp.P[2] - kp.P[2];
-          const double ez = eta * oogpq, zz = zeta * oogpq;
-          const double T = zeta * ez * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
-          double F[C::kMmax + 1];
-          rk_boys<C::kMmax>(a.boys_tay, T, pfac, F);
-          rk::Geo<double> geo;
-          geo.PAx = bp.P[0] - q.A[0]; geo.PAy = bp.P[1] - q.A[1]; geo.PAz = bp.P[2] - q.A[2];
-          geo.QCx = kp.P[0] - q.C[0]; geo.QCy = kp.P[1] - q.C[1]; geo.QCz = kp.P[2] - q.C[2];
-          geo.WPx = -ez * PQx; geo.WPy = -ez * PQy; geo.WPz = -ez * PQz;
-          geo.WQx = zz * PQx; geo.WQy = zz * PQy; geo.WQz = zz * PQz;
-          geo.oo2z = 0.5 * bp.oog;
-          geo.roz = ez;
-          geo.oo2e = 0.5 * kp.oog;
-          geo.roe = zz;
-          geo.oo2ze = 0.5 * oogpq;
-          double s[14];
-          C::template prim<double>(F, geo, WJ, WK, s, I);
-          const double wa = 2.0 * (q.bsw ? bp.a2 : bp.a1), wb = 2.0 * (q.bsw ? bp.a1 : bp.a2);
-          const double wd = 2.0 * (q.ksw ? kp.a1 : kp.a2);
+      double F[C::kMmax + 1];
+      rk::Geo<double> geo;
+      if (rk_prologue<C::kMmax>(a, q, ib, ik, scr, F, geo)) {
+        ++kept;
+        double s[14];
+        C::template prim<double>(F, geo, WJ, WK, s, I);
+        const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
+        const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
+        const double wa = 2.0 * (q.bsw ? bp.a2 : bp.a1), wb = 2.0 * (q.bsw ? bp.a1 : bp.a2);
+        const double wd = 2.0 * (q.ksw ? kp.a1 : kp.a2);
 #pragma unroll
-          for (int x = 0; x < kSets; ++x) {
-            const double* sx = s + 7 * x;
+        for (int x = 0; x < kSets; ++x) {
+          const double* sx = s + 7 * x;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-              acc[x][i] = fma(wa, sx[1 + i], acc[x][i]);
-              acc[x][3 + i] = fma(wb, sx[1 + i], acc[x][3 + i]);
-              acc[x][7 + i] = fma(wd, sx[4 + i], acc[x][7 + i]);
-            }
-            acc[x][6] = fma(wb, sx[0], acc[x][6]);
-            acc[x][10] = fma(wd, sx[0], acc[x][10]);
+          for (int i = 0; i < 3; ++i) {
+            acc[x][i] = fma(wa, sx[1 + i], acc[x][i]);
+            acc[x][3 + i] = fma(wb, sx[1 + i], acc[x][3 + i]);
+            acc[x][7 + i] = fma(wd, sx[4 + i], acc[x][7 + i]);
           }
+          acc[x][6] = fma(wb, sx[0], acc[x][6]);
+          acc[x][10] = fma(wd, sx[0], acc[x][10]);
         }
       }
-      kept += keep ? 1 : 0;
       ib += gb;
       ik += gk;
       if (ik >= q.nkpp) {
@@ -208,10 +223,103 @@ __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
   if (a.prim_count && my_prims) atomicAdd(a.prim_count, my_prims);
 }
 
+// First-derivative shell sets of an explicit list, G lanes per quartet: the
+// accumulators of gen_grad.py's DerivCls in registers, the twelve sets written
+// in the caller's order (centre C by translational invariance).
+//
+// What bounds it: the FP64 pipe; the program kernel it replaces left most lanes
+// of a level idle in these classes, whose primitive quartets are the many (a
+// water dimer in cc-pVDZ: 8 of 10 ms).  It ends at L = 3: from (pp|pp) on the
+// accumulators (540 there) no longer fit the registers, and few primitive
+// quartets are left.
 template <int LA, int LB, int LC, int LD>
-cudaError_t rk_grad_launch_one(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+__global__ void __launch_bounds__(128, 2) rk_deriv_kernel(EriArgs a) {
+  using C = rk::DerivCls<LA, LB, LC, LD>;
+  constexpr int N0 = C::kN0, N1 = C::kN1, N2 = C::kN2, N3 = C::kN3, N = C::kNsph;
+  const int G = a.group;
+  const int lane = threadIdx.x & 31;
+  const int g = lane & (G - 1);
+  const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
+  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const long long step = ((long long)gridDim.x * blockDim.x) / G;
+  PrimScreen scr;
+  scr.prec = a.precision;
+  scr.ln_prec = a.ln_prec;
+  scr.fprec = a.fprecision;
+  scr.fln_prec = a.fln_prec;
+  for (long long qi = first; qi < a.nitems; qi += step) {
+    const QuartetItem it = a.items[qi];
+    RkQuartet<double> q;
+    rk_load<double>(a, it.bra_pair, it.ket_pair, it.flags & 1, (it.flags >> 1) & 1, q);
+    double I[C::kNacc];
+#pragma unroll
+    for (int i = 0; i < C::kNacc; ++i) I[i] = 0.0;
+    const int nq = q.nbpp * q.nkpp;
+    int kept = 0;
+    int ib = g / q.nkpp, ik = g - ib * q.nkpp;
+    const int gb = G / q.nkpp, gk = G - gb * q.nkpp;
+    for (int p = g; p < nq; p += G) {
+      double F[C::kMmax + 1];
+      rk::Geo<double> geo;
+      if (rk_prologue<C::kMmax>(a, q, ib, ik, scr, F, geo)) {
+        ++kept;
+        const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
+        const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
+        const double w[3] = {2.0 * (q.bsw ? bp.a2 : bp.a1), 2.0 * (q.bsw ? bp.a1 : bp.a2),
+                             2.0 * (q.ksw ? kp.a1 : kp.a2)};
+        C::template prim<double>(F, geo, w, I);
+      }
+      ib += gb;
+      ik += gk;
+      if (ik >= q.nkpp) {
+        ik -= q.nkpp;
+        ++ib;
+      }
+    }
+    for (int o = G >> 1; o > 0; o >>= 1) {
+#pragma unroll
+      for (int i = 0; i < C::kNacc; ++i) I[i] += rk_shfl_xor<double>(gmask, I[i], o, G);
+      kept += __shfl_xor_sync(gmask, kept, o, G);
+    }
+    if (a.is_null && g == 0) a.is_null[it.pad] = kept == 0 ? 1 : 0;
+    if (kept == 0) continue;
+    double v[9 * N];
+    C::template sets<double>(I, q.AB, q.CD, v);
+    const int fl = it.flags >> 2;
+    const bool sbk = fl & 1, stb = (fl >> 1) & 1, stk = (fl >> 2) & 1;
+    // canonical position -> caller position, and the strides there
+    const int perm[4] = {sbk ? (stk ? 3 : 2) : (stb ? 1 : 0), sbk ? (stk ? 2 : 3) : (stb ? 0 : 1),
+                         sbk ? (stb ? 1 : 0) : (stk ? 3 : 2), sbk ? (stb ? 0 : 1) : (stk ? 2 : 3)};
+    const int dims[4] = {N0, N1, N2, N3};
+    int str[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      str[t] = 1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (perm[u] > perm[t]) str[t] *= dims[u];
+    }
+    double* o = a.out + it.out;
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      if ((e & (G - 1)) != g) continue;
+      double* oe = o + (e / (N1 * N2 * N3)) * str[0] + ((e / (N2 * N3)) % N1) * str[1] +
+                   ((e / N3) % N2) * str[2] + (e % N3) * str[3];
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        const double dA = v[s * N + e], dB = v[(3 + s) * N + e], dD = v[(6 + s) * N + e];
+        oe[(size_t)(perm[0] * 3 + s) * N] = dA;
+        oe[(size_t)(perm[1] * 3 + s) * N] = dB;
+        oe[(size_t)(perm[2] * 3 + s) * N] = -(dA + dB + dD);
+        oe[(size_t)(perm[3] * 3 + s) * N] = dD;
+      }
+    }
+  }
+}
+
+template <class K>
+cudaError_t rk_deriv_launch_any(K k, const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   const int block = 128;
-  auto k = rk_grad_kernel<LA, LB, LC, LD>;
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, block, 0) != cudaSuccess || occ < 1)
     occ = 1;
@@ -219,6 +327,16 @@ cudaError_t rk_grad_launch_one(const EriArgs& a, long long work, int nsm, cudaSt
   const long long grid = std::max(1LL, std::min((long long)nsm * occ, need));
   k<<<(unsigned)grid, block, 0, st>>>(a);
   return cudaGetLastError();
+}
+
+template <int LA, int LB, int LC, int LD>
+cudaError_t rk_grad_launch_one(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_deriv_launch_any(rk_grad_kernel<LA, LB, LC, LD>, a, work, nsm, st);
+}
+
+template <int LA, int LB, int LC, int LD>
+cudaError_t rk_deriv_launch_one(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_deriv_launch_any(rk_deriv_kernel<LA, LB, LC, LD>, a, work, nsm, st);
 }
 
 }  // namespace lgx

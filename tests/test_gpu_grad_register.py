@@ -45,3 +45,26 @@ def test_register_gradients_vs_program_kernel(lgx, monkeypatch, ls, depth):
     assert st.prim_quartets == rst.prim_quartets
     assert np.max(np.abs(gJ - rJ)) < 1e-11 * np.max(np.abs(rJ))
     assert np.max(np.abs(gK - rK)) < 1e-11 * np.max(np.abs(rK))
+
+
+@pytest.mark.parametrize("n", [150, 3000, 9000])
+def test_register_derivative_sets_vs_program_kernel(lgx, monkeypatch, n):
+    # every order of shells up to f; block, host- and GPU-classified list sizes
+    rng = np.random.default_rng(7)
+    shells = []
+    for l, k in [(0, 5), (1, 3), (2, 1), (0, 1), (3, 1), (1, 1), (2, 2), (3, 2)]:
+        ex = np.exp(rng.uniform(np.log(0.2), np.log(8.0), k))
+        shells.append(lgx.Shell(l, list(zip(ex, rng.uniform(0.2, 1.0, k))),
+                                rng.uniform(-1.5, 1.5, 3), pure=l > 1))
+    bs = lgx.BasisSet(shells)
+    q = rng.integers(0, len(bs), (n, 4)).astype(np.int32)
+    res = []
+    for off in ("0", "1"):
+        monkeypatch.setenv("LGX_DISABLE_RK", off)
+        ctx = lgx.Context(0)
+        ctx.set_basis(bs)
+        res.append(ctx.compute_batch(q, 1))
+        ctx.close()
+    (a, _, na), (b, _, nb) = res
+    assert np.array_equal(na, nb)
+    assert np.max(np.abs(a - b)) < 1e-11 * np.max(np.abs(b))
