@@ -221,7 +221,7 @@ struct lgx_context {
   // enqueued (the FP32 branch has its own scratch).
   static constexpr int kMaxBranches = 4;  // streams per precision
   bool overlap = true;
-  int branches = 3;
+  int branches = 4;
   // 0: longest first onto the least-loaded branch, issued longest first;
   // 1: round-robin in bin order (default: best or level on (H2O)32 cc-pVDZ,
   // (H2O)8 and (H2O)64 cc-pVTZ); 2: as 0 but issued in bin order
@@ -1129,18 +1129,39 @@ lgx_status run_list(lgx_context* ctx, BasisDev& B, const ListPlan& plan, int der
   // joined back into ctx->stream, one work counter and one program-kernel
   // slot scratch per launch / branch): a short list, such as the raised and
   // lowered quartets of a second-derivative set, then costs its slowest
-  // class rather than the sum of its classes
+  // class rather than the sum of its classes.  The launches with the longest
+  // chains go first, over all eight streams: one lane's or warp's serial FP64
+  // work (64 cycles per warp instruction and scheduler), not the total, sets
+  // the time of most launches of a list.
   const int ng = int(plan.segs.size());
-  const int nbr = std::min(ng, lgx_context::kMaxBranches);
+  constexpr int kStreams = 2 * lgx_context::kMaxBranches;
+  const int nbr = std::min(ng, kStreams);
   const bool split = ctx->overlap && nbr > 1;
   CK(ctx->xcounters.ensure(size_t(ng) * sizeof(unsigned long long)));
   CK(cudaMemsetAsync(ctx->xcounters.p, 0, size_t(ng) * sizeof(unsigned long long), ctx->stream));
+  std::vector<ProgDev*> progs(ng, nullptr);
+  std::vector<double> est(ng, 0.0);
+  std::vector<int> order(ng);
+  for (int i = 0; i < ng; ++i) {
+    const ListSeg& seg = plan.segs[i];
+    lgx_status s = get_prog(ctx, seg.la, seg.lb, seg.lc, seg.ld, deriv, &progs[i]);
+    if (s != LGX_OK) return s;
+    const ClassProgramHost& H = progs[i]->host;
+    const double prim = 60.0 + 0.5 * double(H.vrr_flops), post = 0.5 * double(H.post_flops);
+    // operations of one warp, and the warps each scheduler runs in turn
+    const double lanes = seg.group > 0 ? seg.group : 8.0;
+    const double chain = seg.group > 0 ? seg.nq / lanes * prim + post : (seg.nq * prim + post) / lanes;
+    const double warps = seg.group > 0 ? double(seg.count) * seg.group / 32.0 : double(seg.count);
+    est[i] = chain * std::max(1.0, warps / (4.0 * ctx->nsm)) * (seg.fp32 ? 0.1 : 1.0);
+    order[i] = i;
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return est[x] > est[y]; });
+  auto stream = [&](int b) {
+    return b < lgx_context::kMaxBranches ? ctx->s64[b] : ctx->s32[b - lgx_context::kMaxBranches];
+  };
   if (split) {
     CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
-    for (int b = 0; b < nbr; ++b) {
-      CK(cudaStreamWaitEvent(ctx->s64[b], ctx->ev_fork, 0));
-      CK(cudaStreamWaitEvent(ctx->s32[b], ctx->ev_fork, 0));
-    }
+    for (int b = 0; b < nbr; ++b) CK(cudaStreamWaitEvent(stream(b), ctx->ev_fork, 0));
   }
   struct Restore {  // launch stream / scratch back to the context defaults
     lgx_context* c;
@@ -1149,17 +1170,14 @@ lgx_status run_list(lgx_context* ctx, BasisDev& B, const ListPlan& plan, int der
       c->scratch = nullptr;
     }
   } restore{ctx};
-  size_t gi = 0;
   lgx_status s = LGX_OK;
-  for (const ListSeg& seg : plan.segs) {
-    ProgDev* P = nullptr;
-    s = get_prog(ctx, seg.la, seg.lb, seg.lc, seg.ld, deriv, &P);
-    if (s != LGX_OK) break;
+  for (int gi = 0; gi < ng; ++gi) {
+    const ListSeg& seg = plan.segs[order[gi]];
     const bool fp32 = seg.fp32;
     if (split) {
-      const int b = int(gi) % nbr;
-      ctx->launch_stream = fp32 ? ctx->s32[b] : ctx->s64[b];
-      ctx->scratch = (fp32 || b > 0) ? &ctx->gscratch_br[(fp32 ? nbr : 0) + b] : &ctx->gscratch;
+      const int b = gi % nbr;
+      ctx->launch_stream = stream(b);
+      ctx->scratch = b > 0 ? &ctx->gscratch_br[b] : &ctx->gscratch;
     }
     EriArgs a{};
     a.counter = ctx->xcounters.as<unsigned long long>() + gi;
@@ -1173,17 +1191,14 @@ lgx_status run_list(lgx_context* ctx, BasisDev& B, const ListPlan& plan, int der
     a.is_null = d_isnull;
     a.kschwarz = d_kschwarz;
     const Variant v{0, seg.group, 0};
-    s = run_eri(ctx, B, *P, fp32 ? mode32 : mode, fp32, a, a.nitems, seg.nq,
+    s = run_eri(ctx, B, *progs[order[gi]], fp32 ? mode32 : mode, fp32, a, a.nitems, seg.nq,
                 seg.group > 0 ? &v : nullptr);
     if (s != LGX_OK) break;
-    ++gi;
   }
   if (split) {  // joined on every path, so ctx->stream orders after all branch work
     for (int b = 0; b < nbr; ++b) {
-      CK(cudaEventRecord(ctx->ev_join[2 * b], ctx->s64[b]));
-      CK(cudaEventRecord(ctx->ev_join[2 * b + 1], ctx->s32[b]));
-      CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join[2 * b], 0));
-      CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join[2 * b + 1], 0));
+      CK(cudaEventRecord(ctx->ev_join[b], stream(b)));
+      CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join[b], 0));
     }
   }
   return s;
@@ -1594,7 +1609,13 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
   // FP32 launches run beside FP64-pipe-bound ones.
   const bool split = ctx->overlap && !ctx->noalloc && nlaunch > 1;
   pr.split = split;
-  const int nbr = std::max(1, std::min(ctx->branches, lgx_context::kMaxBranches));
+  // A pass of one precision spreads over both precisions' streams.
+  const bool two = mode32 >= 0;
+  const int nhalf = std::max(1, std::min(ctx->branches, lgx_context::kMaxBranches));
+  const int nbr = two ? nhalf : 2 * nhalf;
+  auto stream = [&](bool fp32, int b) {
+    return fp32 ? ctx->s32[b] : (b < nhalf ? ctx->s64[b] : ctx->s32[b - nhalf]);
+  };
   if (split && ctx->branch_policy == 1) {  // round-robin in bin order
     int nxt[2] = {0, 0};
     for (auto& j : jobs) j.branch = nxt[j.fp32 ? 1 : 0]++ % nbr;
@@ -1603,7 +1624,7 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
     for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
     std::stable_sort(ord.begin(), ord.end(),
                      [&](size_t x, size_t y) { return jobs[x].est > jobs[y].est; });
-    double load[2][lgx_context::kMaxBranches] = {};
+    double load[2][2 * lgx_context::kMaxBranches] = {};
     for (size_t i : ord) {
       Job& j = jobs[i];
       double* l = load[j.fp32 ? 1 : 0];
@@ -1644,7 +1665,7 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
   CK(cudaEventRecordWithFlags(ctx->ev0, ctx->stream, evflags));
   if (split) {
     CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
-    for (int b = 0; b < nbr; ++b) {
+    for (int b = 0; b < nhalf; ++b) {
       CK(cudaStreamWaitEvent(ctx->s64[b], ctx->ev_fork, 0));
       CK(cudaStreamWaitEvent(ctx->s32[b], ctx->ev_fork, 0));
     }
@@ -1676,9 +1697,9 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
     cudaStream_t st = ctx->stream;
     if (split) {
       const int b = j.branch;
-      st = fp32 ? ctx->s32[b] : ctx->s64[b];
+      st = stream(fp32, b);
       // program-kernel slot scratch: one region per branch
-      ctx->scratch = (fp32 || b > 0) ? &ctx->gscratch_br[(fp32 ? nbr : 0) + b] : &ctx->gscratch;
+      ctx->scratch = (fp32 || b > 0) ? &ctx->gscratch_br[(fp32 ? nhalf : 0) + b] : &ctx->gscratch;
       if (!fp32 && mode32 >= 0) a.max_bps = ctx->fp64_bps;
       if (fp32) a.max_bps = ctx->fp32_bps;
     }
@@ -1693,7 +1714,7 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
     pr.recs.push_back({int(j.bi), sp, fp32, v, kmode});
   }
   if (split) {
-    for (int b = 0; b < nbr; ++b) {
+    for (int b = 0; b < nhalf; ++b) {
       CK(cudaEventRecord(ctx->ev_join[2 * b], ctx->s64[b]));
       CK(cudaEventRecord(ctx->ev_join[2 * b + 1], ctx->s32[b]));
       CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join[2 * b], 0));
