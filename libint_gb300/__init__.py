@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import enum
+import math
 import os
 from typing import Iterable, Sequence
 
@@ -155,14 +156,15 @@ class Shell:
 
     def _c(self) -> _lgx.LgxShell:
         r = _lgx.LgxShell()
-        r.l = self.l
-        r.pure = 1 if self.pure else 0
-        r.nprim = len(self.alpha)
-        for x in range(3):
-            r.origin[x] = self.O[x]
-        r.alpha = _lgx.ptr(self.alpha)
-        r.coeff = _lgx.ptr(self.coeff)
+        self._pack(r, 0)
         return r
+
+    def _pack(self, arr, k: int):
+        """Writes the shell into entry k of an array of LgxShell."""
+        x, y, z = self.O.tolist()
+        _lgx.SHELL_STRUCT.pack_into(arr, k * _lgx.SHELL_STRUCT.size, self.l,
+                                    1 if self.pure else 0, len(self.alpha), 0, x, y, z,
+                                    _lgx.address(self.alpha), _lgx.address(self.coeff))
 
     def __repr__(self):
         return "Shell(l=%d, pure=%s, nprim=%d, O=%s)" % (self.l, self.pure, self.nprim(),
@@ -346,27 +348,31 @@ class Context:
         """One shell set (list of nsets arrays, or None when fully screened).
         pair_ln_prec: None, or (bra, ket) ln_prec of caller-precomputed
         ShellPair data (lgx_compute_shellset_pairs; deriv 0 or 1)."""
-        arr = (_lgx.LgxShell * 4)(*[s._c() for s in shells])
+        arr = (_lgx.LgxShell * 4)()
+        for k, s in enumerate(shells):
+            s._pack(arr, k)
         nsets = {0: 1, 1: 12, 2: 78}[int(deriv)]
-        nv = int(np.prod([s.size() for s in shells]))
-        out = np.zeros(nsets * nv)
+        shape = tuple([s.size() for s in shells])
+        nv = math.prod(shape)
+        out = np.empty(nsets * nv)
         ns, nvals, isnull = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         if pair_ln_prec is None:
             st = self._lib.lgx_compute_shellset(self._h, arr, int(deriv), float(precision),
-                                                int(screening), _lgx.ptr(out), out.size,
+                                                int(screening), _lgx.address(out), out.size,
                                                 ctypes.byref(ns), ctypes.byref(nvals),
                                                 ctypes.byref(isnull))
         else:
             pl = np.asarray(pair_ln_prec, dtype=np.float64).reshape(2)
             st = self._lib.lgx_compute_shellset_pairs(self._h, arr, int(deriv), float(precision),
                                                       int(screening), _lgx.ptr(pl),
-                                                      _lgx.ptr(out), out.size, ctypes.byref(ns),
-                                                      ctypes.byref(nvals), ctypes.byref(isnull))
-        self._check(st, "lgx_compute_shellset")
+                                                      _lgx.address(out), out.size,
+                                                      ctypes.byref(ns), ctypes.byref(nvals),
+                                                      ctypes.byref(isnull))
+        if st != _lgx.LGX_OK:
+            self._check(st, "lgx_compute_shellset")
         if isnull.value:
             return None
-        shape = tuple(s.size() for s in shells)
-        return [out[i * nv:(i + 1) * nv].reshape(shape) for i in range(ns.value)]
+        return list(out.reshape((nsets,) + shape))
 
     def compute_primitive_set(self, ls, prims, AB, CD, deriv=0):
         """Contracted Cartesian shell set(s) (l1 l2|l3 l4) from caller-computed
@@ -636,10 +642,11 @@ class Engine:
         ctx.set_operator(self.oper, self._omega)  # contexts are shared between engines
         r = ctx.compute_shellset(full, self.deriv_order, self._precision, self.screening)
         if r is not None:
-            shape = tuple(s.size() for s in shells)
-            sel = [0] if self.deriv_order == 0 else (
-                _DERIV_SETS[rank] if self.deriv_order == 1 else range(78))
-            r = [r[i].reshape(shape) for i in sel]
+            if rank != 4:
+                shape = tuple(s.size() for s in shells)
+                sel = [0] if self.deriv_order == 0 else (
+                    _DERIV_SETS[rank] if self.deriv_order == 1 else range(78))
+                r = [r[i].reshape(shape) for i in sel]
         self._results = r if r is not None else [None] * self.nshellsets()
         if r is None:
             return None

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 
 from . import build as _build
 
@@ -39,6 +40,10 @@ class LgxShell(ctypes.Structure):
     _fields_ = [("l", ctypes.c_int32), ("pure", ctypes.c_int32),
                 ("nprim", ctypes.c_int32), ("pad_", ctypes.c_int32),
                 ("origin", ctypes.c_double * 3), ("alpha", _dp), ("coeff", _dp)]
+
+
+SHELL_STRUCT = struct.Struct("@4i3d2P")  # LgxShell
+assert SHELL_STRUCT.size == ctypes.sizeof(LgxShell)
 
 
 class LgxJkStats(ctypes.Structure):
@@ -97,13 +102,13 @@ SIGNATURES = {
     "lgx_version": (ctypes.c_char_p, []),
     "lgx_compute_shellset": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(LgxShell),
                                             ctypes.c_int, ctypes.c_double, ctypes.c_int,
-                                            _dp, ctypes.c_size_t,
+                                            ctypes.c_void_p, ctypes.c_size_t,
                                             ctypes.POINTER(ctypes.c_int),
                                             ctypes.POINTER(ctypes.c_int),
                                             ctypes.POINTER(ctypes.c_int)]),
     "lgx_compute_shellset_pairs": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(LgxShell),
                                                   ctypes.c_int, ctypes.c_double, ctypes.c_int,
-                                                  _dp, _dp, ctypes.c_size_t,
+                                                  _dp, ctypes.c_void_p, ctypes.c_size_t,
                                                   ctypes.POINTER(ctypes.c_int),
                                                   ctypes.POINTER(ctypes.c_int),
                                                   ctypes.POINTER(ctypes.c_int)]),
@@ -188,6 +193,11 @@ def check(status: int, ctx=None, what: str = ""):
         if ctx is not None:
             msg = (what + ": " if what else "") + load().lgx_last_error(ctx).decode()
         raise LgxError(status, msg)
+
+
+def address(a) -> int:
+    """Address of an array's data (ptr without the ctypes objects)."""
+    return a.__array_interface__["data"][0]
 
 
 def ptr(a, ct=ctypes.c_double):

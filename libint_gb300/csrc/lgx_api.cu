@@ -104,13 +104,17 @@ struct BasisDev {
   int nshell = 0, nprim_total = 0, nbf = 0, natoms = 0;
   std::vector<int> l, pure, nprim, prim_off, bf_off, atom;
   std::vector<double> O, alpha, coeff;
-  DBuf ints, dbls, flts;
+  DBuf blob;  // every array of the basis and its pair table, one upload
+  const PairRec* dpairs = nullptr;
+  const int* dpp_pair = nullptr;
+  const unsigned char* dpair_swap = nullptr;
+  const QuartetItem* ditem = nullptr;  // work item of the quartet (0 1|2 3)
   DevBasis dev{};
   // pairs
   std::vector<PairRec> hpairs;
   std::vector<unsigned char> hswap;
   long long npp = 0;
-  DBuf pairs, pprims, ppds, pp_pair, pair_swap;
+  DBuf pprims, ppds;
   bool pairs_ok = false;
   unsigned long long pairs_version = 0;  // bumped whenever pprims is rewritten
   double pairs_lnprec = 0;
@@ -151,6 +155,8 @@ struct BinCache {
 };
 
 }  // namespace
+
+constexpr size_t kPinIn = 128 * 1024, kPinOut = 512 * 1024;
 
 // Launch variant of one class bin: the register kernel with G lanes per
 // quartet, or the program kernel with interpreted or generated post stage
@@ -263,6 +269,11 @@ struct lgx_context {
   double omega = 0.0;
   BasisDev basis, small;
   DBuf gscratch, counter, errflag, primcount;
+  // pinned host memory of the single-shell-set calls: [0, kPinIn) the shells
+  // going up, then results coming back; pin_busy: an upload from it may still
+  // be under way
+  unsigned char* pin = nullptr;
+  bool pin_busy = false;
   DBuf items, out, isnull;
   DBuf list_in, list_keys, list_cnt, list_tab;  // explicit lists classified on the GPU
   DBuf Jacc, Kacc, Dd, Jd, Kd, gsum, gcopies;  // gradients: sum and per-SM copies
@@ -469,6 +480,33 @@ lgx_status get_prog(lgx_context* ctx, int la, int lb, int lc, int ld, int deriv,
   return LGX_OK;
 }
 
+// Canonical quartet (engine.impl.h:1181-1211) -> work item.
+struct Canon {
+  int c[4];  // canonical shells
+  int flags;
+  int la, lb, lc, ld;
+};
+Canon canonicalize(const BasisDev& B, const int* s) {
+  const int l0 = B.l[s[0]], l1 = B.l[s[1]], l2 = B.l[s[2]], l3 = B.l[s[3]];
+  const bool stb = l0 < l1, stk = l2 < l3, sbk = l0 + l1 > l2 + l3;
+  int perm[4];
+  perm[0] = sbk ? (stk ? 3 : 2) : (stb ? 1 : 0);
+  perm[1] = sbk ? (stk ? 2 : 3) : (stb ? 0 : 1);
+  perm[2] = sbk ? (stb ? 1 : 0) : (stk ? 3 : 2);
+  perm[3] = sbk ? (stb ? 0 : 1) : (stk ? 2 : 3);
+  Canon q;
+  for (int k = 0; k < 4; ++k) q.c[k] = s[perm[k]];
+  const bool bsw = q.c[0] < q.c[1];  // stored pair has s1 >= s2
+  const bool ksw = q.c[2] < q.c[3];
+  q.flags = (bsw ? 1 : 0) | (ksw ? 2 : 0) |
+            ((sbk ? 1 : 0) | (stb ? 2 : 0) | (stk ? 4 : 0)) << 2;
+  q.la = B.l[q.c[0]];
+  q.lb = B.l[q.c[1]];
+  q.lc = B.l[q.c[2]];
+  q.ld = B.l[q.c[3]];
+  return q;
+}
+
 // ---------------------------------------------------------------- basis
 // lmax: LGX_MAX_L for callers' bases; one more for the Cartesian raised
 // shells of the second-derivative composition.
@@ -508,47 +546,6 @@ lgx_status upload_basis(lgx_context* ctx, BasisDev& B, int nshell, const int32_t
   B.O.assign(origins, origins + 3 * nshell);
   B.alpha.assign(alpha, alpha + np);
   B.coeff.assign(coeff, coeff + np);
-  // device copies: ints [l|pure|nprim|prim_off|bf_off|atom], doubles [O|alpha|coeff]
-  std::vector<int> hi;
-  hi.reserve(6 * nshell);
-  for (auto* v : {&B.l, &B.pure, &B.nprim, &B.prim_off, &B.bf_off, &B.atom})
-    hi.insert(hi.end(), v->begin(), v->end());
-  std::vector<double> hd;
-  hd.reserve(3 * nshell + 2 * np);
-  hd.insert(hd.end(), B.O.begin(), B.O.end());
-  hd.insert(hd.end(), B.alpha.begin(), B.alpha.end());
-  hd.insert(hd.end(), B.coeff.begin(), B.coeff.end());
-  CK(B.ints.ensure(hi.size() * sizeof(int)));
-  CK(B.dbls.ensure(hd.size() * sizeof(double)));
-  CK(cudaMemcpyAsync(B.ints.p, hi.data(), hi.size() * sizeof(int), cudaMemcpyHostToDevice,
-                     ctx->stream));
-  CK(cudaMemcpyAsync(B.dbls.p, hd.data(), hd.size() * sizeof(double), cudaMemcpyHostToDevice,
-                     ctx->stream));
-  const int* ib = B.ints.as<int>();
-  const double* db = B.dbls.as<double>();
-  B.dev.nshell = nshell;
-  B.dev.l = ib;
-  B.dev.pure = ib + nshell;
-  B.dev.nprim = ib + 2 * nshell;
-  B.dev.prim_off = ib + 3 * nshell;
-  B.dev.bf_off = ib + 4 * nshell;
-  B.dev.atom = ib + 5 * nshell;
-  B.dev.O = db;
-  B.dev.alpha = db + 3 * nshell;
-  B.dev.coeff = db + 3 * nshell + np;
-  {
-    std::vector<float> hf(6 * size_t(nshell));
-    for (int i = 0; i < 3 * nshell; ++i) {
-      const float hi = float(B.O[i]);
-      hf[i] = hi;
-      hf[3 * nshell + i] = float(B.O[i] - double(hi));
-    }
-    CK(B.flts.ensure(hf.size() * sizeof(float)));
-    CK(cudaMemcpyAsync(B.flts.p, hf.data(), hf.size() * sizeof(float), cudaMemcpyHostToDevice,
-                       ctx->stream));
-    B.dev.Ohi = B.flts.as<float>();
-    B.dev.Olo = B.flts.as<float>() + 3 * nshell;
-  }
   B.pairs_ok = false;
   B.schwarz_ok = false;
   // pair table layout (all s1 >= s2)
@@ -569,21 +566,85 @@ lgx_status upload_basis(lgx_context* ctx, BasisDev& B, int nshell, const int32_t
   if (off > std::numeric_limits<int>::max())
     return fail(ctx, LGX_ERR_TOO_LARGE, "too many primitive pairs");
   B.npp = off;
-  std::vector<int> ppp(off);
-  for (long long p = 0; p < npairs; ++p)
-    for (int k = 0; k < B.hpairs[p].npp; ++k) ppp[B.hpairs[p].pp_off + k] = int(p);
-  CK(B.pairs.ensure(npairs * sizeof(PairRec)));
-  CK(B.pp_pair.ensure(off * sizeof(int)));
+  // One device blob and one copy: doubles [O|alpha|coeff], pair records, ints
+  // [l|pure|nprim|prim_off|bf_off|atom], floats [Ohi|Olo], pair of each
+  // primitive pair, pair swaps, and the item of the quartet of shells 0-3.
+  const size_t nd = 3 * size_t(nshell) + 2 * size_t(np), ni = 6 * size_t(nshell);
+  size_t bytes = 0;
+  auto place = [&](size_t n) {
+    const size_t at = bytes;
+    bytes = (bytes + n + 15) & ~size_t(15);
+    return at;
+  };
+  const size_t od = place(nd * sizeof(double)), op = place(npairs * sizeof(PairRec)),
+               oi = place(ni * sizeof(int)), of = place(6 * size_t(nshell) * sizeof(float)),
+               opp = place(size_t(off) * sizeof(int)), os = place(npairs),
+               oq = place(sizeof(QuartetItem));
+  // small bases (one shell set's) go through pinned memory and are not waited
+  // for: their calls end with a wait of their own
+  const bool pinned = bytes <= kPinIn;
+  std::vector<unsigned char> pageable;
+  unsigned char* h = ctx->pin;
+  if (pinned) {
+    if (ctx->pin_busy) CK(cudaStreamSynchronize(ctx->stream));
+    ctx->pin_busy = true;
+  } else {
+    pageable.resize(bytes);
+    h = pageable.data();
+  }
+  {
+    double* d = reinterpret_cast<double*>(h + od);
+    std::copy(B.O.begin(), B.O.end(), d);
+    std::copy(B.alpha.begin(), B.alpha.end(), d + 3 * nshell);
+    std::copy(B.coeff.begin(), B.coeff.end(), d + 3 * nshell + np);
+    std::memcpy(h + op, B.hpairs.data(), npairs * sizeof(PairRec));
+    int* i = reinterpret_cast<int*>(h + oi);
+    for (auto* v : {&B.l, &B.pure, &B.nprim, &B.prim_off, &B.bf_off, &B.atom})
+      i = std::copy(v->begin(), v->end(), i);
+    float* f = reinterpret_cast<float*>(h + of);
+    for (int k = 0; k < 3 * nshell; ++k) {
+      const float hi = float(B.O[k]);
+      f[k] = hi;
+      f[3 * nshell + k] = float(B.O[k] - double(hi));
+    }
+    int* ppp = reinterpret_cast<int*>(h + opp);
+    for (long long q = 0; q < npairs; ++q)
+      for (int k = 0; k < B.hpairs[q].npp; ++k) ppp[B.hpairs[q].pp_off + k] = int(q);
+    std::memcpy(h + os, B.hswap.data(), npairs);
+    QuartetItem it{};
+    if (nshell >= 4) {
+      const int q[4] = {0, 1, 2, 3};
+      const Canon c = canonicalize(B, q);
+      it.bra_pair = int(pidx(std::max(c.c[0], c.c[1]), std::min(c.c[0], c.c[1])));
+      it.ket_pair = int(pidx(std::max(c.c[2], c.c[3]), std::min(c.c[2], c.c[3])));
+      it.flags = c.flags;
+    }
+    std::memcpy(h + oq, &it, sizeof(it));
+  }
+  CK(B.blob.ensure(bytes));
   CK(B.pprims.ensure(off * sizeof(PrimPairRec)));
   CK(B.ppds.ensure(off * sizeof(PrimPairJKds)));
-  CK(B.pair_swap.ensure(npairs));
-  CK(cudaMemcpyAsync(B.pairs.p, B.hpairs.data(), npairs * sizeof(PairRec),
-                     cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(B.pp_pair.p, ppp.data(), off * sizeof(int), cudaMemcpyHostToDevice,
-                     ctx->stream));
-  CK(cudaMemcpyAsync(B.pair_swap.p, B.hswap.data(), npairs, cudaMemcpyHostToDevice,
-                     ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  CK(cudaMemcpyAsync(B.blob.p, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  const unsigned char* g = B.blob.as<unsigned char>();
+  const double* db = reinterpret_cast<const double*>(g + od);
+  const int* ib = reinterpret_cast<const int*>(g + oi);
+  B.dev.nshell = nshell;
+  B.dev.l = ib;
+  B.dev.pure = ib + nshell;
+  B.dev.nprim = ib + 2 * nshell;
+  B.dev.prim_off = ib + 3 * nshell;
+  B.dev.bf_off = ib + 4 * nshell;
+  B.dev.atom = ib + 5 * nshell;
+  B.dev.O = db;
+  B.dev.alpha = db + 3 * nshell;
+  B.dev.coeff = db + 3 * nshell + np;
+  B.dev.Ohi = reinterpret_cast<const float*>(g + of);
+  B.dev.Olo = B.dev.Ohi + 3 * nshell;
+  B.dpairs = reinterpret_cast<const PairRec*>(g + op);
+  B.dpp_pair = reinterpret_cast<const int*>(g + opp);
+  B.dpair_swap = g + os;
+  B.ditem = reinterpret_cast<const QuartetItem*>(g + oq);
+  if (!pinned) CK(cudaStreamSynchronize(ctx->stream));
   return LGX_OK;
 }
 
@@ -599,9 +660,9 @@ lgx_status ensure_jk_records(lgx_context* ctx, BasisDev& B) {
 
 lgx_status ensure_pairs(lgx_context* ctx, BasisDev& B, double ln_prec, int method) {
   if (B.pairs_ok && B.pairs_lnprec == ln_prec && B.pairs_method == method) return LGX_OK;
-  CK(launch_shellpairs(B.dev, B.pairs.as<PairRec>(), int(B.hpairs.size()),
+  CK(launch_shellpairs(B.dev, B.dpairs, int(B.hpairs.size()),
                        B.pprims.as<PrimPairRec>(), B.ppds.as<PrimPairJKds>(),
-                       B.pp_pair.as<int>(), B.npp, ln_prec, method, ctx->stream));
+                       B.dpp_pair, B.npp, ln_prec, method, ctx->stream));
   B.pairs_ok = true;
   ++B.pairs_version;
   B.pairs_lnprec = ln_prec;
@@ -687,10 +748,10 @@ lgx_status plan_launch(lgx_context* ctx, const ProgDev& P, int mode, bool fp32,
 // Context and basis pointers every kernel launch needs.
 void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
   a.basis = B.dev;
-  a.pairs = B.pairs.as<PairRec>();
+  a.pairs = B.dpairs;
   a.pprims = B.pprims.as<PrimPairRec>();
   a.ppds = B.ppds.as<PrimPairJKds>();
-  a.pair_swap = B.pair_swap.as<unsigned char>();
+  a.pair_swap = B.dpair_swap;
   a.boys = ctx->boys.as<double>();
   a.boys_tay = ctx->boys_tay.as<double>();
   a.boys32 = ctx->boys32.as<float>();
@@ -860,33 +921,6 @@ lgx_status check_errflag(lgx_context* ctx) {
     return fail(ctx, LGX_ERR_WATCHDOG, "device work loop exceeded its bound");
   }
   return LGX_OK;
-}
-
-// Canonical quartet (engine.impl.h:1181-1211) -> work item.
-struct Canon {
-  int c[4];  // canonical shells
-  int flags;
-  int la, lb, lc, ld;
-};
-Canon canonicalize(const BasisDev& B, const int* s) {
-  const int l0 = B.l[s[0]], l1 = B.l[s[1]], l2 = B.l[s[2]], l3 = B.l[s[3]];
-  const bool stb = l0 < l1, stk = l2 < l3, sbk = l0 + l1 > l2 + l3;
-  int perm[4];
-  perm[0] = sbk ? (stk ? 3 : 2) : (stb ? 1 : 0);
-  perm[1] = sbk ? (stk ? 2 : 3) : (stb ? 0 : 1);
-  perm[2] = sbk ? (stb ? 1 : 0) : (stk ? 3 : 2);
-  perm[3] = sbk ? (stb ? 0 : 1) : (stk ? 2 : 3);
-  Canon q;
-  for (int k = 0; k < 4; ++k) q.c[k] = s[perm[k]];
-  const bool bsw = q.c[0] < q.c[1];  // stored pair has s1 >= s2
-  const bool ksw = q.c[2] < q.c[3];
-  q.flags = (bsw ? 1 : 0) | (ksw ? 2 : 0) |
-            ((sbk ? 1 : 0) | (stb ? 2 : 0) | (stk ? 4 : 0)) << 2;
-  q.la = B.l[q.c[0]];
-  q.lb = B.l[q.c[1]];
-  q.lc = B.l[q.c[2]];
-  q.ld = B.l[q.c[3]];
-  return q;
 }
 
 // One launch of an explicit list: items [begin, begin + count) of one class
@@ -2334,6 +2368,7 @@ lgx_status lgx_create(lgx_context** out, int device) {
       CK(c->inv_odd.ensure(sizeof(h)));
       CK(cudaMemcpy(c->inv_odd.p, h, sizeof(h), cudaMemcpyHostToDevice));
     }
+    CK(cudaHostAlloc(reinterpret_cast<void**>(&c->pin), kPinIn + kPinOut, cudaHostAllocDefault));
     CK(c->counter.ensure(64));
     CK(c->errflag.ensure(64));
     CK(c->primcount.ensure(64));
@@ -2362,6 +2397,7 @@ lgx_status lgx_destroy(lgx_context* ctx) {
     side.push_back(ctx->s32[b]);
   }
   cudaStream_t st = ctx->stream;
+  if (ctx->pin) cudaFreeHost(ctx->pin);
   delete ctx;
   if (st) cudaStreamDestroy(st);
   for (cudaStream_t x : side)
@@ -2424,19 +2460,46 @@ lgx_status shellset_locked(lgx_context* ctx, const lgx_shell shells[4], int deri
     if (lk > lb) CK(launch_drop_pairs(pp + pk.pp_off, pk.npp, lk, ctx->stream));
     B.pairs_ok = lb == lk;  // a cut table is not reused
   }
-  CK(ctx->out.ensure(size_t(nv * ns) * sizeof(double)));
-  CK(ctx->isnull.ensure(sizeof(int)));
-  const int32_t q[4] = {0, 1, 2, 3};
-  s = run_explicit(ctx, ctx->small, q, 1, deriv, kModeStore, nullptr, ctx->out.as<double>(),
-                   ctx->isnull.as<int>(), precision, screening, nullptr);
+  // values, then the null flag, come back in one copy.  One quartet runs on a
+  // register kernel or the block kernel, neither of which can raise the
+  // watchdog flag, so no further wait reads it.
+  const size_t nb = size_t(nv * ns) * sizeof(double);
+  CK(ctx->out.ensure(nb + sizeof(double)));
+  const BasisDev& B = ctx->small;
+  ListSeg seg{};
+  {
+    const int q[4] = {0, 1, 2, 3};
+    const Canon c = canonicalize(B, q);
+    seg.la = c.la; seg.lb = c.lb; seg.lc = c.lc; seg.ld = c.ld;
+  }
+  ProgDev* P = nullptr;
+  s = get_prog(ctx, seg.la, seg.lb, seg.lc, seg.ld, deriv, &P);
+  if (s != LGX_OK) return s;
+  EriArgs a{};
+  a.precision = precision;
+  a.ln_prec = ln_prec;
+  a.screening = screening;
+  a.items = B.ditem;
+  a.nitems = 1;
+  a.out = ctx->out.as<double>();
+  a.is_null = reinterpret_cast<int*>(a.out + nv * ns);
+  s = run_eri(ctx, ctx->small, *P, kModeStore, false, a, 1, double(np[0] * np[1]) * (np[2] * np[3]));
   if (s != LGX_OK) return s;
   int nul = 0;
-  CK(cudaMemcpyAsync(&nul, ctx->isnull.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(out, ctx->out.p, size_t(nv * ns) * sizeof(double), cudaMemcpyDeviceToHost,
-                     ctx->stream));
+  const bool pinned = nb + sizeof(double) <= kPinOut;
+  unsigned char* h = ctx->pin + kPinIn;
+  if (pinned) {
+    CK(cudaMemcpyAsync(h, ctx->out.p, nb + sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  } else {
+    CK(cudaMemcpyAsync(&nul, a.is_null, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(out, ctx->out.p, nb, cudaMemcpyDeviceToHost, ctx->stream));
+  }
   CK(cudaStreamSynchronize(ctx->stream));
-  s = check_errflag(ctx);
-  if (s != LGX_OK) return s;
+  ctx->pin_busy = false;
+  if (pinned) {
+    std::memcpy(out, h, nb);
+    std::memcpy(&nul, h + nb, sizeof(int));
+  }
   *nsets = ns;
   *nvalues = int(nv);
   *is_null = nul;
