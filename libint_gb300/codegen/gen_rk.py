@@ -6,6 +6,8 @@ For each canonical class (la>=lb, lc>=ld, la+lb<=lc+ld) it emits
       (src/bin/libint/vrr_11_twoprep_11.h:145-223,305-383), straight-line,
       each needed (e0|f0)^(m) computed once, targets added into acc[]
       (the HGP contraction point, src/bin/libint/dg.cc:1177-1189);
+  vrr_fused<T>: the same with the targets that no other node reads accumulated
+      as one FMA chain each (two operations fewer; sums round differently);
   hrr<T>(acc, AB, CD, cart): HRR on the bra then the ket
       (src/bin/libint/hrr.h:246-347) into the Cartesian shell set;
   sph<T>(cart, out): Cartesian -> real solid harmonics for every l>=2 index
@@ -167,63 +169,89 @@ def gen_class(la, lb, lc, ld):
     targets = [(e, f) for le in range(la, la + lb + 1) for e in comps(le)
                for lf in range(lc, lc + ld + 1) for f in comps(lf)]
     acc_index = {t: k for k, t in enumerate(targets)}
-    em = Emitter()
-    names = {}
     xyz = "xyz"
-    used_n = set()
 
-    def node(e, f, m):
-        key = (e, f, m)
-        if key in names:
-            return names[key]
-        if sum(e) == 0 and sum(f) == 0:
-            names[key] = "F[%d]" % m
-            return names[key]
-        if sum(f) > 0:
-            j = first_dir(f)
-            f1 = sh(f, j, -1)
-            a = node(e, f1, m)
-            b = node(e, f1, m + 1)
-            expr = "fma(g.WQ%s, %s, g.QC%s * %s)" % (xyz[j], b, xyz[j], a)
-            if f1[j] > 0:
-                f2 = sh(f1, j, -1)
-                c = node(e, f2, m)
-                d = node(e, f2, m + 1)
-                used_n.add(("e", f1[j]))
-                expr = "fma(oo2e_%d, fma(-g.roe, %s, %s), %s)" % (f1[j], d, c, expr)
-            if e[j] > 0:
-                x = node(sh(e, j, -1), f1, m + 1)
-                used_n.add(("ze", e[j]))
-                expr = "fma(oo2ze_%d, %s, %s)" % (e[j], x, expr)
-        else:
+    def emit_vrr(fused):
+        """Straight-line VRR; fused: a target that no other node reads goes
+        into its accumulator as one FMA chain instead of a sum of its own."""
+        em = Emitter()
+        names = {}
+        used_n = set()
+        read = set()
+
+        def terms(e, f, m):
+            """(first factor, node) pairs and nested pairs of one node."""
+            if sum(f) > 0:
+                j = first_dir(f)
+                f1 = sh(f, j, -1)
+                out = [("g.QC" + xyz[j], (e, f1, m)), ("g.WQ" + xyz[j], (e, f1, m + 1))]
+                if f1[j] > 0:
+                    f2 = sh(f1, j, -1)
+                    used_n.add(("e", f1[j]))
+                    out.append(("oo2e_%d" % f1[j], (e, f2, m), "g.roe", (e, f2, m + 1)))
+                if e[j] > 0:
+                    used_n.add(("ze", e[j]))
+                    out.append(("oo2ze_%d" % e[j], (sh(e, j, -1), f1, m + 1)))
+                return out
             i = first_dir(e)
             e1 = sh(e, i, -1)
-            a = node(e1, f, m)
-            b = node(e1, f, m + 1)
-            expr = "fma(g.WP%s, %s, g.PA%s * %s)" % (xyz[i], b, xyz[i], a)
+            out = [("g.PA" + xyz[i], (e1, f, m)), ("g.WP" + xyz[i], (e1, f, m + 1))]
             if e1[i] > 0:
                 e2 = sh(e1, i, -1)
-                c = node(e2, f, m)
-                d = node(e2, f, m + 1)
                 used_n.add(("z", e1[i]))
-                expr = "fma(oo2z_%d, fma(-g.roz, %s, %s), %s)" % (e1[i], d, c, expr)
-        names[key] = em.tmp(expr)
-        return names[key]
+                out.append(("oo2z_%d" % e1[i], (e2, f, m), "g.roz", (e2, f, m + 1)))
+            return out
 
-    body = []
-    for t, k in acc_index.items():
-        v = node(t[0], t[1], 0)
-        em.lines.append("    acc[%d] += %s;" % (k, v))
-    pre = []
-    for kind, n in sorted(used_n):
-        if kind == "z":
-            pre.append("    const T oo2z_%d = T(%d) * g.oo2z;" % (n, n))
-        elif kind == "e":
-            pre.append("    const T oo2e_%d = T(%d) * g.oo2e;" % (n, n))
-        else:
-            pre.append("    const T oo2ze_%d = T(%d) * g.oo2ze;" % (n, n))
-    vrr_body = pre + em.lines
-    vrr_flops = sum(l.count("fma(") * 2 + l.count(" * ") for l in em.lines) + len(acc_index)
+        def name(key):
+            read.add(key)
+            return node(*key)
+
+        def chain(e, f, m, start):
+            # order of the operands as the sums are written: c2 s2 + c1 s1, then
+            # the second and third terms
+            t = terms(e, f, m)
+            a, b = name(t[0][1]), name(t[1][1])
+            expr = "%s * %s" % (t[0][0], a) if start is None else \
+                "fma(%s, %s, %s)" % (t[0][0], a, start)
+            expr = "fma(%s, %s, %s)" % (t[1][0], b, expr)
+            for x in t[2:]:
+                if len(x) == 4:
+                    c, d = name(x[1]), name(x[3])
+                    expr = "fma(%s, fma(-%s, %s, %s), %s)" % (x[0], x[2], d, c, expr)
+                else:
+                    expr = "fma(%s, %s, %s)" % (x[0], name(x[1]), expr)
+            return expr
+
+        def node(e, f, m):
+            key = (e, f, m)
+            if key not in names:
+                if sum(e) == 0 and sum(f) == 0:
+                    names[key] = "F[%d]" % m
+                else:
+                    names[key] = em.tmp(chain(e, f, m, None))
+            return names[key]
+
+        for t in acc_index:  # which targets other nodes read
+            node(t[0], t[1], 0)
+        keep = set(read)
+        em.__init__()
+        names.clear()
+        for t, k in acc_index.items():
+            key = (t[0], t[1], 0)
+            if fused and key not in keep and sum(t[0]) + sum(t[1]) > 0:
+                em.lines.append("    acc[%d] = %s;" % (k, chain(*key, "acc[%d]" % k)))
+            else:
+                em.lines.append("    acc[%d] += %s;" % (k, node(*key)))
+        pre = []
+        for kind, n in sorted(used_n):
+            src = {"z": "oo2z", "e": "oo2e", "ze": "oo2ze"}[kind]
+            pre.append("    const T %s_%d = T(%d) * g.%s;" % (src, n, n, src))
+        return pre + em.lines
+
+    vrr_body = emit_vrr(False)
+    vrr_fused = emit_vrr(True)
+    vrr_flops = sum(l.count("fma(") * 2 + l.count(" * ") for l in vrr_body
+                    if not l.startswith("    const T oo2")) + len(acc_index)
 
     # ---------------- HRR
     hem = Emitter()
@@ -306,6 +334,10 @@ def gen_class(la, lb, lc, ld):
     s.append("  template <typename T>\n  static __device__ __forceinline__ void vrr(const T* F, "
              "const Geo<T>& g, T* acc) {")
     s.extend(vrr_body)
+    s.append("  }")
+    s.append("  template <typename T>\n  static __device__ __forceinline__ void vrr_fused(const T* F, "
+             "const Geo<T>& g, T* acc) {")
+    s.extend(vrr_fused)
     s.append("  }")
     s.append("  template <typename T>\n  static __device__ __forceinline__ void hrr(const T* acc, "
              "const T* AB, const T* CD, T* cart) {")

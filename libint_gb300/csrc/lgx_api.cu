@@ -34,9 +34,10 @@ cudaError_t launch_list_scatter(const ListArgs& a, cudaStream_t st);
 cudaError_t launch_d2f(const double* src, float* dst, long long n, cudaStream_t st);
 cudaError_t launch_shell_block_norm(const DevBasis& b, const double* D, int nbf, double* out,
                                     cudaStream_t st);
-cudaError_t launch_boys_eval(const double* tab, const double* tay, const float* tab32,
-                             const double* inv_odd, int variant, const double* T, long long n,
-                             int mmax, double* F, cudaStream_t st);
+cudaError_t launch_boys_eval(const double* tab, const double* tay, const double* fine,
+                             const float* tab32, const double* inv_odd, int variant,
+                             const double* T, long long n, int mmax, double* F, cudaStream_t st);
+cudaError_t launch_boys_fine(const double* hi, const double* lo, double* fine, cudaStream_t st);
 cudaError_t launch_prim_set(const PrimSetArgs& a, size_t smem, cudaStream_t st);
 cudaError_t launch_eri_block_store(const EriArgs& a, int grid, size_t smem, cudaStream_t st);
 cudaError_t rk_launch(bool fp32, int mode, bool att, int la, int lb, int lc, int ld, const EriArgs& a,
@@ -203,7 +204,7 @@ struct lgx_context {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
   std::string err;
-  DBuf boys, boys_tay, boys32, boys_split, sph_off, sph_c, sph_cd, sph_cf, Df, inv_odd;
+  DBuf boys, boys_tay, boys_fine, boys32, boys_split, sph_off, sph_c, sph_cd, sph_cf, Df, inv_odd;
   std::map<int, std::unique_ptr<ProgDev>> progs;
   bool use_rk = true;  // register kernels for the small classes
   bool use_post = true;  // generated post stages for the large J/K classes
@@ -313,8 +314,10 @@ int fp32_kernel_mode(const lgx_context* ctx, int mode, int base_mode) {
 // ------------------------------------------------------- host constants
 // Boys table: F_m(k/64), m < kBoysCols, from the Maclaurin series (top m)
 // and downward recursion in long double.
-std::vector<double> make_boys_table() {
+// lo: what the rounding to FP64 leaves.
+std::vector<double> make_boys_table(std::vector<double>& lo) {
   std::vector<double> t(size_t(kBoysRows) * kBoysCols);
+  lo.resize(t.size());
   for (int k = 0; k < kBoysRows; ++k) {
     const long double T = (long double)k * kBoysDT;
     const int M = kBoysCols - 1;
@@ -326,10 +329,15 @@ std::vector<double> make_boys_table() {
     }
     const long double eT = expl(-T);
     long double f = eT * sum;
-    t[size_t(k) * kBoysCols + M] = (double)f;
+    auto put = [&](int m) {
+      const size_t i = size_t(k) * kBoysCols + m;
+      t[i] = (double)f;
+      lo[i] = (double)(f - (long double)t[i]);
+    };
+    put(M);
     for (int m = M - 1; m >= 0; --m) {
       f = (2 * T * f + eT) / (2 * m + 1);
-      t[size_t(k) * kBoysCols + m] = (double)f;
+      put(m);
     }
   }
   return t;
@@ -755,6 +763,7 @@ void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
   a.boys = ctx->boys.as<double>();
   a.boys_tay = ctx->boys_tay.as<double>();
   a.boys32 = ctx->boys32.as<float>();
+  a.boys_fine = ctx->boys_fine.as<double>();
   a.boys_split = ctx->boys_split.as<float>();
   a.inv_odd = ctx->inv_odd.as<double>();
   a.sph_off = ctx->sph_off.as<int>();
@@ -763,6 +772,7 @@ void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
   a.sph_cf = ctx->sph_cf.as<float>();
   a.error_flag = ctx->errflag.as<int>();
   a.op = ctx->op;
+  a.omega = ctx->omega;
   a.omega2 = ctx->omega * ctx->omega;
   a.fprecision = float(a.precision);
   a.fln_prec = float(std::max(a.ln_prec, -1.0e30));
@@ -2273,10 +2283,21 @@ lgx_status lgx_create(lgx_context** out, int device) {
     }
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     for (auto& e : c->ev_join) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    const auto boys = make_boys_table();
+    std::vector<double> boys_lo;
+    const auto boys = make_boys_table(boys_lo);
     const auto sph = make_sph_table();
     CK(c->boys.ensure(boys.size() * sizeof(double)));
     CK(cudaMemcpy(c->boys.p, boys.data(), boys.size() * sizeof(double), cudaMemcpyHostToDevice));
+    {
+      DBuf lo;
+      CK(lo.ensure(boys_lo.size() * sizeof(double)));
+      CK(cudaMemcpy(lo.p, boys_lo.data(), boys_lo.size() * sizeof(double),
+                    cudaMemcpyHostToDevice));
+      CK(c->boys_fine.ensure(kBoysFineSize * sizeof(double)));
+      CK(launch_boys_fine(c->boys.as<double>(), lo.as<double>(), c->boys_fine.as<double>(),
+                          c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+    }
     {
       // pre-divided Taylor coefficients F_{m+i}(T_k)/i!
       std::vector<double> tay(size_t(kBoysRows) * (kBoysMaxM + 1) * kBoysTaylorStride, 0.0);
@@ -3008,7 +3029,8 @@ lgx_status lgx_boys(lgx_context* ctx, int variant, const double* T, int64_t n, i
   CK(ctx->boysF.ensure(nf * sizeof(double)));
   CK(cudaMemcpyAsync(ctx->boysT.p, T, size_t(nin) * sizeof(double), cudaMemcpyHostToDevice,
                      ctx->stream));
-  CK(launch_boys_eval(ctx->boys.as<double>(), ctx->boys_tay.as<double>(), ctx->boys32.as<float>(),
+  CK(launch_boys_eval(ctx->boys.as<double>(), ctx->boys_tay.as<double>(),
+                      ctx->boys_fine.as<double>(), ctx->boys32.as<float>(),
                       ctx->inv_odd.as<double>(), variant, ctx->boysT.as<double>(), n, mmax,
                       ctx->boysF.as<double>(), ctx->stream));
   CK(cudaMemcpyAsync(F, ctx->boysF.p, nf * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

@@ -6,41 +6,22 @@
 
 namespace lgx {
 
-// Boys F_0..F_MMAX(T) times the primitive prefactor pfac.
-//  T <= kBoysTmax: Taylor expansion about the nearest grid point T_k = k/64
-//   of the pre-divided table; every m directly when MMAX <= 2, else the top
-//   m plus the downward recursion, with e^{-T} formed as the tabulated
-//   e^{-T_k} (slot 7 of the m = 0 row) times the Maclaurin series of
-//   e^{T_k - T} (|T_k - T| <= 1/128).
-//  T > kBoysTmax (= 50): F_0 = sqrt(pi/T)/2 and the upward recursion
-//   F_{m+1} = (2m+1)/(2T) F_m with the e^{-T} terms dropped; the relative
-//   error of that, the regularised upper incomplete gamma Q(m+1/2, T), is
-//   below 2e-16 for m <= 5 and 1.7e-15 for m = 6 at T = 50.
-// FP64 evaluation once the branch and the grid point are chosen: asym
-// selects the asymptotic branch; otherwise k is the grid point and md =
-// T_k - T.  PF: multiply by pfac (the mixed scheme's FP32 kernels apply
-// their prefactor in FP32, so they skip the FP64 products by 1).  NT: terms
-// of the Taylor series and of the e^{T_k - T} series (the remainder is below
-// |md|^NT/NT! of F_m: 6 terms 3.2e-16 for the FP64 kernels; 4 terms 1.6e-10
-// for values that are rounded to FP32 next, whose half-ulp is 6e-8).  R32:
-// 1/sqrt(T) of the asymptotic branch by one FP64 Newton step from the FP32
-// estimate (relative error ~1.4e-13, again for values rounded to FP32 next)
-// instead of the full-precision FP64 rsqrt.
-template <int MMAX, bool PF = true, int NT = 6, bool R32 = false>
+// The store kernels' FP64 evaluation for values that are rounded to FP32 next,
+// once the branch and the grid point are chosen (rk_boys_b64): the 1/64 grid's
+// pre-divided table, k the grid point and md = T_k - T, every m directly when
+// MMAX <= 2, else the top m and the downward recursion with e^{-T} as the
+// tabulated e^{-T_k} times the series of e^{md}; 4 terms, 1.6e-10 of F_m, whose
+// half-ulp is 6e-8.  asym: sqrt(pi/T)/2 and the upward recursion without the
+// e^{-T} terms, 1/sqrt(T) by one FP64 Newton step from the FP32 estimate.
+template <int MMAX>
 __device__ __forceinline__ void rk_boys_core(const double* __restrict__ tay, double T, bool asym,
-                                             int k, double md, double pfac, double* F) {
-  static_assert(NT >= 2 && NT <= 7, "the table holds 7 Taylor coefficients per m");
+                                             int k, double md, double* F) {
   static_assert(MMAX <= 6, "asymptotic branch without e^{-T} is exact to 2e-15 only for m <= 6");
   if (asym) {
-    double rs;
-    if constexpr (R32) {
-      const double r0 = f2d_int(rsqrtf(d2f_int(T)));  // relative error <= ~3e-7
-      rs = fma(0.5 * r0, fma(-(T * r0), r0, 1.0), r0);
-    } else {
-      rs = rsqrt(T);
-    }
+    const double r0 = f2d_int(rsqrtf(d2f_int(T)));  // relative error <= ~3e-7
+    const double rs = fma(0.5 * r0, fma(-(T * r0), r0, 1.0), r0);
     const double oo2T = 0.5 * (rs * rs);
-    double f = PF ? (0.88622692545275801365 * pfac) * rs : 0.88622692545275801365 * rs;
+    double f = 0.88622692545275801365 * rs;
     F[0] = f;
 #pragma unroll
     for (int m = 0; m < MMAX; ++m) {
@@ -50,47 +31,105 @@ __device__ __forceinline__ void rk_boys_core(const double* __restrict__ tay, dou
     return;
   }
   const double* row = tay + (k * (kBoysMaxM + 1)) * kBoysTaylorStride;
+  auto series = [&](const double* c) {
+    double s = __ldg(c + 3);
+    s = fma(s, md, __ldg(c + 2));
+    s = fma(s, md, __ldg(c + 1));
+    return fma(s, md, __ldg(c));
+  };
   if (MMAX <= 2) {
 #pragma unroll
-    for (int m = 0; m <= MMAX; ++m) {
-      const double* c = row + m * kBoysTaylorStride;
-      double s = __ldg(c + NT - 1);
-#pragma unroll
-      for (int i = NT - 2; i >= 0; --i) s = fma(s, md, __ldg(c + i));
-      F[m] = PF ? s * pfac : s;
-    }
+    for (int m = 0; m <= MMAX; ++m) F[m] = series(row + m * kBoysTaylorStride);
   } else {
-    const double* c = row + MMAX * kBoysTaylorStride;
-    double s = __ldg(c + NT - 1);
-#pragma unroll
-    for (int i = NT - 2; i >= 0; --i) s = fma(s, md, __ldg(c + i));
-    if (PF) s *= pfac;
+    double s = series(row + MMAX * kBoysTaylorStride);
     F[MMAX] = s;
-    // e^{md} = sum_{i < NT} md^i / i!, Horner from the top term
-    constexpr double inv_fact[7] = {1.0, 1.0, 0.5, 1.0 / 6.0, 1.0 / 24.0, 1.0 / 120.0,
-                                    1.0 / 720.0};
-    double e = inv_fact[NT - 1];
-#pragma unroll
-    for (int i = NT - 2; i >= 0; --i) e = fma(e, md, inv_fact[i]);
-    const double eTp = PF ? (__ldg(row + 7) * pfac) * e : __ldg(row + 7) * e;  // pfac e^{-T}
+    double e = 1.0 / 6.0;
+    e = fma(e, md, 0.5);
+    e = fma(e, md, 1.0);
+    e = fma(e, md, 1.0);
+    const double eT = __ldg(row + 7) * e;
     const double twoT = 2.0 * T;
 #pragma unroll
     for (int m = MMAX - 1; m >= 0; --m) {
-      s = fma(twoT, s, eTp) * (1.0 / (2 * m + 1));
+      s = fma(twoT, s, eT) * (1.0 / (2 * m + 1));
       F[m] = s;
     }
   }
 }
 
+// The register kernels' FP64 Boys function, F_m(T) pfac, from the fine tables.
+//  T <= 50: c0 + md (c1 + md (c2 + md (c3 + c4 md))), md = T_j - T, the inner
+//   bracket in FP32; every m directly for MMAX <= 2, else the top m, and
+//   e^{-T} = e^{-T_j} e^{md} by the same kind of series.
+//  T > 50: sqrt(pi/T)/2 and the upward recursion without its e^{-T} terms
+//   (MMAX <= 2), or the top m, (2m-1)!! / 2^m times it / T^m.
+//  MMAX > 2: the downward recursion, with e^{-T} = 0 beyond T = 50 (it is below
+//   1.7e-15 of F_6 there), which lanes of both branches run together.
+// What bounds it: the FP64 pipe (2 lanes per cycle and SM), so everything that
+// only chooses (branch, grid point) or lies below 2^-32 runs in integer and
+// FP32 instructions: per m 3 FP64 operations instead of 5 on the 1/64 grid, and
+// 1 instead of 4 for the grid point.  The tables (0.8 MB for MMAX = 0, 2.5 MB
+// for 2) stay in L2.
 template <int MMAX>
-__device__ __forceinline__ void rk_boys(const double* __restrict__ tay, double T, double pfac,
+__device__ __forceinline__ void rk_boys(const double* __restrict__ fine, double T, double pfac,
                                         double* F) {
-  // nearest grid point: adding 1.5*2^52 rounds T*32 to an integer held in
-  // the low mantissa bits (read back with an integer move)
-  const double t32 = fma(T, kBoysInvDT, 6755399441055744.0);
-  const int k = __double2loint(t32);
-  const double md = fma(t32 - 6755399441055744.0, kBoysDT, -T);  // = -(T - T_k)
-  rk_boys_core<MMAX>(tay, T, T > kBoysTmax, k, md, pfac, F);
+  static_assert(MMAX <= kBoysFineM, "fine tables and the asymptotic branch end at m = 6");
+  const float Tf = d2f_int(T);
+  const bool asym = Tf > float(kBoysTmax);
+  if (asym && MMAX <= 2) {
+    const double rs = rsqrt64(T);
+    const double oo2T = 0.5 * (rs * rs);
+    double f = (0.88622692545275801365 * pfac) * rs;
+    F[0] = f;
+#pragma unroll
+    for (int m = 0; m < MMAX; ++m) {
+      f *= (2 * m + 1) * oo2T;
+      F[m + 1] = f;
+    }
+    return;
+  }
+  const int j = asym ? 0 : __float2int_rn(Tf * float(kBoysFineInv));
+  const double md = fma(i2d_int(j), 1.0 / kBoysFineInv, -T);
+  const float mdf = d2f_int(md);
+  const double2* row = reinterpret_cast<const double2*>(fine + boys_fine_off(MMAX) +
+                                                        j * boys_fine_cols(MMAX));
+  auto series = [&](int e) {  // of the row's entry e
+    const double2 a = __ldg(row + 2 * e), b = __ldg(row + 2 * e + 1);
+    const float c3 = __int_as_float(__double2loint(b.y)), c4 = __int_as_float(__double2hiint(b.y));
+    double s = fma(md, f2d_int(fmaf(mdf, c4, c3)), b.x);
+    s = fma(md, s, a.y);
+    return fma(md, s, a.x);
+  };
+  if (MMAX <= 2) {
+#pragma unroll
+    for (int m = 0; m <= MMAX; ++m) F[m] = series(m) * pfac;
+    return;
+  }
+  double s, eTp = 0.0;
+  if (asym) {
+    const double rs = rsqrt64(T);
+    const double r2 = rs * rs;
+    double c = 0.88622692545275801365;  // (2m-1)!! / 2^m sqrt(pi)/2
+#pragma unroll
+    for (int m = 0; m < MMAX; ++m) c *= 0.5 * (2 * m + 1);
+    s = (c * pfac) * rs;
+#pragma unroll
+    for (int m = 0; m < MMAX; ++m) s *= r2;
+  } else {
+    s = series(0) * pfac;
+    // e^{md} = 1 + md (1 + md (1/2 + md (1/6 + md/24)))
+    double e = fma(md, f2d_int(fmaf(mdf, 1.0f / 24.0f, 1.0f / 6.0f)), 0.5);
+    e = fma(md, e, 1.0);
+    e = fma(md, e, 1.0);
+    eTp = (__ldg(row + 2).x * pfac) * e;
+  }
+  F[MMAX] = s;
+  const double twoT = 2.0 * T;
+#pragma unroll
+  for (int m = MMAX - 1; m >= 0; --m) {
+    s = fma(twoT, s, eTp) * (1.0 / (2 * m + 1));
+    F[m] = s;
+  }
 }
 
 // The mixed scheme's FP64 Boys function of an FP32 quartet (store kernels), given its
@@ -111,11 +150,11 @@ __device__ __forceinline__ void rk_boys_b64(const double* __restrict__ tay, dsf 
   const float mdh = __fadd_rn(__fmul_rn(float(k), float(kBoysDT)), -T.hi);
   const double md = f2d_int(mdh) - f2d_int(T.lo);
   if (MMAX <= 2 && !asym) {  // direct Taylor series: T itself is not needed
-    rk_boys_core<MMAX, false, 4>(tay, 0.0, false, k, md, 1.0, F);
+    rk_boys_core<MMAX>(tay, 0.0, false, k, md, F);
     return;
   }
   const double T64 = f2d_int(T.hi) + f2d_int(T.lo);
-  rk_boys_core<MMAX, false, 4, true>(tay, T64, asym, k, md, 1.0, F);
+  rk_boys_core<MMAX>(tay, T64, asym, k, md, F);
 }
 
 // The Boys function of the mixed scheme's J/K kernels times the FP32

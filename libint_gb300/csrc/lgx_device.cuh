@@ -30,6 +30,24 @@ constexpr int kBoysRows = int(kBoysTmax * 64.0) + 2;  // 3202 grid points
 // entry 7 of the m = 0 row holds e^{-T_k}.
 constexpr int kBoysTaylorStride = 8;
 
+// Fine FP64 tables of the register kernels (compile-time mmax <= 6), on a
+// 1/512 grid up to kBoysTmax, filled on the GPU from the 1/64 table: an entry
+// (m, j) is four doubles {c0, c1, c2, (float c3, float c4)} with c_i =
+// F_{m+i}(T_j) / i!.  |T_j - T| <= 2^-10, so the terms from the third on are
+// below 2^-32 of F_m and FP32 carries them (2^-56 of F_m); the series stops at
+// 2^-57.  Per mmax one packed table: rows of the entries of m = 0..mmax for
+// mmax <= 2, of mmax alone and e^{-T_j} above.
+constexpr int kBoysFineInv = 512;
+constexpr int kBoysFineRows = 50 * kBoysFineInv + 2;
+constexpr int kBoysFineM = 6;
+__host__ __device__ constexpr int boys_fine_cols(int mmax) { return mmax <= 2 ? 4 * (mmax + 1) : 6; }
+__host__ __device__ constexpr int boys_fine_off(int mmax) {
+  int o = 0;
+  for (int m = 0; m < mmax; ++m) o += kBoysFineRows * boys_fine_cols(m);
+  return o;
+}
+constexpr int kBoysFineSize = boys_fine_off(kBoysFineM + 1);
+
 // Split FP32 tables of the mixed scheme's J/K kernels: the grid values
 // F_m(T_k) as hi = float(F), lo = float(F - hi).
 //  packed, one per mmax <= kBoysSplitM (the register kernels' compile-time
@@ -93,6 +111,17 @@ __device__ __forceinline__ float d2f_int(double x) {
   if (e <= 0) return __uint_as_float(sign);
   if (e >= 255 || bits >= 0x7f800000u) return __uint_as_float(sign | 0x7f800000u);
   return __uint_as_float(sign | bits);
+}
+
+// 1/sqrt(x), x normal and positive: the special-function unit's estimate r and
+// one step of third order, r + r e (1/2 + 3/8 e) with e = 1 - x r^2 (from an
+// estimate good to 2^-20 the step leaves 2^-60).  Five FP64 instructions, which
+// is what counts in kernels bound by that pipe.
+__device__ __forceinline__ double rsqrt64(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-(x * r), r, 1.0);
+  return fma(r * e, fma(e, 0.375, 0.5), r);
 }
 
 // double(n) for a small non-negative integer n < 2^20 with integer

@@ -133,6 +133,7 @@ struct EriArgs {
   const double* boys;     // [kBoysRows][kBoysCols] F_m(T_k)
   const double* boys_tay; // pre-divided Taylor table (kBoysTaylorStride)
   const float* boys32;    // FP32 copy of the Boys table
+  const double* boys_fine;  // fine FP64 tables (boys_fine_off)
   const float* boys_split;  // split FP32 tables (boys_split_off, kBoysGenOff)
   const double* inv_odd;  // 1/(2m+1), m < 40
   // Cartesian -> solid harmonics, sparse: nonzeros of row (l, p) are
@@ -149,7 +150,7 @@ struct EriArgs {
   // two-body operator: 0 coulomb 1/r, 1 erf(omega r)/r, 2 erfc(omega r)/r
   // (attenuated: program kernel instantiations and the ATT register kernels)
   int op;
-  double omega2;  // omega^2
+  double omega, omega2;  // omega and its square
   // work
   const QuartetItem* items;
   long long nitems;

@@ -29,23 +29,38 @@ __device__ __forceinline__ double rk_f64(float x) { return f2d_int(x); }
 //   erfc(omega r)/r:  F_m(T) - s^{m+1/2} F_m(s T)
 // (s T <= T, so the same Taylor grid serves).  omega = 0 gives zero (erf)
 // and the Coulomb integrals (erfc).
+// FP64: the whole Boys step of the attenuated operators, F = the core integrals
+// times pfac.  sqrt(s) and s come from one reciprocal square root; erf needs no
+// F_m(T).  Returns false when they vanish: erf at omega = 0, and erfc where
+// s T > 50, as both parts are then asymptotic and equal (their difference is
+// below e^-50 of F_m; evaluated, it was the rounding noise of two equal sums).
 template <int MMAX>
-__device__ __forceinline__ void rk_attenuate(const EriArgs& a, double T, double rho, double pfac,
-                                             double* F) {
+__device__ __forceinline__ bool rk_boys_att(const EriArgs& a, double T, double rho, double pfac,
+                                            double* F) {
   if (!(a.omega2 > 0.0)) {
-    if (a.op == 1)
-#pragma unroll
-      for (int m = 0; m <= MMAX; ++m) F[m] = 0.0;
-    return;
+    if (a.op == 1) return false;
+    rk_boys<MMAX>(a.boys_fine, T, pfac, F);
+    return true;
   }
-  const double s = a.omega2 / (a.omega2 + rho);
+  const double r = rsqrt64(a.omega2 + rho);
+  const double s = a.omega2 * (r * r);
+  const double sT = s * T;
+  if (a.op == 2 && d2f_int(sT) > float(kBoysTmax)) return false;
   double G[MMAX + 1];
-  rk_boys<MMAX>(a.boys_tay, T * s, pfac, G);
-  double f = sqrt(s);
+  rk_boys<MMAX>(a.boys_fine, sT, pfac * (a.omega * r), G);
+  if (a.op == 1) {
+    double f = 1.0;
 #pragma unroll
-  for (int m = 0; m <= MMAX; ++m, f *= s) F[m] = a.op == 1 ? f * G[m] : F[m] - f * G[m];
+    for (int m = 0; m <= MMAX; ++m, f *= s) F[m] = m == 0 ? G[0] : f * G[m];
+    return true;
+  }
+  rk_boys<MMAX>(a.boys_fine, T, pfac, F);
+  double f = s;
+  F[0] -= G[0];
+#pragma unroll
+  for (int m = 1; m <= MMAX; ++m, f *= s) F[m] = fma(-f, G[m], F[m]);
+  return true;
 }
-
 template <int MMAX>
 __device__ __forceinline__ void rk_attenuate(const EriArgs& a, float T, float rho, float pfac,
                                              float* F) {
@@ -127,19 +142,22 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<double
   if (!ln_kept(a, bp.fln_scr + kp.fln_scr, q.bra_pp + ib, q.ket_pp + ik, scr)) return false;
   const double zeta = bp.zeta, eta = kp.zeta;
   const double gpq = zeta + eta;
-  const double rs = rsqrt(gpq);
+  const double rs = rsqrt64(gpq);
   const double pfac = bp.Kc * kp.Kc * rs;
   if ((__double_as_longlong(pfac) & 0x7fffffffffffffffll) < __double_as_longlong(scr.prec))
     return false;
   const double oogpq = rs * rs;
   const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1], PQz = bp.P[2] - kp.P[2];
-  const double rho = zeta * eta * oogpq;
+  const double ez = eta * oogpq, zz = zeta * oogpq;
+  const double rho = zeta * ez;
   const double T = rho * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
   double F[C::kMmax + 1];
-  rk_boys<C::kMmax>(a.boys_tay, T, pfac, F);
-  if constexpr (ATT) rk_attenuate<C::kMmax>(a, T, rho, pfac, F);
+  if constexpr (ATT) {
+    if (!rk_boys_att<C::kMmax>(a, T, rho, pfac, F)) return true;
+  } else {
+    rk_boys<C::kMmax>(a.boys_fine, T, pfac, F);
+  }
   rk::Geo<double> g;
-  const double ez = eta * oogpq, zz = zeta * oogpq;
   g.PAx = bp.P[0] - q.A[0]; g.PAy = bp.P[1] - q.A[1]; g.PAz = bp.P[2] - q.A[2];
   g.QCx = kp.P[0] - q.C[0]; g.QCy = kp.P[1] - q.C[1]; g.QCz = kp.P[2] - q.C[2];
   g.WPx = -ez * PQx; g.WPy = -ez * PQy; g.WPz = -ez * PQz;
@@ -149,7 +167,7 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<double
   g.oo2e = 0.5 * kp.oog;
   g.roe = zz;
   g.oo2ze = 0.5 * oogpq;
-  C::template vrr<double>(F, g, acc);
+  C::template vrr_fused<double>(F, g, acc);
   return true;
 }
 
@@ -180,7 +198,9 @@ __device__ __forceinline__ PrimF32 rk_pp32(const PrimPairRec& r, bool sw) {
 // One primitive quartet into acc (FP32).  AC = A - C of the quartet.
 // bidx, kidx: the two primitive pairs' PrimPairRec indices (the FP64
 // values of the screening decisions inside the rounding band).
-template <class C, bool ATT>
+// FUSE: fused accumulation, for kernels that hand out sums over quartets; the
+// store kernels keep the rounding of the single sums.
+template <class C, bool ATT, bool FUSE>
 __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<float>& q,
                                         const PrimF32& bp, const PrimF32& kp, int bidx,
                                         int kidx, const PrimScreen& scr, float* acc) {
@@ -211,7 +231,10 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<float>
   g.oo2e = 0.5f * kp.k.z;
   g.roe = zz;
   g.oo2ze = 0.5f * oogpq;
-  C::template vrr<float>(F, g, acc);
+  if constexpr (FUSE)
+    C::template vrr_fused<float>(F, g, acc);
+  else
+    C::template vrr<float>(F, g, acc);
   return true;
 }
 
@@ -249,12 +272,13 @@ __device__ __forceinline__ bool rk_prim_b64(const EriArgs& a, const RkQuartet<fl
     bds = a.ppds + bidx;
     kds = a.ppds + kidx;
   }
-  const dsf T =
-      ds_boys_arg(__ldg(&bds->hi), __ldg(&bds->lo), __ldg(&kds->hi), __ldg(&kds->lo), rho, oogpq);
   float F[C::kMmax + 1];
+  const float4 bh = __ldg(&bds->hi), bl = __ldg(&bds->lo), kh = __ldg(&kds->hi),
+               kl = __ldg(&kds->lo);
   if constexpr (BOYS == 2) {
-    rk_boys_split<C::kMmax>(a.boys_split, T, pfac, F);
+    rk_boys_split<C::kMmax>(a.boys_split, ds_boys_arg(bh, bl, kh, kl, rho, oogpq), pfac, F);
   } else {
+    const dsf T = ds_boys_arg(bh, bl, kh, kl, rho, oogpq);
     double F64[C::kMmax + 1];
     rk_boys_b64<C::kMmax>(a.boys_tay, T, F64);
 #pragma unroll
@@ -271,7 +295,10 @@ __device__ __forceinline__ bool rk_prim_b64(const EriArgs& a, const RkQuartet<fl
   g.oo2e = 0.5f * kp.k.z;
   g.roe = zz;
   g.oo2ze = 0.5f * oogpq;
-  C::template vrr<float>(F, g, acc);
+  if constexpr (BOYS == 2)
+    C::template vrr_fused<float>(F, g, acc);
+  else
+    C::template vrr<float>(F, g, acc);
   return true;
 }
 
@@ -392,7 +419,9 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
                       ? 1
                       : 0;
         } else {
-          kept += rk_prim<C, ATT>(a, q, bp, kp, q.bra_pp + ib, q.ket_pp + ik, scr, acc) ? 1 : 0;
+          kept += rk_prim<C, ATT, mode_jk(MODE)>(a, q, bp, kp, q.bra_pp + ib, q.ket_pp + ik, scr, acc)
+                      ? 1
+                      : 0;
         }
       } else {
         kept += rk_prim<C, ATT>(a, q, ib, ik, scr, acc) ? 1 : 0;

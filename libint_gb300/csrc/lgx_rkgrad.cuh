@@ -37,7 +37,7 @@ __device__ __forceinline__ bool rk_prologue(const EriArgs& a, const RkQuartet<do
   const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
   if (!ln_kept(a, bp.fln_scr + kp.fln_scr, q.bra_pp + ib, q.ket_pp + ik, scr)) return false;
   const double zeta = bp.zeta, eta = kp.zeta;
-  const double rs = rsqrt(zeta + eta);
+  const double rs = rsqrt64(zeta + eta);
   const double pfac = bp.Kc * kp.Kc * rs;
   // |pfac|, with the Conservative factor where the list is screened by it
   if (a.screening == 1) {
@@ -52,7 +52,7 @@ __device__ __forceinline__ bool rk_prologue(const EriArgs& a, const RkQuartet<do
   const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1], PQz = bp.P[2] - kp.P[2];
   const double ez = eta * oogpq, zz = zeta * oogpq;
   const double T = zeta * ez * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
-  rk_boys<MMAX>(a.boys_tay, T, pfac, F);
+  rk_boys<MMAX>(a.boys_fine, T, pfac, F);
   geo.PAx = bp.P[0] - q.A[0]; geo.PAy = bp.P[1] - q.A[1]; geo.PAz = bp.P[2] - q.A[2];
   geo.QCx = kp.P[0] - q.C[0]; geo.QCy = kp.P[1] - q.C[1]; geo.QCz = kp.P[2] - q.C[2];
   geo.WPx = -ez * PQx; geo.WPy = -ez * PQy; geo.WPz = -ez * PQz;

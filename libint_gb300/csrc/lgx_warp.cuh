@@ -387,12 +387,14 @@ __device__ __forceinline__ bool prologue(const EriArgs& a, const QuartetGeom<flo
   if constexpr (B64 != 0) {
     const PrimPairJKds* bd = a.ppds + g.bra_pp + ib;
     const PrimPairJKds* kd = a.ppds + g.ket_pp + ik;
-    const dsf Td = ds_boys_arg(__ldg(&bd->hi), __ldg(&bd->lo), __ldg(&kd->hi), __ldg(&kd->lo),
-                                rho, oogpq);
+    const float4 bh = __ldg(&bd->hi), bl = __ldg(&bd->lo), kh = __ldg(&kd->hi),
+                 kl = __ldg(&kd->lo);
     if constexpr (B64 == 2)
-      boys_split_stage(a.boys_split, Td, a.prog.mmax, pfac, st + kStF);
+      boys_split_stage(a.boys_split, ds_boys_arg(bh, bl, kh, kl, rho, oogpq), a.prog.mmax,
+                       pfac, st + kStF);
     else
-      boys_b64_stage(a.boys_tay, a.inv_odd, Td, a.prog.mmax, pfac, st + kStF);
+      boys_b64_stage(a.boys_tay, a.inv_odd, ds_boys_arg(bh, bl, kh, kl, rho, oogpq), a.prog.mmax,
+                     pfac, st + kStF);
   } else if constexpr (ATT) {
     if (a.op != 1) boys_to_stage(a.boys32, T, a.prog.mmax, pfac, st + kStF);
     attenuate<float>(a, T, rho, a.prog.mmax, pfac, st + kStF);
