@@ -237,6 +237,40 @@ __device__ __forceinline__ dsf ds_boys_arg(const float4& bh, const float4& bl, c
   return ds_mul(rho, ds_add(ds_add(ds_sqr(dx), ds_sqr(dy)), ds_sqr(dz)));
 }
 
+// ds_boys_arg for the J/K kernels with the steps that their accuracy does not
+// need left out: differences, the sum of squares and the product stay
+// unnormalised (lo is only ever added), ~80 FP32 operations instead of ~130;
+// T to 2^-44 relative beyond the records' 2^-48 |P|.
+__device__ __forceinline__ dsf ds_boys_arg_jk(const float4& bh, const float4& bl, const float4& kh,
+                                              const float4& kl, float rho0, float oogpq) {
+  // rho = rho0 + (zeta eta - rho0 (zeta + eta)) / (zeta + eta)
+  const float p = __fmul_rn(bh.w, kh.w);
+  const dsf a = ds_two_sum(bh.w, kh.w);
+  const float q = __fmul_rn(rho0, a.hi);
+  const float t = fmaf(-rho0, __fadd_rn(a.lo, __fadd_rn(bl.w, kl.w)),
+                       fmaf(bh.w, kl.w, __fmul_rn(bl.w, kh.w)));
+  const float r = __fadd_rn(__fadd_rn(p, -q),
+                            __fadd_rn(__fadd_rn(fmaf(bh.w, kh.w, -p), -fmaf(rho0, a.hi, -q)), t));
+  const float c = __fmul_rn(r, oogpq);
+  // |P - Q|^2
+  float lo = 0.0f;
+  auto square = [&](float b, float bb, float k, float kk) {
+    const dsf d = ds_two_sum(b, -k);
+    const float l = __fadd_rn(d.lo, __fadd_rn(bb, -kk));
+    const float s = __fmul_rn(d.hi, d.hi);
+    lo = __fadd_rn(lo, fmaf(d.hi, d.hi, -s));
+    lo = fmaf(l, fmaf(2.0f, d.hi, l), lo);
+    return s;
+  };
+  const float sx = square(bh.x, bl.x, kh.x, kl.x), sy = square(bh.y, bl.y, kh.y, kl.y),
+              sz = square(bh.z, bl.z, kh.z, kl.z);
+  const dsf s1 = ds_two_sum(sx, sy);
+  const dsf s2 = ds_two_sum(s1.hi, sz);
+  lo = __fadd_rn(lo, __fadd_rn(s1.lo, s2.lo));
+  const float th = __fmul_rn(rho0, s2.hi);
+  return ds_fast_two_sum(th, fmaf(rho0, lo, fmaf(c, s2.hi, fmaf(rho0, s2.hi, -th))));
+}
+
 // T^{-1/2} and 1/(2T) of a double-float T (normal, positive) as hi + lo, from
 // the FP32 estimate r0: e = 1 - T r0^2 (|e| <= ~3e-7) is formed exactly enough
 // by three FMAs on the rounded product q = T.hi r0, and r = r0 + r0 e/2 leaves

@@ -276,7 +276,7 @@ __device__ __forceinline__ bool rk_prim_b64(const EriArgs& a, const RkQuartet<fl
   const float4 bh = __ldg(&bds->hi), bl = __ldg(&bds->lo), kh = __ldg(&kds->hi),
                kl = __ldg(&kds->lo);
   if constexpr (BOYS == 2) {
-    rk_boys_split<C::kMmax>(a.boys_split, ds_boys_arg(bh, bl, kh, kl, rho, oogpq), pfac, F);
+    rk_boys_split<C::kMmax>(a.boys_split, ds_boys_arg_jk(bh, bl, kh, kl, rho, oogpq), pfac, F);
   } else {
     const dsf T = ds_boys_arg(bh, bl, kh, kl, rho, oogpq);
     double F64[C::kMmax + 1];

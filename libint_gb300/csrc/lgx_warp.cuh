@@ -390,7 +390,7 @@ __device__ __forceinline__ bool prologue(const EriArgs& a, const QuartetGeom<flo
     const float4 bh = __ldg(&bd->hi), bl = __ldg(&bd->lo), kh = __ldg(&kd->hi),
                  kl = __ldg(&kd->lo);
     if constexpr (B64 == 2)
-      boys_split_stage(a.boys_split, ds_boys_arg(bh, bl, kh, kl, rho, oogpq), a.prog.mmax,
+      boys_split_stage(a.boys_split, ds_boys_arg_jk(bh, bl, kh, kl, rho, oogpq), a.prog.mmax,
                        pfac, st + kStF);
     else
       boys_b64_stage(a.boys_tay, a.inv_odd, ds_boys_arg(bh, bl, kh, kl, rho, oogpq), a.prog.mmax,
