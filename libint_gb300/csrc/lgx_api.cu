@@ -26,6 +26,7 @@ cudaError_t launch_shellpairs(const DevBasis& b, const PairRec* pairs, int npair
                               long long npp, double ln_prec, int method, cudaStream_t st);
 cudaError_t launch_jk_finalize(const double* Jacc, const double* Kacc, double* J,
                                double* K, int nbf, cudaStream_t st);
+cudaError_t launch_ztab(const double* exps, int nexp, int n, double2* out, cudaStream_t st);
 cudaError_t launch_drop_pairs(PrimPairRec* pp, int n, double ln_prec, cudaStream_t st);
 size_t stage_bytes_per_warp(bool fp32, int rows);
 int eri_blocks_per_sm(int mode, bool fp32, int block, size_t smem);
@@ -110,6 +111,12 @@ struct BasisDev {
   const int* dpp_pair = nullptr;
   const unsigned char* dpair_swap = nullptr;
   const QuartetItem* ditem = nullptr;  // work item of the quartet (0 1|2 3)
+  // exponent-pair table (EriArgs::ztab): distinct exponents, entries per row
+  // (0: none), and whether it is built
+  const double* dexps = nullptr;
+  int nexp = 0, nz = 0;
+  DBuf ztab;
+  bool ztab_ok = false;
   DevBasis dev{};
   // pairs
   std::vector<PairRec> hpairs;
@@ -574,10 +581,20 @@ lgx_status upload_basis(lgx_context* ctx, BasisDev& B, int nshell, const int32_t
   if (off > std::numeric_limits<int>::max())
     return fail(ctx, LGX_ERR_TOO_LARGE, "too many primitive pairs");
   B.npp = off;
-  // One device blob and one copy: doubles [O|alpha|coeff], pair records, ints
-  // [l|pure|nprim|prim_off|bf_off|atom], floats [Ohi|Olo], pair of each
+  std::vector<uint64_t> exps(np);  // distinct bit patterns (ordered for any value, NaN too)
+  std::memcpy(exps.data(), B.alpha.data(), np * sizeof(double));
+  const std::vector<uint64_t> ebits = exps;
+  std::sort(exps.begin(), exps.end());
+  exps.erase(std::unique(exps.begin(), exps.end()), exps.end());
+  B.nexp = int(exps.size());
+  // a table for what runs more than one quartet, 69 MB at most
+  B.nz = nshell > 12 && B.nexp <= 64 ? B.nexp * (B.nexp + 1) / 2 : 0;
+  B.ztab_ok = false;
+  // One device blob and one copy: doubles [O|alpha|coeff|distinct exponents],
+  // pair records, ints [l|pure|nprim|prim_off|bf_off|atom|eid], floats [Ohi|Olo], pair of each
   // primitive pair, pair swaps, and the item of the quartet of shells 0-3.
-  const size_t nd = 3 * size_t(nshell) + 2 * size_t(np), ni = 6 * size_t(nshell);
+  const size_t nd = 3 * size_t(nshell) + 2 * size_t(np) + exps.size(),
+               ni = 6 * size_t(nshell) + size_t(np);
   size_t bytes = 0;
   auto place = [&](size_t n) {
     const size_t at = bytes;
@@ -605,10 +622,13 @@ lgx_status upload_basis(lgx_context* ctx, BasisDev& B, int nshell, const int32_t
     std::copy(B.O.begin(), B.O.end(), d);
     std::copy(B.alpha.begin(), B.alpha.end(), d + 3 * nshell);
     std::copy(B.coeff.begin(), B.coeff.end(), d + 3 * nshell + np);
+    std::memcpy(d + 3 * nshell + 2 * np, exps.data(), exps.size() * sizeof(double));
     std::memcpy(h + op, B.hpairs.data(), npairs * sizeof(PairRec));
     int* i = reinterpret_cast<int*>(h + oi);
     for (auto* v : {&B.l, &B.pure, &B.nprim, &B.prim_off, &B.bf_off, &B.atom})
       i = std::copy(v->begin(), v->end(), i);
+    for (uint64_t e : ebits)
+      *i++ = int(std::lower_bound(exps.begin(), exps.end(), e) - exps.begin());
     float* f = reinterpret_cast<float*>(h + of);
     for (int k = 0; k < 3 * nshell; ++k) {
       const float hi = float(B.O[k]);
@@ -646,6 +666,8 @@ lgx_status upload_basis(lgx_context* ctx, BasisDev& B, int nshell, const int32_t
   B.dev.O = db;
   B.dev.alpha = db + 3 * nshell;
   B.dev.coeff = db + 3 * nshell + np;
+  B.dexps = db + 3 * nshell + 2 * np;
+  B.dev.eid = ib + 6 * nshell;
   B.dev.Ohi = reinterpret_cast<const float*>(g + of);
   B.dev.Olo = B.dev.Ohi + 3 * nshell;
   B.dpairs = reinterpret_cast<const PairRec*>(g + op);
@@ -667,6 +689,11 @@ lgx_status ensure_jk_records(lgx_context* ctx, BasisDev& B) {
 }
 
 lgx_status ensure_pairs(lgx_context* ctx, BasisDev& B, double ln_prec, int method) {
+  if (B.nz > 0 && !B.ztab_ok) {
+    CK(B.ztab.ensure(size_t(B.nz) * B.nz * sizeof(double2)));
+    CK(launch_ztab(B.dexps, B.nexp, B.nz, B.ztab.as<double2>(), ctx->stream));
+    B.ztab_ok = true;
+  }
   if (B.pairs_ok && B.pairs_lnprec == ln_prec && B.pairs_method == method) return LGX_OK;
   CK(launch_shellpairs(B.dev, B.dpairs, int(B.hpairs.size()),
                        B.pprims.as<PrimPairRec>(), B.ppds.as<PrimPairJKds>(),
@@ -758,6 +785,8 @@ void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
   a.basis = B.dev;
   a.pairs = B.dpairs;
   a.pprims = B.pprims.as<PrimPairRec>();
+  a.ztab = B.nz > 0 ? B.ztab.as<double2>() : nullptr;
+  a.nz = B.nz;
   a.ppds = B.ppds.as<PrimPairJKds>();
   a.pair_swap = B.dpair_swap;
   a.boys = ctx->boys.as<double>();

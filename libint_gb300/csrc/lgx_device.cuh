@@ -79,6 +79,7 @@ struct DevBasis {
   const double* O;      // [3*nshell]
   const double* alpha;  // flattened
   const double* coeff;  // flattened, normalization embedded
+  const int* eid;       // per primitive: index among the basis's distinct exponents
   const float* Ohi;     // [3*nshell] float(O)
   const float* Olo;     // [3*nshell] float(O - Ohi): Ohi + Olo = O to ~1e-15
 };
@@ -136,21 +137,24 @@ __device__ __forceinline__ double i2d_int(int n) {
 // One primitive pair of a shell pair (s1, s2) as stored (s1 = first shell),
 // with FP64 fields for the FP64 kernels and FP32 copies (centre-relative
 // P, so FP32 P-Q differences keep their precision) for the FP32 kernels.
+// PA, hoog, ta1 / ta2 and zid are what the FP64 primitive loop would otherwise
+// form again for every primitive quartet on the pipe that bounds it.
 struct __align__(16) PrimPairRec {
   double P[3];
-  double Kc;      // sqrt(2) pi^{5/4} exp(-rho AB^2)/gamma * c1 * c2
-  double oog;     // 1/(alpha1 + alpha2)
-  double zeta;    // alpha1 + alpha2
-  double a1, a2;  // exponents of s1 and s2
-  double ln_scr;  // ln of the pair screening factor (shell.h:1041-1059)
+  double Kc;        // sqrt(2) pi^{5/4} exp(-rho AB^2)/gamma * c1 * c2
+  double hoog;      // 1/(2 (alpha1 + alpha2))
+  double zeta;      // alpha1 + alpha2
+  double ta1, ta2;  // twice the exponents of s1 and s2
+  double PA[6];     // P - O(s1), P - O(s2)
+  double ln_scr;    // ln of the pair screening factor (shell.h:1041-1059)
   float fKc, fzeta, foog, fln_scr;
-  float fPA1[3];  // P - O(s1)
-  float fPA2[3];  // P - O(s2)
+  float fPA1[3];    // P - O(s1)
+  float fPA2[3];    // P - O(s2)
   float fa1, fa2;
-  float fnonsph;  // Conservative screening factor
-  float pad;
+  float fnonsph;    // Conservative screening factor
+  int zid;          // index of the exponent pair (EriArgs::ztab)
 };
-static_assert(sizeof(PrimPairRec) == 128, "PrimPairRec layout");
+static_assert(sizeof(PrimPairRec) == 176, "PrimPairRec layout");
 
 // FP32 primitive-pair record of the J/K bins (two float4): {K c1 c2,
 // zeta, 1/zeta, ln screening factor} and {P - O(first canonical centre),

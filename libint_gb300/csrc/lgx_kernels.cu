@@ -59,25 +59,53 @@ __global__ void shellpair_kernel(DevBasis b, const PairRec* pairs, int npairs, P
     drop = degenerate || ln_scr < ln_prec;
   }
   r.Kc = degenerate ? 0.0 : 5.9149671727956128778 * exp(mrAB2) * oog * c1 * c2;
-  r.oog = oog;
+  r.hoog = 0.5 * oog;
   r.zeta = gamma;
-  r.a1 = a1;
-  r.a2 = a2;
+  r.ta1 = 2.0 * a1;
+  r.ta2 = 2.0 * a2;
+  for (int x = 0; x < 3; ++x) {
+    r.PA[x] = r.P[x] - A[x];
+    r.PA[3 + x] = r.P[x] - B[x];
+  }
   r.ln_scr = drop ? -1.0e300 : ln_scr;
   r.fKc = float(r.Kc);
   r.fzeta = float(gamma);
   r.foog = float(oog);
   r.fln_scr = drop ? -3.0e38f : float(ln_scr);
   for (int x = 0; x < 3; ++x) {
-    r.fPA1[x] = float(r.P[x] - A[x]);
-    r.fPA2[x] = float(r.P[x] - B[x]);
+    r.fPA1[x] = float(r.PA[x]);
+    r.fPA2[x] = float(r.PA[3 + x]);
   }
   r.fa1 = float(a1);
   r.fa2 = float(a2);
   r.fnonsph = float(nonsph);
-  r.pad = 0.f;
+  const int e1 = b.eid[b.prim_off[s1] + p1], e2 = b.eid[b.prim_off[s2] + p2];
+  r.zid = max(e1, e2) * (max(e1, e2) + 1) / 2 + min(e1, e2);
   pp[t] = r;
   ppds[t] = make_jkds(r.P[0], r.P[1], r.P[2], gamma);
+}
+
+// Exponent-pair table: entry (i, j) of n x n is {1/sqrt(z_i + z_j), 1/(z_i +
+// z_j)} of the exponent sums z of the basis's distinct exponent pairs.
+__global__ void ztab_kernel(const double* __restrict__ exps, int nexp, int n,
+                            double2* __restrict__ out) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= (long long)n * n) return;
+  auto zeta = [&](int k) {
+    int e1 = int((sqrtf(8.0f * k + 1.0f) - 1.0f) * 0.5f);
+    while (e1 * (e1 + 1) / 2 > k) --e1;
+    while ((e1 + 1) * (e1 + 2) / 2 <= k) ++e1;
+    return exps[e1] + exps[k - e1 * (e1 + 1) / 2];
+  };
+  const double rs = rsqrt64(zeta(int(t / n)) + zeta(int(t % n)));
+  out[t] = make_double2(rs, rs * rs);
+}
+
+cudaError_t launch_ztab(const double* exps, int nexp, int n, double2* out, cudaStream_t st) {
+  const int block = 256;
+  const long long tot = (long long)n * n;
+  ztab_kernel<<<(unsigned)((tot + block - 1) / block), block, 0, st>>>(exps, nexp, n, out);
+  return cudaGetLastError();
 }
 
 // FP32 J/K records: record r takes primitive pair src[r] & 0x7fffffff,

@@ -125,6 +125,8 @@ struct EriArgs {
   DevBasis basis;
   const PairRec* pairs;
   const PrimPairRec* pprims;
+  const double2* ztab;       // {rsqrt, reciprocal} of zeta + eta per exponent-pair pair, or null
+  int nz;                    // row length of ztab
   const PrimPairJKds* ppds;  // double-float P and zeta per primitive pair (pprims index)
   const PrimPairJK32* jk32;  // J/K bins: coalesced FP32 records (may be null)
   const PrimPairJKds* jkds;  // J/K bins: their double-float P and zeta (same layout)

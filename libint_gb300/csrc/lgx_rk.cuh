@@ -84,7 +84,6 @@ struct RkQuartet {
   int sh[4];
   int bra_pp, ket_pp, nbpp, nkpp;
   bool bsw, ksw;
-  double A[3], C[3];  // FP64 kernels only
   T AB[3], CD[3], AC[3];
 };
 
@@ -108,8 +107,6 @@ __device__ __forceinline__ void rk_load(const EriArgs& a, int bpair, int kpair, 
     for (int x = 0; x < 3; ++x) {
       const double A = a.basis.O[3 * q.sh[0] + x], B = a.basis.O[3 * q.sh[1] + x];
       const double C = a.basis.O[3 * q.sh[2] + x], D = a.basis.O[3 * q.sh[3] + x];
-      q.A[x] = A;
-      q.C[x] = C;
       q.AB[x] = A - B;
       q.CD[x] = C - D;
       q.AC[x] = A - C;
@@ -130,6 +127,17 @@ __device__ __forceinline__ void rk_load(const EriArgs& a, int bpair, int kpair, 
   }
 }
 
+// {1/sqrt(zeta + eta), 1/(zeta + eta)} of a primitive quartet: from the basis's
+// exponent-pair table, seven FP64 instructions of about 40 in the s/p classes
+// (a basis has few distinct exponents, (H2O)n cc-pVTZ 26: 351^2 entries, 2 MB);
+// computed where the basis has too many for a table.
+__device__ __forceinline__ double2 rk_gpq(const EriArgs& a, const PrimPairRec& bp,
+                                          const PrimPairRec& kp) {
+  if (a.ztab) return __ldg(a.ztab + (size_t)bp.zid * a.nz + kp.zid);
+  const double rs = rsqrt64(bp.zeta + kp.zeta);
+  return make_double2(rs, rs * rs);
+}
+
 // One primitive quartet into acc (FP64).  Returns false when screened out.
 // The ln-screen runs on the FP32 copies with the FP64 values inside the
 // rounding band (ln_kept) and the pfac screen compares the IEEE bit
@@ -141,12 +149,11 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<double
   const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
   if (!ln_kept(a, bp.fln_scr + kp.fln_scr, q.bra_pp + ib, q.ket_pp + ik, scr)) return false;
   const double zeta = bp.zeta, eta = kp.zeta;
-  const double gpq = zeta + eta;
-  const double rs = rsqrt64(gpq);
+  const double2 gpq = rk_gpq(a, bp, kp);
+  const double rs = gpq.x, oogpq = gpq.y;
   const double pfac = bp.Kc * kp.Kc * rs;
   if ((__double_as_longlong(pfac) & 0x7fffffffffffffffll) < __double_as_longlong(scr.prec))
     return false;
-  const double oogpq = rs * rs;
   const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1], PQz = bp.P[2] - kp.P[2];
   const double ez = eta * oogpq, zz = zeta * oogpq;
   const double rho = zeta * ez;
@@ -158,13 +165,15 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<double
     rk_boys<C::kMmax>(a.boys_fine, T, pfac, F);
   }
   rk::Geo<double> g;
-  g.PAx = bp.P[0] - q.A[0]; g.PAy = bp.P[1] - q.A[1]; g.PAz = bp.P[2] - q.A[2];
-  g.QCx = kp.P[0] - q.C[0]; g.QCy = kp.P[1] - q.C[1]; g.QCz = kp.P[2] - q.C[2];
+  const double* PA = bp.PA + (q.bsw ? 3 : 0);
+  const double* QC = kp.PA + (q.ksw ? 3 : 0);
+  g.PAx = PA[0]; g.PAy = PA[1]; g.PAz = PA[2];
+  g.QCx = QC[0]; g.QCy = QC[1]; g.QCz = QC[2];
   g.WPx = -ez * PQx; g.WPy = -ez * PQy; g.WPz = -ez * PQz;
   g.WQx = zz * PQx; g.WQy = zz * PQy; g.WQz = zz * PQz;
-  g.oo2z = 0.5 * bp.oog;
+  g.oo2z = bp.hoog;
   g.roz = ez;
-  g.oo2e = 0.5 * kp.oog;
+  g.oo2e = kp.hoog;
   g.roe = zz;
   g.oo2ze = 0.5 * oogpq;
   C::template vrr_fused<double>(F, g, acc);

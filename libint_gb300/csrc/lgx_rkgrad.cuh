@@ -37,7 +37,8 @@ __device__ __forceinline__ bool rk_prologue(const EriArgs& a, const RkQuartet<do
   const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
   if (!ln_kept(a, bp.fln_scr + kp.fln_scr, q.bra_pp + ib, q.ket_pp + ik, scr)) return false;
   const double zeta = bp.zeta, eta = kp.zeta;
-  const double rs = rsqrt64(zeta + eta);
+  const double2 gpq = rk_gpq(a, bp, kp);
+  const double rs = gpq.x, oogpq = gpq.y;
   const double pfac = bp.Kc * kp.Kc * rs;
   // |pfac|, with the Conservative factor where the list is screened by it
   if (a.screening == 1) {
@@ -48,18 +49,19 @@ __device__ __forceinline__ bool rk_prologue(const EriArgs& a, const RkQuartet<do
              __double_as_longlong(scr.prec)) {
     return false;
   }
-  const double oogpq = rs * rs;
   const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1], PQz = bp.P[2] - kp.P[2];
   const double ez = eta * oogpq, zz = zeta * oogpq;
   const double T = zeta * ez * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
   rk_boys<MMAX>(a.boys_fine, T, pfac, F);
-  geo.PAx = bp.P[0] - q.A[0]; geo.PAy = bp.P[1] - q.A[1]; geo.PAz = bp.P[2] - q.A[2];
-  geo.QCx = kp.P[0] - q.C[0]; geo.QCy = kp.P[1] - q.C[1]; geo.QCz = kp.P[2] - q.C[2];
+  const double* PA = bp.PA + (q.bsw ? 3 : 0);
+  const double* QC = kp.PA + (q.ksw ? 3 : 0);
+  geo.PAx = PA[0]; geo.PAy = PA[1]; geo.PAz = PA[2];
+  geo.QCx = QC[0]; geo.QCy = QC[1]; geo.QCz = QC[2];
   geo.WPx = -ez * PQx; geo.WPy = -ez * PQy; geo.WPz = -ez * PQz;
   geo.WQx = zz * PQx; geo.WQy = zz * PQy; geo.WQz = zz * PQz;
-  geo.oo2z = 0.5 * bp.oog;
+  geo.oo2z = bp.hoog;
   geo.roz = ez;
-  geo.oo2e = 0.5 * kp.oog;
+  geo.oo2e = kp.hoog;
   geo.roe = zz;
   geo.oo2ze = 0.5 * oogpq;
   return true;
@@ -153,8 +155,8 @@ __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
         C::template prim<double>(F, geo, WJ, WK, s, I);
         const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
         const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
-        const double wa = 2.0 * (q.bsw ? bp.a2 : bp.a1), wb = 2.0 * (q.bsw ? bp.a1 : bp.a2);
-        const double wd = 2.0 * (q.ksw ? kp.a1 : kp.a2);
+        const double wa = (q.bsw ? bp.ta2 : bp.ta1), wb = (q.bsw ? bp.ta1 : bp.ta2);
+        const double wd = (q.ksw ? kp.ta1 : kp.ta2);
 #pragma unroll
         for (int x = 0; x < kSets; ++x) {
           const double* sx = s + 7 * x;
@@ -265,8 +267,8 @@ __global__ void __launch_bounds__(128, 2) rk_deriv_kernel(EriArgs a) {
         ++kept;
         const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
         const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
-        const double w[3] = {2.0 * (q.bsw ? bp.a2 : bp.a1), 2.0 * (q.bsw ? bp.a1 : bp.a2),
-                             2.0 * (q.ksw ? kp.a1 : kp.a2)};
+        const double w[3] = {(q.bsw ? bp.ta2 : bp.ta1), (q.bsw ? bp.ta1 : bp.ta2),
+                             (q.ksw ? kp.ta1 : kp.ta2)};
         C::template prim<double>(F, geo, w, I);
       }
       ib += gb;

@@ -334,26 +334,28 @@ __device__ __forceinline__ bool prologue(const EriArgs& a, const QuartetGeom<dou
     boys_to_stage(a.boys, a.inv_odd, T, a.prog.mmax, pfac, st + kStF);
   }
   const double ez = eta * oogpq, zz = zeta * oogpq;
-  st[kStPA + 0] = bp.P[0] - g.A[0];
-  st[kStPA + 1] = bp.P[1] - g.A[1];
-  st[kStPA + 2] = bp.P[2] - g.A[2];
-  st[kStQC + 0] = kp.P[0] - g.C[0];
-  st[kStQC + 1] = kp.P[1] - g.C[1];
-  st[kStQC + 2] = kp.P[2] - g.C[2];
+  const double* PA = bp.PA + (g.bra_sw ? 3 : 0);
+  const double* QC = kp.PA + (g.ket_sw ? 3 : 0);
+  st[kStPA + 0] = PA[0];
+  st[kStPA + 1] = PA[1];
+  st[kStPA + 2] = PA[2];
+  st[kStQC + 0] = QC[0];
+  st[kStQC + 1] = QC[1];
+  st[kStQC + 2] = QC[2];
   st[kStWP + 0] = -ez * PQx;
   st[kStWP + 1] = -ez * PQy;
   st[kStWP + 2] = -ez * PQz;
   st[kStWQ + 0] = zz * PQx;
   st[kStWQ + 1] = zz * PQy;
   st[kStWQ + 2] = zz * PQz;
-  st[kStOo2z] = 0.5 * bp.oog;
+  st[kStOo2z] = bp.hoog;
   st[kStRoz] = ez;
-  st[kStOo2e] = 0.5 * kp.oog;
+  st[kStOo2e] = kp.hoog;
   st[kStRoe] = zz;
   st[kStOo2ze] = 0.5 * oogpq;
-  st[kStW + 0] = 2.0 * (g.bra_sw ? bp.a2 : bp.a1);
-  st[kStW + 1] = 2.0 * (g.bra_sw ? bp.a1 : bp.a2);
-  st[kStW + 2] = 2.0 * (g.ket_sw ? kp.a1 : kp.a2);
+  st[kStW + 0] = g.bra_sw ? bp.ta2 : bp.ta1;
+  st[kStW + 1] = g.bra_sw ? bp.ta1 : bp.ta2;
+  st[kStW + 2] = g.ket_sw ? kp.ta1 : kp.ta2;
   return true;
 }
 
