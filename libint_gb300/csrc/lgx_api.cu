@@ -240,7 +240,10 @@ struct lgx_context {
   // 1: round-robin in bin order (default: best or level on (H2O)32 cc-pVDZ,
   // (H2O)8 and (H2O)64 cc-pVTZ); 2: as 0 but issued in bin order
   int branch_policy = 1;
-  int fp64_bps = 0;
+  // the FP64 launches' cap is what leaves FP32 launches room now that FP64 ones keep
+  // their SMs busy to the end: -1, one block per SM up to L = 2 and two above
+  // ((H2O)32 cc-pVDZ 161 ms without a cap, 136 with it; (H2O)20 cc-pVTZ 670 and 636)
+  int fp64_bps = -1;
   int fp32_bps = 0;  // as fp64_bps, for the FP32 launches of a mixed pass
   cudaStream_t s64[kMaxBranches] = {}, s32[kMaxBranches] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[2 * kMaxBranches] = {};
@@ -860,6 +863,11 @@ lgx_status run_rk(lgx_context* ctx, BasisDev& B, const ProgDev& P, int mode, boo
                   EriArgs a, long long nwork, int group) {
   fill_common(ctx, B, a);
   a.group = group;
+  if (!a.counter) {  // else zeroed by the caller
+    a.counter = ctx->counter.as<unsigned long long>();
+    CK(cudaMemsetAsync(ctx->counter.p, 0, sizeof(unsigned long long),
+                       ctx->launch_stream ? ctx->launch_stream : ctx->stream));
+  }
   if (mode == kModeGrad) {
     CK(rk_grad_launch(P.host.la, P.host.lb, P.host.lc, P.host.ld, a, nwork, ctx->nsm,
                       ctx->launch_stream ? ctx->launch_stream : ctx->stream));
@@ -1773,7 +1781,9 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
       st = stream(fp32, b);
       // program-kernel slot scratch: one region per branch
       ctx->scratch = (fp32 || b > 0) ? &ctx->gscratch_br[(fp32 ? nhalf : 0) + b] : &ctx->gscratch;
-      if (!fp32 && mode32 >= 0) a.max_bps = ctx->fp64_bps;
+      if (!fp32 && mode32 >= 0)
+        a.max_bps = ctx->fp64_bps >= 0 ? ctx->fp64_bps
+                                       : (bin.la + bin.lb + bin.lc + bin.ld <= 2 ? 1 : 2);
       if (fp32) a.max_bps = ctx->fp32_bps;
     }
     ctx->launch_stream = st;
@@ -2406,7 +2416,7 @@ lgx_status lgx_create(lgx_context** out, int device) {
     if (const char* e = getenv("LGX_TUNE")) c->tune = (e[0] != '0');
     if (const char* e = getenv("LGX_GRAPHS")) c->use_graphs = (e[0] != '0');
     if (const char* e = getenv("LGX_OVERLAP")) c->overlap = (e[0] != '0');
-    if (const char* e = getenv("LGX_FP64_BPS")) c->fp64_bps = std::max(0, atoi(e));
+    if (const char* e = getenv("LGX_FP64_BPS")) c->fp64_bps = std::max(-1, atoi(e));
     if (const char* e = getenv("LGX_FP32_BPS")) c->fp32_bps = std::max(0, atoi(e));
     if (const char* e = getenv("LGX_BRANCHES")) c->branches = std::max(1, atoi(e));
     if (const char* e = getenv("LGX_BRANCH_POLICY")) c->branch_policy = std::min(2, std::max(0, atoi(e)));
@@ -2531,6 +2541,7 @@ lgx_status shellset_locked(lgx_context* ctx, const lgx_shell shells[4], int deri
   a.screening = screening;
   a.items = B.ditem;
   a.nitems = 1;
+  a.counter = ctx->counter.as<unsigned long long>();  // not read: one chunk
   a.out = ctx->out.as<double>();
   a.is_null = reinterpret_cast<int*>(a.out + nv * ns);
   s = run_eri(ctx, ctx->small, *P, kModeStore, false, a, 1, double(np[0] * np[1]) * (np[2] * np[3]));

@@ -342,6 +342,36 @@ constexpr int rk_min_blocks() {
   return t >= 0 ? t : (sizeof(T) == 8 && LA + LB + LC + LD >= 5 ? 1 : 0);
 }
 
+// Chunks of one launch in the order the warps take them.
+// DYN (FP64 launches): the first nwarps chunks one each, the rest from the launch's
+// counter as warps become free, the next index asked for before the chunk's work
+// and read after it.  A bin lists its depths ascending, so its chunks go from the
+// last to the first: those with the most primitive quartets start first and the
+// launch ends on the cheapest.  In index order with a fixed stride the SMs idled
+// for half of an FP64 launch: (ss|ps) of (H2O)12 cc-pVDZ kept the FP64 pipe busy for
+// 79% of the active but 40% of the elapsed cycles.  FP32 launches have ten times
+// the chunks, of a tenth of the time, and keep a fixed stride ((H2O)32 cc-pVDZ
+// mixed pass 147 ms; 169 ms with the counters, which all warps hit).
+template <bool DYN>
+struct RkChunks {
+  long long idx, n, nwarps;
+  unsigned long long nxt;
+  __device__ __forceinline__ RkChunks(const EriArgs& a, long long total, int per, long long warp,
+                                      long long warps)
+      : idx(warp), n((total + per - 1) / per), nwarps(warps), nxt(0) {}
+  __device__ __forceinline__ bool left() const { return idx < n; }
+  __device__ __forceinline__ long long at(int reversed) const { return DYN && reversed ? n - 1 - idx : idx; }
+  __device__ __forceinline__ void fetch(const EriArgs& a, int lane) {
+    if (DYN && n > nwarps && lane == 0) nxt = atomicAdd(a.counter, 1ull);
+  }
+  __device__ __forceinline__ void next(int lane) {
+    if (DYN)
+      idx = n > nwarps ? nwarps + (long long)__shfl_sync(0xffffffffu, nxt, 0) : n;
+    else
+      idx += nwarps;
+  }
+};
+
 // ATT: attenuated operator (erf / erfc, EriArgs::op), J/K mode only; the
 // Coulomb instances (ATT = false) carry none of its code.
 template <typename T, int LA, int LB, int LC, int LD, int MODE, bool ATT = false>
@@ -359,10 +389,12 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
   const long long first = a.implicit ? a.bin.first : 0;
   const long long total = a.implicit ? a.bin.total : a.nitems;
   unsigned long long my_prims = 0;
-  // Warp chunks of per_warp consecutive quartets, strided over the grid:
-  // consecutive quartets share a bin segment (same bra pair, same depth).
-  for (long long c = warp_id; c * per_warp < total; c += nwarps) {
-    const long long c0 = first + c * per_warp;
+  // Warp chunks of per_warp consecutive quartets (consecutive quartets share a
+  // bin segment: same bra pair, same depth), see RkChunks.
+  RkChunks<sizeof(T) == 8> ch(a, total, per_warp, warp_id, nwarps);
+  for (; ch.left(); ch.next(lane)) {
+    ch.fetch(a, lane);
+    const long long c0 = first + ch.at(a.implicit) * per_warp;
     const long long qi = c0 + (lane / G);
     int seg = 0;
     if (a.implicit) {

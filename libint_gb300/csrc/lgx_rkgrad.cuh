@@ -89,8 +89,10 @@ __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
   scr.ln_prec = a.ln_prec;
   scr.fprec = a.fprecision;
   scr.fln_prec = a.fln_prec;
-  for (long long c = warp_id; c * per_warp < total; c += nwarps) {
-    const long long c0 = first + c * per_warp;
+  RkChunks<true> ch(a, total, per_warp, warp_id, nwarps);
+  for (; ch.left(); ch.next(lane)) {
+    ch.fetch(a, lane);
+    const long long c0 = first + ch.at(1) * per_warp;
     const long long qi = c0 + (lane / G);
     // segment of each quartet of the chunk (see rk_kernel)
     const int seg0 = bin_segment(a.bin, c0);

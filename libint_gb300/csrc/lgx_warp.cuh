@@ -884,8 +884,14 @@ __global__ void __launch_bounds__(128) eri_warp_kernel(EriArgs a) {
       if (lane == 0) atomicExch(a.error_flag, 1);
       break;
     }
-    const long long end = first + min(total, start + (long long)a.chunk);
+    long long end = min(total, start + (long long)a.chunk);
+    if (a.implicit) {  // deepest contractions first
+      const long long e = total - start;
+      start = total - end;
+      end = e;
+    }
     start += first;
+    end += first;
     int seg = 0;
     if (a.implicit) seg = bin_segment(a.bin, start);
     for (long long q = start; q < end; ++q) {
