@@ -51,16 +51,30 @@ N_UNITS = 24  # instantiation translation units (compiled in parallel)
 # listed get 1 for FP64 classes with L >= 5 (left to itself the compiler
 # gives several of them 32 registers and 25-57 KB of spills per thread; with
 # 1 their serial (H2O)64 cc-pVTZ launches ran 14-29% faster), else 0.  The
-# listed ones: the spill-free settings that beat the compiler's choice by
-# 7-11% in a sweep of 0, 1, 3, 4, 6, 8 over tuned serial passes of
-# (H2O)64 cc-pVTZ.  Caps that make the FP32 kernels spill were faster in
-# serial passes but slower inside the graph pass, where the spills compete
-# for L2 with the concurrent launches ((ps|ps) of the mixed scheme at 8:
-# 434 GB of DRAM traffic and +40% time), so none is listed.
+# listed FP32 ones: settings that won by 3-14% over tuned serial passes.  The
+# mixed scheme's kernels wait on loads (Boys table, pair records) with 20 warps
+# an SM; the caps add a fifth to a half of the warps for spills of a few words:
+# (H2O)32 cc-pVDZ mixed pass 136 -> 128 ms, (H2O)20 cc-pVTZ 637 -> 626 ms.  One
+# step tighter each ((ss|ps) at 8, (ps|ps) at 7 blocks) gains another 1-3% in
+# serial launches and nothing in the pass, and tighter still the spills compete
+# for L2 with the concurrent launches.
 MIN_BLOCKS = {
     ("float", "kModeJK", (1, 0, 3, 0)): 4,
     ("float", "kModeJK", (2, 0, 2, 0)): 4,
+    ("float", "kModeJKB64", (0, 0, 0, 0)): 8,
+    ("float", "kModeJKB64", (0, 0, 1, 0)): 7,
+    ("float", "kModeJKB64", (0, 0, 1, 1)): 6,
+    ("float", "kModeJKB64", (0, 0, 2, 0)): 6,
+    ("float", "kModeJKB64", (0, 0, 2, 1)): 5,
     ("float", "kModeJKB64", (0, 0, 3, 3)): 3,
+    ("float", "kModeJKB64", (1, 0, 1, 0)): 6,
+    ("float", "kModeJKB64", (1, 0, 1, 1)): 5,
+    ("float", "kModeJKB64", (1, 0, 2, 0)): 5,
+    ("float", "kModeJKB64", (1, 0, 2, 1)): 4,
+    ("float", "kModeJKB64", (1, 0, 2, 2)): 3,
+    ("float", "kModeJKB64", (1, 1, 2, 0)): 4,
+    ("float", "kModeJKB64", (2, 0, 2, 0)): 4,
+    ("float", "kModeJKB64", (2, 0, 2, 1)): 3,
 }
 MODE_IDS = {"kModeStore": 0, "kModeSchwarz": 1, "kModeJK": 2, "kModeJKB64": 4,
             "kModeStoreB64": 5}
