@@ -40,7 +40,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, HERE)
-from gen_rk import (Emitter, _write_if_changed, comps, first_dir, lit, ncart,  # noqa: E402
+from gen_rk import (RK_MAX_L_STORE, Emitter, _write_if_changed, comps, first_dir, lit, ncart,  # noqa: E402
                     rk_classes, sh, sph_matrix)
 
 GEN_DIR = os.path.join(os.path.dirname(HERE), "csrc", "gen")
@@ -413,6 +413,8 @@ def main():
     classes = sorted(classes, key=lambda c: -sum(c))
     names, decls = [], []
     items = [("grad", c) for c in classes] + [("deriv", c) for c in rk_classes(DERIV_MAX_L)]
+    items += [("one0", c) for c in rk_classes(RK_MAX_L_STORE)]
+    items += [("one1", c) for c in rk_classes(DERIV_MAX_L)]
     items.sort(key=lambda t: -sum(t[1]))
     for k in range(N_UNITS):
         name = "grad_unit_%02d.cu" % k
@@ -422,6 +424,12 @@ def main():
         for kind, c in items[k::N_UNITS]:
             fn = "rk_%s_launch_%d%d%d%d" % ((kind,) + c)
             decls.append((kind, c, fn))
+            if kind.startswith("one"):
+                lines.append("cudaError_t %s(const EriArgs& a, int blocks, cudaStream_t st) {" % fn)
+                lines.append("  return rk_one_launch_one<%d, %d, %d, %d, %s>(a, blocks, st);" %
+                             (c + (kind[3],)))
+                lines.append("}")
+                continue
             lines.append("cudaError_t %s(const EriArgs& a, long long work, int nsm, "
                          "cudaStream_t st) {" % fn)
             lines.append("  return rk_%s_launch_one<%d, %d, %d, %d>(a, work, nsm, st);" %
@@ -432,8 +440,9 @@ def main():
     d = ["// GENERATED by libint_gb300/codegen/gen_grad.py -- do not edit.",
          "// Run-time dispatch of the register-resident derivative kernels.",
          '#include "../lgx_kernels.cuh"', "", "namespace lgx {"]
-    for _, _, fn in sorted(decls):
-        d.append("cudaError_t %s(const EriArgs& a, long long work, int nsm, cudaStream_t st);" % fn)
+    for kind, _, fn in sorted(decls):
+        d.append("cudaError_t %s(const EriArgs& a, %s, cudaStream_t st);" %
+                 (fn, "int blocks" if kind.startswith("one") else "long long work, int nsm"))
     for name, lmax in (("grad", GRAD_MAX_L), ("deriv", DERIV_MAX_L)):
         d += ["", "cudaError_t rk_%s_launch(int la, int lb, int lc, int ld, const EriArgs& a, "
               "long long work, int nsm," % name, "                           cudaStream_t st) {",
@@ -445,7 +454,16 @@ def main():
         d += ["  }", "  return cudaErrorNotSupported;", "}", "",
               "bool rk_%s_available(int la, int lb, int lc, int ld) {" % name,
               "  return la <= 3 && lc <= 3 && la + lb + lc + ld <= %d;" % lmax, "}"]
-    d += ["}  // namespace lgx"]
+    d += ["", "// One quartet over several blocks (derivative order 0 or 1); its accumulators "
+          "per block", "// in doubles, or 0 when there is no kernel.",
+          "cudaError_t rk_one_launch(int deriv, int la, int lb, int lc, int ld, const EriArgs& a, "
+          "int blocks,", "                          cudaStream_t st) {",
+          "  switch ((((deriv * 8 + la) * 8 + lb) * 8 + lc) * 8 + ld) {"]
+    for kind, c, fn in sorted(decls):
+        if kind.startswith("one"):
+            d.append("    case %d: return %s(a, blocks, st);" %
+                     ((((int(kind[3]) * 8 + c[0]) * 8 + c[1]) * 8 + c[2]) * 8 + c[3], fn))
+    d += ["  }", "  return cudaErrorNotSupported;", "}", "}  // namespace lgx"]
     _write_if_changed(os.path.join(GEN_DIR, "grad_dispatch.cu"), "\n".join(d) + "\n")
     return names + ["grad_dispatch.cu"]
 

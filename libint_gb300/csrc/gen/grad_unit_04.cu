@@ -8,10 +8,19 @@ cudaError_t rk_grad_launch_1130(const EriArgs& a, long long work, int nsm, cudaS
 cudaError_t rk_grad_launch_1120(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<1, 1, 2, 0>(a, work, nsm, st);
 }
+cudaError_t rk_one0_launch_1120(const EriArgs& a, int blocks, cudaStream_t st) {
+  return rk_one_launch_one<1, 1, 2, 0, 0>(a, blocks, st);
+}
 cudaError_t rk_deriv_launch_0030(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_deriv_launch_one<0, 0, 3, 0>(a, work, nsm, st);
 }
+cudaError_t rk_one1_launch_0030(const EriArgs& a, int blocks, cudaStream_t st) {
+  return rk_one_launch_one<0, 0, 3, 0, 1>(a, blocks, st);
+}
 cudaError_t rk_deriv_launch_1010(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_deriv_launch_one<1, 0, 1, 0>(a, work, nsm, st);
+}
+cudaError_t rk_deriv_launch_0010(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
+  return rk_deriv_launch_one<0, 0, 1, 0>(a, work, nsm, st);
 }
 }  // namespace lgx

@@ -5,11 +5,20 @@ namespace lgx {
 cudaError_t rk_grad_launch_0022(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<0, 0, 2, 2>(a, work, nsm, st);
 }
+cudaError_t rk_one0_launch_0022(const EriArgs& a, int blocks, cudaStream_t st) {
+  return rk_one_launch_one<0, 0, 2, 2, 0>(a, blocks, st);
+}
 cudaError_t rk_grad_launch_0021(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<0, 0, 2, 1>(a, work, nsm, st);
 }
+cudaError_t rk_one0_launch_0021(const EriArgs& a, int blocks, cudaStream_t st) {
+  return rk_one_launch_one<0, 0, 2, 1, 0>(a, blocks, st);
+}
 cudaError_t rk_grad_launch_0011(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<0, 0, 1, 1>(a, work, nsm, st);
+}
+cudaError_t rk_one0_launch_1010(const EriArgs& a, int blocks, cudaStream_t st) {
+  return rk_one_launch_one<1, 0, 1, 0, 0>(a, blocks, st);
 }
 cudaError_t rk_grad_launch_0000(const EriArgs& a, long long work, int nsm, cudaStream_t st) {
   return rk_grad_launch_one<0, 0, 0, 0>(a, work, nsm, st);

@@ -50,6 +50,8 @@ bool rk_grad_available(int la, int lb, int lc, int ld);
 cudaError_t rk_deriv_launch(int la, int lb, int lc, int ld, const EriArgs& a, long long work,
                             int nsm, cudaStream_t st);
 bool rk_deriv_available(int la, int lb, int lc, int ld);
+cudaError_t rk_one_launch(int deriv, int la, int lb, int lc, int ld, const EriArgs& a, int blocks,
+                          cudaStream_t st);
 cudaError_t launch_grad_sum(const double* copies, int ncopies, long long stride, int n, double* g,
                             cudaStream_t st);
 cudaError_t launch_jk_records(const PrimPairRec* pp, const int* src, long long n,
@@ -2433,6 +2435,7 @@ lgx_status lgx_create(lgx_context** out, int device) {
     CK(c->errflag.ensure(64));
     CK(c->primcount.ensure(64));
     CK(cudaMemset(c->errflag.p, 0, 64));
+    CK(cudaMemset(c->counter.p, 0, 64));
   }
   *out = ctx.release();
   return LGX_OK;
@@ -2544,8 +2547,21 @@ lgx_status shellset_locked(lgx_context* ctx, const lgx_shell shells[4], int deri
   a.counter = ctx->counter.as<unsigned long long>();  // not read: one chunk
   a.out = ctx->out.as<double>();
   a.is_null = reinterpret_cast<int*>(a.out + nv * ns);
-  s = run_eri(ctx, ctx->small, *P, kModeStore, false, a, 1, double(np[0] * np[1]) * (np[2] * np[3]));
-  if (s != LGX_OK) return s;
+  const int nq = np[0] * np[1] * np[2] * np[3];
+  if (nq > 1 && rk_eligible(ctx, B, *P, kModeStore, false)) {
+    // the register classes' quartet over several blocks (rk_one_kernel); 16
+    // blocks of at most 1024 sums; the ticket is the context's second counter,
+    // zero from creation on
+    const int blocks = std::min(16, (nq + 127) / 128);
+    CK(ctx->gscratch.ensure(size_t(blocks) * 1024 * sizeof(double)));
+    fill_common(ctx, B, a);
+    a.gscratch = ctx->gscratch.p;
+    a.counter = ctx->counter.as<unsigned long long>() + 1;
+    CK(rk_one_launch(deriv, seg.la, seg.lb, seg.lc, seg.ld, a, blocks, ctx->stream));
+  } else {
+    s = run_eri(ctx, ctx->small, *P, kModeStore, false, a, 1, double(nq));
+    if (s != LGX_OK) return s;
+  }
   int nul = 0;
   const bool pinned = nb + sizeof(double) <= kPinOut;
   unsigned char* h = ctx->pin + kPinIn;

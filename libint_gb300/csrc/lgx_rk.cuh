@@ -372,6 +372,34 @@ struct RkChunks {
   }
 };
 
+// Stores one shell set in the caller's order, the elements split between G lanes.
+template <class C, typename T>
+__device__ __forceinline__ void rk_store_set(const EriArgs& a, int flags, long long outoff,
+                                             const T* v, int G, int g) {
+  constexpr int N0 = C::kN0, N1 = C::kN1, N2 = C::kN2, N3 = C::kN3;
+  const int fl = flags >> 2;
+  const bool sbk = fl & 1, stb = (fl >> 1) & 1, stk = (fl >> 2) & 1;
+  int perm[4];
+  perm[0] = sbk ? (stk ? 3 : 2) : (stb ? 1 : 0);
+  perm[1] = sbk ? (stk ? 2 : 3) : (stb ? 0 : 1);
+  perm[2] = sbk ? (stb ? 1 : 0) : (stk ? 3 : 2);
+  perm[3] = sbk ? (stb ? 0 : 1) : (stk ? 2 : 3);
+  const int dims[4] = {N0, N1, N2, N3};
+  int tn[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) tn[perm[t]] = dims[t];
+  double* o = a.out + outoff;
+#pragma unroll
+  for (int e = 0; e < C::kNsph; ++e) {
+    if ((e & (G - 1)) != g) continue;
+    const int ci[4] = {e / (N1 * N2 * N3), (e / (N2 * N3)) % N1, (e / N3) % N2, e % N3};
+    int it[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) it[perm[t]] = ci[t];
+    o[((it[0] * tn[1] + it[1]) * tn[2] + it[2]) * tn[3] + it[3]] = rk_f64(v[e]);
+  }
+}
+
 // ATT: attenuated operator (erf / erfc, EriArgs::op), J/K mode only; the
 // Coulomb instances (ATT = false) carry none of its code.
 template <typename T, int LA, int LB, int LC, int LD, int MODE, bool ATT = false>
@@ -497,27 +525,7 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
       for (int e = 0; e < C::kNsph; ++e) mx = fmax(mx, fabs(rk_f64(v[e])));
       if (g == 0) a.kschwarz[outoff] = sqrt(mx);
     } else if (mode_store(MODE)) {
-      const int fl = flags >> 2;
-      const bool sbk = fl & 1, stb = (fl >> 1) & 1, stk = (fl >> 2) & 1;
-      int perm[4];
-      perm[0] = sbk ? (stk ? 3 : 2) : (stb ? 1 : 0);
-      perm[1] = sbk ? (stk ? 2 : 3) : (stb ? 0 : 1);
-      perm[2] = sbk ? (stb ? 1 : 0) : (stk ? 3 : 2);
-      perm[3] = sbk ? (stb ? 0 : 1) : (stk ? 2 : 3);
-      const int dims[4] = {N0, N1, N2, N3};
-      int tn[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) tn[perm[t]] = dims[t];
-      double* o = a.out + outoff;
-#pragma unroll
-      for (int e = 0; e < C::kNsph; ++e) {
-        if ((e & (G - 1)) != g) continue;
-        const int ci[4] = {e / (N1 * N2 * N3), (e / (N2 * N3)) % N1, (e / N3) % N2, e % N3};
-        int it[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) it[perm[t]] = ci[t];
-        o[((it[0] * tn[1] + it[1]) * tn[2] + it[2]) * tn[3] + it[3]] = rk_f64(v[e]);
-      }
+      rk_store_set<C>(a, flags, outoff, v, G, g);
     } else if (mode_jk(MODE)) {
       const T deg = T((q.sh[0] == q.sh[1] ? 1 : 2) * (q.sh[2] == q.sh[3] ? 1 : 2) *
                       (bpair == kpair ? 1 : 2));

@@ -227,6 +227,46 @@ __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
   if (a.prim_count && my_prims) atomicAdd(a.prim_count, my_prims);
 }
 
+// Stores the twelve derivative sets of one quartet from its accumulators, the
+// elements split between G lanes.
+template <class C>
+__device__ __forceinline__ void rk_store_deriv(const EriArgs& a, const QuartetItem& it,
+                                               const RkQuartet<double>& q, const double* I, int G,
+                                               int g) {
+  constexpr int N0 = C::kN0, N1 = C::kN1, N2 = C::kN2, N3 = C::kN3, N = C::kNsph;
+  double v[9 * N];
+  C::template sets<double>(I, q.AB, q.CD, v);
+  const int fl = it.flags >> 2;
+  const bool sbk = fl & 1, stb = (fl >> 1) & 1, stk = (fl >> 2) & 1;
+  // canonical position -> caller position, and the strides there
+  const int perm[4] = {sbk ? (stk ? 3 : 2) : (stb ? 1 : 0), sbk ? (stk ? 2 : 3) : (stb ? 0 : 1),
+                       sbk ? (stb ? 1 : 0) : (stk ? 3 : 2), sbk ? (stb ? 0 : 1) : (stk ? 2 : 3)};
+  const int dims[4] = {N0, N1, N2, N3};
+  int str[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    str[t] = 1;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (perm[u] > perm[t]) str[t] *= dims[u];
+  }
+  double* o = a.out + it.out;
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    if ((e & (G - 1)) != g) continue;
+    double* oe = o + (e / (N1 * N2 * N3)) * str[0] + ((e / (N2 * N3)) % N1) * str[1] +
+                 ((e / N3) % N2) * str[2] + (e % N3) * str[3];
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      const double dA = v[s * N + e], dB = v[(3 + s) * N + e], dD = v[(6 + s) * N + e];
+      oe[(size_t)(perm[0] * 3 + s) * N] = dA;
+      oe[(size_t)(perm[1] * 3 + s) * N] = dB;
+      oe[(size_t)(perm[2] * 3 + s) * N] = -(dA + dB + dD);
+      oe[(size_t)(perm[3] * 3 + s) * N] = dD;
+    }
+  }
+}
+
 // First-derivative shell sets of an explicit list, G lanes per quartet: the
 // accumulators of gen_grad.py's DerivCls in registers, the twelve sets written
 // in the caller's order (centre C by translational invariance).
@@ -239,7 +279,6 @@ __global__ void __launch_bounds__(128, 2) rk_grad_kernel(EriArgs a) {
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(128, 2) rk_deriv_kernel(EriArgs a) {
   using C = rk::DerivCls<LA, LB, LC, LD>;
-  constexpr int N0 = C::kN0, N1 = C::kN1, N2 = C::kN2, N3 = C::kN3, N = C::kNsph;
   const int G = a.group;
   const int lane = threadIdx.x & 31;
   const int g = lane & (G - 1);
@@ -287,38 +326,127 @@ __global__ void __launch_bounds__(128, 2) rk_deriv_kernel(EriArgs a) {
     }
     if (a.is_null && g == 0) a.is_null[it.pad] = kept == 0 ? 1 : 0;
     if (kept == 0) continue;
-    double v[9 * N];
-    C::template sets<double>(I, q.AB, q.CD, v);
-    const int fl = it.flags >> 2;
-    const bool sbk = fl & 1, stb = (fl >> 1) & 1, stk = (fl >> 2) & 1;
-    // canonical position -> caller position, and the strides there
-    const int perm[4] = {sbk ? (stk ? 3 : 2) : (stb ? 1 : 0), sbk ? (stk ? 2 : 3) : (stb ? 0 : 1),
-                         sbk ? (stb ? 1 : 0) : (stk ? 3 : 2), sbk ? (stb ? 0 : 1) : (stk ? 2 : 3)};
-    const int dims[4] = {N0, N1, N2, N3};
-    int str[4];
+    rk_store_deriv<C>(a, it, q, I, G, g);
+  }
+}
+
+// One quartet over several blocks: every thread takes its own primitive
+// quartets, a block adds its threads' accumulators through shared memory and puts
+// the sums to a.gscratch; the block that comes last (a.error_flag is not touched;
+// the ticket a.counter counts blocks and is left at zero) adds the blocks' sums,
+// transforms and stores.
+//
+// What bounds it: one scheduler's FP64 rate, 64 cycles a warp instruction, so a
+// single warp needed 77 us for the 81 primitive quartets of a (pp|pp) set and 40%
+// of that went into the shuffled sums.  One warp a scheduler and a column of the
+// accumulators per thread afterwards: 4 warps a block, as many blocks as give each
+// thread one primitive quartet (16 at most).
+template <int LA, int LB, int LC, int LD, int DERIV>
+__global__ void __launch_bounds__(128, 1) rk_one_kernel(EriArgs a) {
+  using Cd = rk::DerivCls<DERIV ? LA : 0, DERIV ? LB : 0, DERIV ? LC : 0, DERIV ? LD : 0>;
+  using Ce = rk::Cls<LA, LB, LC, LD>;
+  constexpr int NA = DERIV ? Cd::kNacc : Ce::kNacc;
+  constexpr int MM = DERIV ? Cd::kMmax : Ce::kMmax;
+  extern __shared__ double s_acc[];  // [rows][NA + 1]
+  __shared__ int s_kept;
+  __shared__ unsigned s_last;
+  const int tid = threadIdx.x;
+  const QuartetItem it = a.items[0];
+  RkQuartet<double> q;
+  rk_load<double>(a, it.bra_pair, it.ket_pair, it.flags & 1, (it.flags >> 1) & 1, q);
+  PrimScreen scr;
+  scr.prec = a.precision;
+  scr.ln_prec = a.ln_prec;
+  scr.fprec = a.fprecision;
+  scr.fln_prec = a.fln_prec;
+  if (tid == 0) s_kept = 0;
+  __syncthreads();
+  double I[NA];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      str[t] = 1;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (perm[u] > perm[t]) str[t] *= dims[u];
-    }
-    double* o = a.out + it.out;
-#pragma unroll
-    for (int e = 0; e < N; ++e) {
-      if ((e & (G - 1)) != g) continue;
-      double* oe = o + (e / (N1 * N2 * N3)) * str[0] + ((e / (N2 * N3)) % N1) * str[1] +
-                   ((e / N3) % N2) * str[2] + (e % N3) * str[3];
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const double dA = v[s * N + e], dB = v[(3 + s) * N + e], dD = v[(6 + s) * N + e];
-        oe[(size_t)(perm[0] * 3 + s) * N] = dA;
-        oe[(size_t)(perm[1] * 3 + s) * N] = dB;
-        oe[(size_t)(perm[2] * 3 + s) * N] = -(dA + dB + dD);
-        oe[(size_t)(perm[3] * 3 + s) * N] = dD;
+  for (int i = 0; i < NA; ++i) I[i] = 0.0;
+  const int nq = q.nbpp * q.nkpp;
+  int kept = 0;
+  for (int p = blockIdx.x * 128 + tid; p < nq; p += gridDim.x * 128) {
+    const int ib = p / q.nkpp, ik = p - ib * q.nkpp;
+    if constexpr (DERIV) {
+      double F[MM + 1];
+      rk::Geo<double> geo;
+      if (rk_prologue<MM>(a, q, ib, ik, scr, F, geo)) {
+        ++kept;
+        const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
+        const PrimPairRec& kp = a.pprims[q.ket_pp + ik];
+        const double w[3] = {q.bsw ? bp.ta2 : bp.ta1, q.bsw ? bp.ta1 : bp.ta2,
+                             q.ksw ? kp.ta1 : kp.ta2};
+        Cd::template prim<double>(F, geo, w, I);
       }
+    } else {
+      kept += rk_prim<Ce, false>(a, q, ib, ik, scr, I) ? 1 : 0;
     }
   }
+  const int rows = min(128, nq);
+  if (tid < rows) {
+#pragma unroll
+    for (int i = 0; i < NA; ++i) s_acc[tid * (NA + 1) + i] = I[i];
+  }
+  if (kept) atomicAdd(&s_kept, kept);
+  __syncthreads();
+  double* part = reinterpret_cast<double*>(a.gscratch);
+  for (int i = tid; i < NA; i += 128) {
+    // four running sums: the chain of dependent additions is what takes time
+    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+    int r = 0;
+    for (; r + 4 <= rows; r += 4) {
+      s0 += s_acc[r * (NA + 1) + i];
+      s1 += s_acc[(r + 1) * (NA + 1) + i];
+      s2 += s_acc[(r + 2) * (NA + 1) + i];
+      s3 += s_acc[(r + 3) * (NA + 1) + i];
+    }
+    for (; r < rows; ++r) s0 += s_acc[r * (NA + 1) + i];
+    part[(size_t)blockIdx.x * (NA + 1) + i] = (s0 + s1) + (s2 + s3);
+  }
+  if (tid == 0) part[(size_t)blockIdx.x * (NA + 1) + NA] = double(s_kept);
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(a.counter, 1ull) == gridDim.x - 1 ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (tid == 0) *a.counter = 0;
+  for (int i = tid; i <= NA; i += 128) {
+    double s = 0;
+    for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(part + (size_t)b * (NA + 1) + i);
+    s_acc[i] = s;
+  }
+  __syncthreads();
+  if (tid >= 32) return;
+  const bool null = !(s_acc[NA] > 0.0);
+  if (a.is_null && tid == 0) a.is_null[it.pad] = null ? 1 : 0;
+  if (null) return;
+#pragma unroll
+  for (int i = 0; i < NA; ++i) I[i] = s_acc[i];
+  if constexpr (DERIV) {
+    rk_store_deriv<Cd>(a, it, q, I, 32, tid);
+  } else {
+    double cart[Ce::kNcart];
+    Ce::template hrr<double>(I, q.AB, q.CD, cart);
+    double v[Ce::kNsph];
+    Ce::template sph<double>(cart, v);
+    rk_store_set<Ce>(a, it.flags, it.out, v, 32, tid);
+  }
+}
+
+template <int LA, int LB, int LC, int LD, int DERIV>
+cudaError_t rk_one_launch_one(const EriArgs& a, int blocks, cudaStream_t st) {
+  constexpr int NA = DERIV ? rk::DerivCls<DERIV ? LA : 0, DERIV ? LB : 0, DERIV ? LC : 0,
+                                          DERIV ? LD : 0>::kNacc
+                           : rk::Cls<LA, LB, LC, LD>::kNacc;
+  static_assert(128 * (NA + 1) * sizeof(double) <= 227 * 1024, "accumulators of one block");
+  auto k = rk_one_kernel<LA, LB, LC, LD, DERIV>;
+  const size_t smem = size_t(128) * (NA + 1) * sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k<<<blocks, 128, smem, st>>>(a);
+  return cudaGetLastError();
 }
 
 template <class K>
