@@ -897,6 +897,20 @@ lgx_status run_block_store(lgx_context* ctx, BasisDev& B, const ProgDev& P, EriA
   const size_t slot_bytes = size_t(a.slot_stride) * sizeof(double);
   const size_t smem_cap = std::min<size_t>(ctx->smem_optin, 200 * 1024);
   const int grid = int(std::max<long long>(1, nwork));
+  // scratch of the transform: the program's own for one set; for the sets of a
+  // phase together, behind everything else in shared memory
+  const int nsets = P.host.sets_per_phase;
+  const size_t tmp_bytes = nsets > 1 ? size_t(nsets) * P.host.ncart4 * sizeof(double) : 0;
+  auto together = [&](size_t smem, size_t slots_at) {
+    if (tmp_bytes == 0 || smem + tmp_bytes > smem_cap) {
+      a.sph_sets = 1;
+      a.sph_tmp = P.host.sph_tmp;
+      return smem;
+    }
+    a.sph_sets = nsets;
+    a.sph_tmp = int((smem - slots_at) / sizeof(double));
+    return smem + tmp_bytes;
+  };
   a.global_slots = 0;
   // small classes: each warp contracts its own primitive quartets (8 staged
   // rows and the accumulators per warp in shared memory), no block-wide
@@ -905,8 +919,8 @@ lgx_status run_block_store(lgx_context* ctx, BasisDev& B, const ProgDev& P, EriA
   if ((kBlockThreads / 32) * per_warp <= smem_cap) {
     a.warp_rows = 1;
     a.stage_rows = 8;
-    CK(launch_eri_block_store(a, grid, (kBlockThreads / 32) * per_warp,
-                              ctx->launch_stream ? ctx->launch_stream : ctx->stream));
+    const size_t smem = together((kBlockThreads / 32) * per_warp, stage_bytes_per_warp(false, 8));
+    CK(launch_eri_block_store(a, grid, smem, ctx->launch_stream ? ctx->launch_stream : ctx->stream));
     return LGX_OK;
   }
   a.warp_rows = 0;
@@ -921,6 +935,10 @@ lgx_status run_block_store(lgx_context* ctx, BasisDev& B, const ProgDev& P, EriA
     a.gscratch = scr.p;
     a.global_slots = 1;
     smem = stage;
+    a.sph_sets = 1;
+    a.sph_tmp = P.host.sph_tmp;
+  } else {
+    smem = together(smem, stage);
   }
   CK(launch_eri_block_store(a, grid, smem, ctx->launch_stream ? ctx->launch_stream : ctx->stream));
   return LGX_OK;

@@ -475,11 +475,14 @@ __global__ void __launch_bounds__(kBlockThreads) eri_block_store_kernel(EriArgs 
     for (int ph = 0; ph < P.nphases; ++ph) {
       run_post_phase<double, BlockGrp>(P, ph, g, slots, tid);
       const int ctr = P.deriv ? (ph == 0 ? 0 : (ph == 1 ? 1 : 3)) : 0;
-      for (int s = 0; s < P.sets_per_phase; ++s) {
+      // the sets of a phase (x, y, z) together where their scratch fits (a third
+      // of the block-wide waits), else one by one
+      const int ns = a.sph_sets;
+      for (int s0 = 0; s0 < P.sets_per_phase; s0 += ns) {
         int dims[4] = {ncart_of(P.la), ncart_of(P.lb), ncart_of(P.lc), ncart_of(P.ld)};
-        double* cart = slots + P.cart_out + s * P.ncart4;
-        const double* V =
-            sph_transform<double, BlockGrp>(a, lsh, pure, dims, cart, slots + P.sph_tmp, tid);
+        const double* V = sph_transform<double, BlockGrp>(
+            a, lsh, pure, dims, slots + P.cart_out + s0 * P.ncart4, slots + a.sph_tmp, tid, ns,
+            P.ncart4);
         const int nsph4 = dims[0] * dims[1] * dims[2] * dims[3];
         int tn[4];
         for (int t = 0; t < 4; ++t) tn[perm[t]] = dims[t];
@@ -493,17 +496,21 @@ __global__ void __launch_bounds__(kBlockThreads) eri_block_store_kernel(EriArgs 
           for (int t = 0; t < 4; ++t) ix[perm[t]] = ci[t];
           return ((ix[0] * tn[1] + ix[1]) * tn[2] + ix[2]) * tn[3] + ix[3];
         };
-        const int ts = P.deriv ? perm[ctr] * 3 + s : 0;
-        double* o = a.out + it.out + (size_t)ts * nsph4;
-        double* cb = slots + P.cbuf + s * P.ncart4;
-        for (int e = tid; e < nsph4; e += nt) {
-          o[caller_index(e)] = V[e];
-          if (P.deriv) cb[e] = (ph == 0 ? 0.0 : cb[e]) - V[e];
-        }
-        __syncthreads();
-        if (P.deriv && ph == P.nphases - 1) {
-          double* oc = a.out + it.out + (size_t)(perm[2] * 3 + s) * nsph4;
-          for (int e = tid; e < nsph4; e += nt) oc[caller_index(e)] = cb[e];
+        double* cb = slots + P.cbuf;
+        double* o = a.out + it.out;
+        const bool last = P.deriv && ph == P.nphases - 1;
+        for (int f = tid; f < ns * nsph4; f += nt) {
+          const int si = f / nsph4, e = f - si * nsph4, s = s0 + si;
+          const double x = V[(size_t)si * P.ncart4 + e];
+          const int ci = caller_index(e);
+          o[(size_t)(P.deriv ? perm[ctr] * 3 + s : 0) * nsph4 + ci] = x;
+          if (P.deriv) {
+            // one thread owns an element through all phases
+            double* c = cb + (size_t)s * P.ncart4 + e;
+            const double cv = (ph == 0 ? 0.0 : *c) - x;
+            *c = cv;
+            if (last) o[(size_t)(perm[2] * 3 + s) * nsph4 + ci] = cv;
+          }
         }
         __syncthreads();
       }

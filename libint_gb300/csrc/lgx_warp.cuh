@@ -627,13 +627,14 @@ __device__ __forceinline__ float sph_coef(const EriArgs& a, int t, float*) {
   return __ldg(a.sph_cf + t);
 }
 
-// Sparse Cartesian -> solid harmonics for the pure indices, ping-ponging
-// between `cart` and `tmp`.  Each lane owns whole columns (all indices but
-// the transformed one), so the row loops and coefficient reads are
-// warp-uniform (broadcast loads).  Returns the result buffer.
+// Sparse Cartesian -> solid harmonics for the pure indices of nsets sets,
+// sstride apart in `cart` and `tmp`, ping-ponging between the two.  Each lane
+// owns whole columns (all indices but the transformed one), so the row loops and
+// coefficient reads are warp-uniform (broadcast loads).  Returns the result
+// buffer.
 template <typename T, class Grp = WarpGrp>
 __device__ T* sph_transform(const EriArgs& a, const int* l, const int* pure, int* dims, T* cart,
-                            T* tmp, int lane) {
+                            T* tmp, int lane, int nsets = 1, int sstride = 0) {
   T* src = cart;
   T* dst = tmp;
   T* tag = nullptr;
@@ -644,10 +645,11 @@ __device__ T* sph_transform(const EriArgs& a, const int* l, const int* pure, int
     for (int t = 0; t < k; ++t) outer *= dims[t];
     for (int t = k + 1; t < 4; ++t) inner *= dims[t];
     const int ncol = outer * inner;
-    for (int c = lane; c < ncol; c += Grp::size()) {
-      const int o = c / inner, i = c - o * inner;
-      const T* sp = src + (size_t)o * nc * inner + i;
-      T* dp = dst + (size_t)o * np * inner + i;
+    for (int c = lane; c < nsets * ncol; c += Grp::size()) {
+      const int s = nsets > 1 ? c / ncol : 0, cs = c - s * ncol;
+      const int o = cs / inner, i = cs - o * inner;
+      const T* sp = src + (size_t)s * sstride + (size_t)o * nc * inner + i;
+      T* dp = dst + (size_t)s * sstride + (size_t)o * np * inner + i;
       for (int p = 0; p < np; ++p) {
         const int t0 = __ldg(a.sph_off + lk * 9 + p), t1 = __ldg(a.sph_off + lk * 9 + p + 1);
         T v = T(0);
