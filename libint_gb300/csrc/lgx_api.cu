@@ -782,9 +782,6 @@ lgx_status plan_launch(lgx_context* ctx, const ProgDev& P, int mode, bool fp32,
   return LGX_OK;
 }
 
-// Register kernels exist for the generated classes (deriv 0; see
-// codegen/gen_rk.py for the limits per mode) with the standard pure flags;
-// everything else runs on the warp-cooperative program kernel.
 // Context and basis pointers every kernel launch needs.
 void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
   a.basis = B.dev;
@@ -812,6 +809,9 @@ void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
   a.fln_prec = float(std::max(a.ln_prec, -1.0e30));
 }
 
+// Register kernels exist for the generated classes (see codegen/gen_rk.py and
+// gen_grad.py for the limits per mode and derivative order) with the standard
+// pure flags; everything else runs on the program kernel.
 bool rk_eligible(const lgx_context* ctx, const BasisDev& B, const ProgDev& P, int mode,
                  bool fp32) {
   if (!ctx->use_rk || !B.std_pure) return false;
