@@ -852,7 +852,10 @@ int fill_group(const lgx_context* ctx, long long nwork, double nq_avg) {
 Variant default_variant(const lgx_context* ctx, const BasisDev& B, const ProgDev& P, int mode,
                         bool fp32, bool implicit, long long nwork, double nq_avg) {
   Variant v;
-  if (rk_eligible(ctx, B, P, mode, fp32)) {
+  // at most one derivative quartet per SM: eight warps each (the block kernel)
+  // beat the register kernel's one (40 quartets of cc-pVDZ: 240 us and 404)
+  const bool few = P.host.deriv && mode == kModeStore && !implicit && nwork <= ctx->nsm;
+  if (!few && rk_eligible(ctx, B, P, mode, fp32)) {
     v.kind = 0;
     v.group = implicit ? fill_group(ctx, nwork, nq_avg) : choose_group(nq_avg);
   } else {
@@ -1056,7 +1059,8 @@ void list_segments(const lgx_context* ctx, const BasisDev& B, int deriv, int mod
     const bool att = ctx->op != LGX_OP_COULOMB;
     const bool cut =
         ctx->use_rk && B.std_pure && mode == kModeStore && !seg.fp32 &&
-        (deriv ? !att && rk_deriv_available(seg.la, seg.lb, seg.lc, seg.ld)
+        (deriv ? !att && count > size_t(ctx->nsm) &&
+                     rk_deriv_available(seg.la, seg.lb, seg.lc, seg.ld)
                : rk_available(false, mode, att, seg.la, seg.lb, seg.lc, seg.ld));
     if (!cut) {
       plan.segs.push_back(seg);
@@ -2566,7 +2570,7 @@ lgx_status shellset_locked(lgx_context* ctx, const lgx_shell shells[4], int deri
   a.out = ctx->out.as<double>();
   a.is_null = reinterpret_cast<int*>(a.out + nv * ns);
   const int nq = np[0] * np[1] * np[2] * np[3];
-  if (nq > 1 && rk_eligible(ctx, B, *P, kModeStore, false)) {
+  if ((nq > 1 || deriv) && rk_eligible(ctx, B, *P, kModeStore, false)) {
     // the register classes' quartet over several blocks (rk_one_kernel); 16
     // blocks of at most 1024 sums; the ticket is the context's second counter,
     // zero from creation on
