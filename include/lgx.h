@@ -55,10 +55,10 @@ typedef int lgx_status;
 /* Precision modes of the batched paths.  In both mixed modes a quartet whose
  * Schwarz bound K12*K34 is below mixed_thresh runs its VRR, HRR, contraction
  * and solid-harmonic transform in FP32, every other quartet entirely in FP64,
- * and J/K are accumulated in FP64.  LGX_MIXED keeps the Boys function of
- * the FP32 quartets in FP64 (its argument T, the Taylor or asymptotic
- * branch, e^{-T} and the downward recursion; Coulomb operator);
- * LGX_MIXED_FP32_BOYS evaluates it in FP32 as well (faster, less exact). */
+ * and J/K are accumulated in FP64.  LGX_MIXED takes the Boys function of
+ * the FP32 quartets to FP32 rounding (its argument T in double-float
+ * arithmetic, each F_m rounded once; Coulomb operator);
+ * LGX_MIXED_FP32_BOYS evaluates both in FP32 (less exact). */
 #define LGX_FP64 0
 #define LGX_MIXED 1
 #define LGX_MIXED_FP32_BOYS 2

@@ -312,8 +312,8 @@ lgx_status fail(lgx_context* c, lgx_status s, const std::string& msg) {
 
 // Precision modes (LGX_FP64, LGX_MIXED, LGX_MIXED_FP32_BOYS): whether a pass
 // splits off an FP32 space, and the kernel mode of its FP32 launches.  The
-// mixed scheme's FP32 kernels evaluate the Boys function in FP64 for the
-// Coulomb operator; the attenuated operators' FP32 kernels keep it in FP32.
+// mixed scheme's FP32 kernels take the Boys function to FP32 rounding for the
+// Coulomb operator; the attenuated operators' FP32 kernels evaluate it in FP32.
 bool mixed_mode(int mode) { return mode == LGX_MIXED || mode == LGX_MIXED_FP32_BOYS; }
 bool valid_mode(int mode) { return mode == LGX_FP64 || mixed_mode(mode); }
 int fp32_kernel_mode(const lgx_context* ctx, int mode, int base_mode) {
@@ -1595,8 +1595,8 @@ void bin_args(const BinCache& C, const BinHost& bin, int sp, EriArgs& a) {
 // quartets for the register and 2^14 for the program kernels: with 2^22 and
 // 2^17 the tuning of (H2O)32 cc-pVDZ took five passes' time.
 // mode32: kernel mode of the FP32 precision space (kModeJK, or kModeJKB64
-// for the mixed scheme with the Boys function in FP64), or -1 when the pass
-// runs every quartet in FP64.
+// for the mixed scheme with the Boys function to FP32 rounding), or -1 when the
+// pass runs every quartet in FP64.
 lgx_status tune_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int mode32,
                      EriArgs base) {
   if (!ctx->tune || ctx->noalloc) return LGX_OK;
