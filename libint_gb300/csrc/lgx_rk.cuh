@@ -207,9 +207,9 @@ __device__ __forceinline__ PrimF32 rk_pp32(const PrimPairRec& r, bool sw) {
 // One primitive quartet into acc (FP32).  AC = A - C of the quartet.
 // bidx, kidx: the two primitive pairs' PrimPairRec indices (the FP64
 // values of the screening decisions inside the rounding band).
-// FUSE: fused accumulation, for kernels that hand out sums over quartets; the
-// store kernels keep the rounding of the single sums.
-template <class C, bool ATT, bool FUSE>
+// The sums keep their single roundings (vrr, not vrr_fused): with FP32 Boys
+// values the mode's results stay those of its store kernels.
+template <class C, bool ATT>
 __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<float>& q,
                                         const PrimF32& bp, const PrimF32& kp, int bidx,
                                         int kidx, const PrimScreen& scr, float* acc) {
@@ -240,10 +240,7 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<float>
   g.oo2e = 0.5f * kp.k.z;
   g.roe = zz;
   g.oo2ze = 0.5f * oogpq;
-  if constexpr (FUSE)
-    C::template vrr_fused<float>(F, g, acc);
-  else
-    C::template vrr<float>(F, g, acc);
+  C::template vrr<float>(F, g, acc);
   return true;
 }
 
@@ -488,9 +485,7 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
                       ? 1
                       : 0;
         } else {
-          kept += rk_prim<C, ATT, mode_jk(MODE)>(a, q, bp, kp, q.bra_pp + ib, q.ket_pp + ik, scr, acc)
-                      ? 1
-                      : 0;
+          kept += rk_prim<C, ATT>(a, q, bp, kp, q.bra_pp + ib, q.ket_pp + ik, scr, acc) ? 1 : 0;
         }
       } else {
         kept += rk_prim<C, ATT>(a, q, ib, ik, scr, acc) ? 1 : 0;
