@@ -161,9 +161,9 @@ class Shell:
 
     def _pack(self, arr, k: int):
         """Writes the shell into entry k of an array of LgxShell."""
-        x, y, z = self.O.tolist()
+        O = self.O  # any indexable sequence of numbers
         _lgx.SHELL_STRUCT.pack_into(arr, k * _lgx.SHELL_STRUCT.size, self.l,
-                                    1 if self.pure else 0, len(self.alpha), 0, x, y, z,
+                                    1 if self.pure else 0, len(self.alpha), 0, O[0], O[1], O[2],
                                     _lgx.address(self.alpha), _lgx.address(self.coeff))
 
     def __repr__(self):
