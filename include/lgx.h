@@ -103,11 +103,13 @@ lgx_status lgx_set_operator(lgx_context* ctx, int op, double omega);
  * evaluated on the GPU by exactly the device function a class kernel uses:
  * variant 0 the program kernels' FP64 evaluator (mmax <= 16), 1 the
  * register kernels' FP64 evaluator (mmax <= 6), 2 and 3 their FP32
- * counterparts, 4 and 5 the LGX_MIXED scheme's FP64 evaluators of the
- * program and register store kernels (4-term series, T as a double-float pair,
- * each value rounded to FP32; mmax <= 16 and <= 6), 6 the register
- * kernels' whole LGX_MIXED path from primitive-pair data: T then holds 8
- * values per argument (Pb.x, Pb.y, Pb.z, zeta, Pk.x, Pk.y, Pk.z, eta;
+ * counterparts.  4 to 9 are the LGX_MIXED scheme's evaluators, T as a
+ * double-float pair and each value rounded to FP32: 4 and 5 those of the
+ * program and register store kernels (FP64, 4-term series; mmax <= 16 and
+ * <= 6), 7 and 8 those of the program and register J/K kernels (leading and
+ * correction part in FP32; mmax <= 16 and <= 6).  6 and 9 are the whole path
+ * of the register store and J/K kernels from primitive-pair data: T then
+ * holds 8 values per argument (Pb.x, Pb.y, Pb.z, zeta, Pk.x, Pk.y, Pk.z, eta;
  * |P| <= 1e4, 1e-10 <= zeta <= 1e10) and the argument is rho |Pb - Pk|^2,
  * rho = zeta eta / (zeta + eta), formed as those kernels form it
  * (double-float records and arithmetic).  All results widened to double.

@@ -35,9 +35,8 @@ cudaError_t launch_list_scatter(const ListArgs& a, cudaStream_t st);
 cudaError_t launch_d2f(const double* src, float* dst, long long n, cudaStream_t st);
 cudaError_t launch_shell_block_norm(const DevBasis& b, const double* D, int nbf, double* out,
                                     cudaStream_t st);
-cudaError_t launch_boys_eval(const double* tab, const double* tay, const double* fine,
-                             const float* tab32, const double* inv_odd, int variant,
-                             const double* T, long long n, int mmax, double* F, cudaStream_t st);
+cudaError_t launch_boys_eval(const BoysTables& t, int variant, const double* T, long long n,
+                             int mmax, double* F, cudaStream_t st);
 cudaError_t launch_boys_fine(const double* hi, const double* lo, double* fine, cudaStream_t st);
 cudaError_t launch_prim_set(const PrimSetArgs& a, size_t smem, cudaStream_t st);
 cudaError_t launch_eri_block_store(const EriArgs& a, int grid, size_t smem, cudaStream_t st);
@@ -3080,14 +3079,16 @@ lgx_status lgx_boys(lgx_context* ctx, int variant, const double* T, int64_t n, i
                     double* F) {
   if (!ctx) return LGX_ERR_INVALID_ARG;
   std::lock_guard<std::mutex> lk(ctx->mu);
-  if (variant < 0 || variant > 6) return fail(ctx, LGX_ERR_INVALID_ARG, "bad Boys variant");
-  const int mmax_cap = (variant == 1 || variant == 3 || variant >= 5) ? 6 : kBoysMaxM;
+  if (variant < 0 || variant > 9) return fail(ctx, LGX_ERR_INVALID_ARG, "bad Boys variant");
+  const bool program = variant == 0 || variant == 2 || variant == 4 || variant == 7;
+  const int mmax_cap = program ? kBoysMaxM : 6;
   if (mmax < 0 || mmax > mmax_cap)
     return fail(ctx, LGX_ERR_INVALID_ARG, "mmax out of range for this evaluator");
   if (n < 0 || (n > 0 && (!T || !F))) return fail(ctx, LGX_ERR_INVALID_ARG, "bad arrays");
   if (n == 0) return LGX_OK;
-  const int64_t nin = variant == 6 ? 8 * n : n;  // variant 6: pair data per argument
-  if (variant == 6) {
+  const bool pairs = variant == 6 || variant == 9;  // pair data per argument
+  const int64_t nin = pairs ? 8 * n : n;
+  if (pairs) {
     // |P| <= 1e4 bohr, 1e-10 <= zeta <= 1e10: the double-float records'
     // range (and a Boys argument that stays finite)
     for (int64_t i = 0; i < n; ++i)
@@ -3107,10 +3108,11 @@ lgx_status lgx_boys(lgx_context* ctx, int variant, const double* T, int64_t n, i
   CK(ctx->boysF.ensure(nf * sizeof(double)));
   CK(cudaMemcpyAsync(ctx->boysT.p, T, size_t(nin) * sizeof(double), cudaMemcpyHostToDevice,
                      ctx->stream));
-  CK(launch_boys_eval(ctx->boys.as<double>(), ctx->boys_tay.as<double>(),
-                      ctx->boys_fine.as<double>(), ctx->boys32.as<float>(),
-                      ctx->inv_odd.as<double>(), variant, ctx->boysT.as<double>(), n, mmax,
-                      ctx->boysF.as<double>(), ctx->stream));
+  const BoysTables tabs{ctx->boys.as<double>(),  ctx->boys_tay.as<double>(),
+                        ctx->boys_fine.as<double>(), ctx->boys32.as<float>(),
+                        ctx->boys_split.as<float>(), ctx->inv_odd.as<double>()};
+  CK(launch_boys_eval(tabs, variant, ctx->boysT.as<double>(), n, mmax, ctx->boysF.as<double>(),
+                      ctx->stream));
   CK(cudaMemcpyAsync(F, ctx->boysF.p, nf * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   return LGX_OK;

@@ -29,6 +29,16 @@ __host__ __device__ constexpr int mode_boys(int m) {
   return m == kModeJKB64 ? 2 : (m == kModeStoreB64 ? 1 : 0);
 }
 
+// Tables of the Boys evaluators (EriArgs) as lgx_boys hands them on.
+struct BoysTables {
+  const double* tab;
+  const double* tay;
+  const double* fine;
+  const float* tab32;
+  const float* split;
+  const double* inv_odd;
+};
+
 // Explicit work item: one shell quartet in canonical orientation.
 struct QuartetItem {
   int bra_pair, ket_pair;  // pair-table indices
