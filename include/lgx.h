@@ -112,7 +112,10 @@ lgx_status lgx_set_operator(lgx_context* ctx, int op, double omega);
  * holds 8 values per argument (Pb.x, Pb.y, Pb.z, zeta, Pk.x, Pk.y, Pk.z, eta;
  * |P| <= 1e4, 1e-10 <= zeta <= 1e10) and the argument is rho |Pb - Pk|^2,
  * rho = zeta eta / (zeta + eta), formed as those kernels form it
- * (double-float records and arithmetic).  All results widened to double.
+ * (double-float records and arithmetic).  10 is the register J/K kernels' FP64
+ * step of the context's attenuated operator (mmax <= 6): T then holds T and rho
+ * of each argument, F the core integrals s^{m+1/2} F_m(s T) (erf) or F_m(T) less
+ * those (erfc), s = omega^2 / (omega^2 + rho).  All results widened to double.
  * The batch counterpart of libint's FmEval_Taylor / FmEval_Chebyshev7
  * eval(F, T, mmax)
  * (include/libint2/boys.h:345-454,679-821), so the evaluators can be

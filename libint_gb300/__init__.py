@@ -319,9 +319,11 @@ class Context:
         `variant` (lgx_boys: 0/1 FP64 program/register kernel, 2/3 FP32,
         4/5 the mixed scheme's store kernels, 7/8 its J/K kernels; 6 and 9:
         T is an (n, 8) array of pair data Pb.xyz, zeta, Pk.xyz, eta, the whole
-        path of the mixed register store and J/K kernels)."""
+        path of the mixed register store and J/K kernels; 10: T is an (n, 2)
+        array of T and rho, the core integrals of the context's attenuated
+        operator)."""
         T = np.ascontiguousarray(T, np.float64)
-        n = T.shape[0] if int(variant) in (6, 9) else T.size
+        n = T.shape[0] if int(variant) in (6, 9, 10) else T.size
         T = T.reshape(-1)
         F = np.zeros((n, int(mmax) + 1))
         self._check(self._lib.lgx_boys(self._h, int(variant), _lgx.ptr(T), n, int(mmax),

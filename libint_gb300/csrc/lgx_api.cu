@@ -802,7 +802,6 @@ void fill_common(const lgx_context* ctx, const BasisDev& B, EriArgs& a) {
   a.sph_cf = ctx->sph_cf.as<float>();
   a.error_flag = ctx->errflag.as<int>();
   a.op = ctx->op;
-  a.omega = ctx->omega;
   a.omega2 = ctx->omega * ctx->omega;
   a.fprecision = float(a.precision);
   a.fln_prec = float(std::max(a.ln_prec, -1.0e30));
@@ -3079,7 +3078,7 @@ lgx_status lgx_boys(lgx_context* ctx, int variant, const double* T, int64_t n, i
                     double* F) {
   if (!ctx) return LGX_ERR_INVALID_ARG;
   std::lock_guard<std::mutex> lk(ctx->mu);
-  if (variant < 0 || variant > 9) return fail(ctx, LGX_ERR_INVALID_ARG, "bad Boys variant");
+  if (variant < 0 || variant > 10) return fail(ctx, LGX_ERR_INVALID_ARG, "bad Boys variant");
   const bool program = variant == 0 || variant == 2 || variant == 4 || variant == 7;
   const int mmax_cap = program ? kBoysMaxM : 6;
   if (mmax < 0 || mmax > mmax_cap)
@@ -3087,7 +3086,9 @@ lgx_status lgx_boys(lgx_context* ctx, int variant, const double* T, int64_t n, i
   if (n < 0 || (n > 0 && (!T || !F))) return fail(ctx, LGX_ERR_INVALID_ARG, "bad arrays");
   if (n == 0) return LGX_OK;
   const bool pairs = variant == 6 || variant == 9;  // pair data per argument
-  const int64_t nin = pairs ? 8 * n : n;
+  const int64_t nin = pairs ? 8 * n : (variant == 10 ? 2 * n : n);
+  if (variant == 10 && ctx->op == LGX_OP_COULOMB)
+    return fail(ctx, LGX_ERR_INVALID_ARG, "variant 10 needs an attenuated operator");
   if (pairs) {
     // |P| <= 1e4 bohr, 1e-10 <= zeta <= 1e10: the double-float records'
     // range (and a Boys argument that stays finite)
@@ -3098,7 +3099,7 @@ lgx_status lgx_boys(lgx_context* ctx, int variant, const double* T, int64_t n, i
         if (!ok) return fail(ctx, LGX_ERR_INVALID_ARG, "pair data out of range");
       }
   } else {
-    for (int64_t i = 0; i < n; ++i)  // the table lookup needs 0 <= T (NaN rejected too)
+    for (int64_t i = 0; i < nin; ++i)  // the table lookup needs 0 <= T (NaN rejected too)
       if (!(T[i] >= 0.0) || !std::isfinite(T[i]))
         return fail(ctx, LGX_ERR_INVALID_ARG, "Boys argument T must be finite and >= 0");
   }
@@ -3110,7 +3111,8 @@ lgx_status lgx_boys(lgx_context* ctx, int variant, const double* T, int64_t n, i
                      ctx->stream));
   const BoysTables tabs{ctx->boys.as<double>(),  ctx->boys_tay.as<double>(),
                         ctx->boys_fine.as<double>(), ctx->boys32.as<float>(),
-                        ctx->boys_split.as<float>(), ctx->inv_odd.as<double>()};
+                        ctx->boys_split.as<float>(), ctx->inv_odd.as<double>(), ctx->op,
+                        ctx->omega * ctx->omega};
   CK(launch_boys_eval(tabs, variant, ctx->boysT.as<double>(), n, mmax, ctx->boysF.as<double>(),
                       ctx->stream));
   CK(cudaMemcpyAsync(F, ctx->boysF.p, nf * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

@@ -61,6 +61,14 @@ __device__ void rk_boys_pairs(const BoysTables& t, int variant, const double* pz
   for (int m = 0; m <= MMAX; ++m) out[m] = double(d2f_int(f[m]));
 }
 
+// Variant 10: the register J/K kernels' FP64 step of the attenuated operators
+// for one (T, rho); zero where it reports that the integrals vanish.
+template <int MMAX>
+__device__ void rk_boys_att_to(const BoysTables& t, const double* arg, double* out) {
+  if (!rk_boys_att<MMAX>(t.fine, t.op, t.omega2, arg[0], arg[1], 1.0, out))
+    for (int m = 0; m <= MMAX; ++m) out[m] = 0.0;
+}
+
 // Fine tables from the 1/64 grid (hi + lo: the grid values beyond FP64): F_m at
 // fine point j by ten terms of its Taylor series about the nearest coarse point
 // (distance at most 4/512), the sum rounded once.
@@ -111,6 +119,20 @@ __global__ void boys_eval_kernel(BoysTables t, int variant, const double* Targ, 
       case 4: rk_boys_pairs<4>(t, variant, pz, out); break;
       case 5: rk_boys_pairs<5>(t, variant, pz, out); break;
       default: rk_boys_pairs<6>(t, variant, pz, out); break;
+    }
+    for (int m = 0; m <= mmax; ++m) F[i * (mmax + 1) + m] = out[m];
+    return;
+  }
+  if (variant == 10) {
+    const double* arg = Targ + 2 * i;
+    switch (mmax) {
+      case 0: rk_boys_att_to<0>(t, arg, out); break;
+      case 1: rk_boys_att_to<1>(t, arg, out); break;
+      case 2: rk_boys_att_to<2>(t, arg, out); break;
+      case 3: rk_boys_att_to<3>(t, arg, out); break;
+      case 4: rk_boys_att_to<4>(t, arg, out); break;
+      case 5: rk_boys_att_to<5>(t, arg, out); break;
+      default: rk_boys_att_to<6>(t, arg, out); break;
     }
     for (int m = 0; m <= mmax; ++m) F[i * (mmax + 1) + m] = out[m];
     return;

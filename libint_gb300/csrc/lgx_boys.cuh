@@ -132,6 +132,45 @@ __device__ __forceinline__ void rk_boys(const double* __restrict__ fine, double 
   }
 }
 
+// The FP64 Boys step of the attenuated operators (register kernels of the J/K
+// passes): F = the core integrals times pfac, with s = omega^2 / (omega^2 + rho)
+// (libint's erf_coulomb_gm_eval / erfc_coulomb_gm_eval,
+// include/libint2/boys.h:1913-1980)
+//   erf(omega r)/r  (op 1):  s^{m+1/2} F_m(s T)
+//   erfc(omega r)/r (op 2):  F_m(T) - s^{m+1/2} F_m(s T)
+// (s T <= T, so the same grid serves).  s is a division and sqrt(s) a square
+// root: both from one reciprocal square root of omega^2 + rho would double the
+// error of s^{m+1/2} (at m = 4 1.4e-15 instead of 8e-16 of F_m).  erf needs no
+// F_m(T).  Returns false when the integrals vanish: erf at omega = 0, and erfc
+// where s T > 50, as both parts are then asymptotic and equal (their difference
+// is below e^-50 of F_m; evaluated, it is the rounding noise of two equal sums).
+template <int MMAX>
+__device__ __forceinline__ bool rk_boys_att(const double* __restrict__ fine, int op, double omega2,
+                                            double T, double rho, double pfac, double* F) {
+  if (!(omega2 > 0.0)) {
+    if (op == 1) return false;
+    rk_boys<MMAX>(fine, T, pfac, F);
+    return true;
+  }
+  const double s = omega2 / (omega2 + rho);
+  const double sT = s * T;
+  if (op == 2 && d2f_int(sT) > float(kBoysTmax)) return false;
+  double G[MMAX + 1];
+  rk_boys<MMAX>(fine, sT, pfac * sqrt(s), G);
+  if (op == 1) {
+    double f = 1.0;
+#pragma unroll
+    for (int m = 0; m <= MMAX; ++m, f *= s) F[m] = m == 0 ? G[0] : f * G[m];
+    return true;
+  }
+  rk_boys<MMAX>(fine, T, pfac, F);
+  double f = s;
+  F[0] -= G[0];
+#pragma unroll
+  for (int m = 1; m <= MMAX; ++m, f *= s) F[m] = fma(-f, G[m], F[m]);
+  return true;
+}
+
 // The mixed scheme's FP64 Boys function of an FP32 quartet (store kernels), given its
 // argument T = T.hi + T.lo in double-float (ds_boys_arg): the branch and the
 // grid point come from T.hi; the offset md = T_k - T = (T_k - T.hi) - T.lo,

@@ -37,6 +37,8 @@ struct BoysTables {
   const float* tab32;
   const float* split;
   const double* inv_odd;
+  int op;         // attenuated operator and omega^2 (variant 10)
+  double omega2;
 };
 
 // Explicit work item: one shell quartet in canonical orientation.
@@ -162,7 +164,7 @@ struct EriArgs {
   // two-body operator: 0 coulomb 1/r, 1 erf(omega r)/r, 2 erfc(omega r)/r
   // (attenuated: program kernel instantiations and the ATT register kernels)
   int op;
-  double omega, omega2;  // omega and its square
+  double omega2;  // omega^2
   // work
   const QuartetItem* items;
   long long nitems;

@@ -21,46 +21,9 @@ namespace lgx {
 __device__ __forceinline__ double rk_f64(double x) { return x; }
 __device__ __forceinline__ double rk_f64(float x) { return f2d_int(x); }
 
-// Attenuated operators (register kernels of the J/K passes): F holds
-// pfac F_m(T) on entry; with s = omega^2 / (omega^2 + rho) the core
-// integrals become (libint's erf_coulomb_gm_eval / erfc_coulomb_gm_eval,
-// include/libint2/boys.h:1913-1980)
-//   erf(omega r)/r :  s^{m+1/2} F_m(s T)
-//   erfc(omega r)/r:  F_m(T) - s^{m+1/2} F_m(s T)
-// (s T <= T, so the same Taylor grid serves).  omega = 0 gives zero (erf)
-// and the Coulomb integrals (erfc).
-// FP64: the whole Boys step of the attenuated operators, F = the core integrals
-// times pfac.  sqrt(s) and s come from one reciprocal square root; erf needs no
-// F_m(T).  Returns false when they vanish: erf at omega = 0, and erfc where
-// s T > 50, as both parts are then asymptotic and equal (their difference is
-// below e^-50 of F_m; evaluated, it was the rounding noise of two equal sums).
-template <int MMAX>
-__device__ __forceinline__ bool rk_boys_att(const EriArgs& a, double T, double rho, double pfac,
-                                            double* F) {
-  if (!(a.omega2 > 0.0)) {
-    if (a.op == 1) return false;
-    rk_boys<MMAX>(a.boys_fine, T, pfac, F);
-    return true;
-  }
-  const double r = rsqrt64(a.omega2 + rho);
-  const double s = a.omega2 * (r * r);
-  const double sT = s * T;
-  if (a.op == 2 && d2f_int(sT) > float(kBoysTmax)) return false;
-  double G[MMAX + 1];
-  rk_boys<MMAX>(a.boys_fine, sT, pfac * (a.omega * r), G);
-  if (a.op == 1) {
-    double f = 1.0;
-#pragma unroll
-    for (int m = 0; m <= MMAX; ++m, f *= s) F[m] = m == 0 ? G[0] : f * G[m];
-    return true;
-  }
-  rk_boys<MMAX>(a.boys_fine, T, pfac, F);
-  double f = s;
-  F[0] -= G[0];
-#pragma unroll
-  for (int m = 1; m <= MMAX; ++m, f *= s) F[m] = fma(-f, G[m], F[m]);
-  return true;
-}
+// Attenuated operators, FP32: F holds pfac F_m(T) on entry and the core
+// integrals of rk_boys_att on return (s T <= T, so the same Taylor grid serves;
+// omega = 0 gives zero for erf and the Coulomb integrals for erfc).
 template <int MMAX>
 __device__ __forceinline__ void rk_attenuate(const EriArgs& a, float T, float rho, float pfac,
                                              float* F) {
@@ -160,7 +123,7 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<double
   const double T = rho * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
   double F[C::kMmax + 1];
   if constexpr (ATT) {
-    if (!rk_boys_att<C::kMmax>(a, T, rho, pfac, F)) return true;
+    if (!rk_boys_att<C::kMmax>(a.boys_fine, a.op, a.omega2, T, rho, pfac, F)) return true;
   } else {
     rk_boys<C::kMmax>(a.boys_fine, T, pfac, F);
   }
