@@ -77,7 +77,7 @@ __device__ __forceinline__ void rk_boys(const double* __restrict__ fine, double 
   const float Tf = d2f_int(T);
   const bool asym = Tf > float(kBoysTmax);
   if (asym && MMAX <= 2) {
-    const double rs = rsqrt64(T);
+    const double rs = rsqrt(T);
     const double oo2T = 0.5 * (rs * rs);
     double f = (0.88622692545275801365 * pfac) * rs;
     F[0] = f;
@@ -107,7 +107,7 @@ __device__ __forceinline__ void rk_boys(const double* __restrict__ fine, double 
   }
   double s, eTp = 0.0;
   if (asym) {
-    const double rs = rsqrt64(T);
+    const double rs = rsqrt(T);
     const double r2 = rs * rs;
     double c = 0.88622692545275801365;  // (2m-1)!! / 2^m sqrt(pi)/2
 #pragma unroll

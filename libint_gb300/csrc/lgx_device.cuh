@@ -114,17 +114,6 @@ __device__ __forceinline__ float d2f_int(double x) {
   return __uint_as_float(sign | bits);
 }
 
-// 1/sqrt(x), x normal and positive: the special-function unit's estimate r and
-// one step of third order, r + r e (1/2 + 3/8 e) with e = 1 - x r^2 (from an
-// estimate good to 2^-20 the step leaves 2^-60).  Five FP64 instructions, which
-// is what counts in kernels bound by that pipe.
-__device__ __forceinline__ double rsqrt64(double x) {
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-(x * r), r, 1.0);
-  return fma(r * e, fma(e, 0.375, 0.5), r);
-}
-
 // double(n) for a small non-negative integer n < 2^20 with integer
 // operations only.
 __device__ __forceinline__ double i2d_int(int n) {

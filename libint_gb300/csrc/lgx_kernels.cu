@@ -97,7 +97,7 @@ __global__ void ztab_kernel(const double* __restrict__ exps, int nexp, int n,
     while ((e1 + 1) * (e1 + 2) / 2 <= k) ++e1;
     return exps[e1] + exps[k - e1 * (e1 + 1) / 2];
   };
-  const double rs = rsqrt64(zeta(int(t / n)) + zeta(int(t % n)));
+  const double rs = rsqrt(zeta(int(t / n)) + zeta(int(t % n)));
   out[t] = make_double2(rs, rs * rs);
 }
 

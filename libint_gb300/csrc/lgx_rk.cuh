@@ -97,7 +97,7 @@ __device__ __forceinline__ void rk_load(const EriArgs& a, int bpair, int kpair, 
 __device__ __forceinline__ double2 rk_gpq(const EriArgs& a, const PrimPairRec& bp,
                                           const PrimPairRec& kp) {
   if (a.ztab) return __ldg(a.ztab + (size_t)bp.zid * a.nz + kp.zid);
-  const double rs = rsqrt64(bp.zeta + kp.zeta);
+  const double rs = rsqrt(bp.zeta + kp.zeta);
   return make_double2(rs, rs * rs);
 }
 
