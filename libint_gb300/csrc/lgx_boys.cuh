@@ -60,11 +60,12 @@ __device__ __forceinline__ void rk_boys_core(const double* __restrict__ tay, dou
 // The register kernels' FP64 Boys function, F_m(T) pfac, from the fine tables.
 //  T <= 50: c0 + md (c1 + md (c2 + md (c3 + c4 md))), md = T_j - T, the inner
 //   bracket in FP32; every m directly for MMAX <= 2, else the top m, and
-//   e^{-T} = e^{-T_j} e^{md} by the same kind of series.
-//  T > 50: sqrt(pi/T)/2 and the upward recursion without its e^{-T} terms
-//   (MMAX <= 2), or the top m, (2m-1)!! / 2^m times it / T^m.
-//  MMAX > 2: the downward recursion, with e^{-T} = 0 beyond T = 50 (it is below
-//   1.7e-15 of F_6 there), which lanes of both branches run together.
+//   e^{-T} = e^{-T_j} e^{md} by the same kind of series
+//   (MMAX > 2: the downward recursion from there).
+//  T > 50: sqrt(pi/T)/2 and the upward recursion without its e^{-T} terms (below
+//   1.7e-15 of F_6 there).  Not the top m and the downward recursion that the
+//   lanes below 50 run: that gives F_0 the error of F_MMAX, 2.3e-15 instead of
+//   2.4e-16 at MMAX = 6, and zero where F_MMAX underflows.
 // What bounds it: the FP64 pipe (2 lanes per cycle and SM), so everything that
 // only chooses (branch, grid point) or lies below 2^-32 runs in integer and
 // FP32 instructions: per m 3 FP64 operations instead of 5 on the 1/64 grid, and
@@ -76,7 +77,7 @@ __device__ __forceinline__ void rk_boys(const double* __restrict__ fine, double 
   static_assert(MMAX <= kBoysFineM, "fine tables and the asymptotic branch end at m = 6");
   const float Tf = d2f_int(T);
   const bool asym = Tf > float(kBoysTmax);
-  if (asym && MMAX <= 2) {
+  if (asym) {
     const double rs = rsqrt(T);
     const double oo2T = 0.5 * (rs * rs);
     double f = (0.88622692545275801365 * pfac) * rs;
@@ -88,7 +89,7 @@ __device__ __forceinline__ void rk_boys(const double* __restrict__ fine, double 
     }
     return;
   }
-  const int j = asym ? 0 : __float2int_rn(Tf * float(kBoysFineInv));
+  const int j = __float2int_rn(Tf * float(kBoysFineInv));
   const double md = fma(i2d_int(j), 1.0 / kBoysFineInv, -T);
   const float mdf = d2f_int(md);
   const double2* row = reinterpret_cast<const double2*>(fine + boys_fine_off(MMAX) +
@@ -105,24 +106,12 @@ __device__ __forceinline__ void rk_boys(const double* __restrict__ fine, double 
     for (int m = 0; m <= MMAX; ++m) F[m] = series(m) * pfac;
     return;
   }
-  double s, eTp = 0.0;
-  if (asym) {
-    const double rs = rsqrt(T);
-    const double r2 = rs * rs;
-    double c = 0.88622692545275801365;  // (2m-1)!! / 2^m sqrt(pi)/2
-#pragma unroll
-    for (int m = 0; m < MMAX; ++m) c *= 0.5 * (2 * m + 1);
-    s = (c * pfac) * rs;
-#pragma unroll
-    for (int m = 0; m < MMAX; ++m) s *= r2;
-  } else {
-    s = series(0) * pfac;
-    // e^{md} = 1 + md (1 + md (1/2 + md (1/6 + md/24)))
-    double e = fma(md, f2d_int(fmaf(mdf, 1.0f / 24.0f, 1.0f / 6.0f)), 0.5);
-    e = fma(md, e, 1.0);
-    e = fma(md, e, 1.0);
-    eTp = (__ldg(row + 2).x * pfac) * e;
-  }
+  double s = series(0) * pfac;
+  // e^{md} = 1 + md (1 + md (1/2 + md (1/6 + md/24)))
+  double e = fma(md, f2d_int(fmaf(mdf, 1.0f / 24.0f, 1.0f / 6.0f)), 0.5);
+  e = fma(md, e, 1.0);
+  e = fma(md, e, 1.0);
+  const double eTp = (__ldg(row + 2).x * pfac) * e;
   F[MMAX] = s;
   const double twoT = 2.0 * T;
 #pragma unroll
