@@ -101,11 +101,24 @@ __device__ __forceinline__ double2 rk_gpq(const EriArgs& a, const PrimPairRec& b
   return make_double2(rs, rs * rs);
 }
 
+// Whether the prefactor screen drops a primitive quartet: |pfac| below the
+// precision, by the IEEE bit patterns (no FP64 instruction).  SCR: the call may
+// ask for Conservative screening (EriArgs::screening 1), whose estimate has the
+// pairs' non-spherical factors and the number of primitive quartets too.
+template <bool SCR>
+__device__ __forceinline__ bool rk_pfac_dropped(const EriArgs& a, const RkQuartet<double>& q,
+                                                const PrimPairRec& bp, const PrimPairRec& kp,
+                                                double pfac, const PrimScreen& scr) {
+  if (SCR && a.screening == 1)
+    return fabs(pfac) * (fmax(1.0, double(bp.fnonsph) * double(kp.fnonsph)) *
+                         double(q.nbpp * q.nkpp)) < scr.prec;
+  return (__double_as_longlong(pfac) & 0x7fffffffffffffffll) < __double_as_longlong(scr.prec);
+}
+
 // One primitive quartet into acc (FP64).  Returns false when screened out.
 // The ln-screen runs on the FP32 copies with the FP64 values inside the
-// rounding band (ln_kept) and the pfac screen compares the IEEE bit
-// patterns, so neither costs an FP64 instruction outside the band.
-template <class C, bool ATT>
+// rounding band (ln_kept).  SCR: as rk_pfac_dropped.
+template <class C, bool ATT, bool SCR>
 __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<double>& q, int ib,
                                         int ik, const PrimScreen& scr, double* acc) {
   const PrimPairRec& bp = a.pprims[q.bra_pp + ib];
@@ -115,8 +128,7 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<double
   const double2 gpq = rk_gpq(a, bp, kp);
   const double rs = gpq.x, oogpq = gpq.y;
   const double pfac = bp.Kc * kp.Kc * rs;
-  if ((__double_as_longlong(pfac) & 0x7fffffffffffffffll) < __double_as_longlong(scr.prec))
-    return false;
+  if (rk_pfac_dropped<SCR>(a, q, bp, kp, pfac, scr)) return false;
   const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1], PQz = bp.P[2] - kp.P[2];
   const double ez = eta * oogpq, zz = zeta * oogpq;
   const double rho = zeta * ez;
@@ -451,7 +463,7 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
           kept += rk_prim<C, ATT>(a, q, bp, kp, q.bra_pp + ib, q.ket_pp + ik, scr, acc) ? 1 : 0;
         }
       } else {
-        kept += rk_prim<C, ATT>(a, q, ib, ik, scr, acc) ? 1 : 0;
+        kept += rk_prim<C, ATT, MODE == kModeStore>(a, q, ib, ik, scr, acc) ? 1 : 0;
       }
       ib += gb;
       ik += gk;

@@ -40,15 +40,7 @@ __device__ __forceinline__ bool rk_prologue(const EriArgs& a, const RkQuartet<do
   const double2 gpq = rk_gpq(a, bp, kp);
   const double rs = gpq.x, oogpq = gpq.y;
   const double pfac = bp.Kc * kp.Kc * rs;
-  // |pfac|, with the Conservative factor where the list is screened by it
-  if (a.screening == 1) {
-    const double mag = fabs(pfac) * fmax(1.0, double(bp.fnonsph) * double(kp.fnonsph)) *
-                       double(q.nbpp * q.nkpp);
-    if (mag < scr.prec) return false;
-  } else if ((__double_as_longlong(pfac) & 0x7fffffffffffffffll) <
-             __double_as_longlong(scr.prec)) {
-    return false;
-  }
+  if (rk_pfac_dropped<true>(a, q, bp, kp, pfac, scr)) return false;
   const double PQx = bp.P[0] - kp.P[0], PQy = bp.P[1] - kp.P[1], PQz = bp.P[2] - kp.P[2];
   const double ez = eta * oogpq, zz = zeta * oogpq;
   const double T = zeta * ez * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
@@ -379,7 +371,7 @@ __global__ void __launch_bounds__(128, 1) rk_one_kernel(EriArgs a) {
         Cd::template prim<double>(F, geo, w, I);
       }
     } else {
-      kept += rk_prim<Ce, false>(a, q, ib, ik, scr, I) ? 1 : 0;
+      kept += rk_prim<Ce, false, true>(a, q, ib, ik, scr, I) ? 1 : 0;
     }
   }
   const int rows = min(128, nq);
