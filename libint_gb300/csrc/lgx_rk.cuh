@@ -344,6 +344,13 @@ struct RkChunks {
   }
 };
 
+// FP32 accumulators hold the sum of this many primitive quartets of a lane before
+// they go to the run's total: with one lane to a quartet of 4096 the plain FP32 sum
+// loses 1.4e-6 of its value (root mean square; terms below half an ulp of the sum
+// are lost), in runs of 128 1e-7, whatever the number of lanes.  The totals live in
+// local memory, touched only by quartets of more than one run.
+constexpr int kRunF32 = 128;
+
 // Stores one shell set in the caller's order, the elements split between G lanes.
 template <class C, typename T>
 __device__ __forceinline__ void rk_store_set(const EriArgs& a, int flags, long long outoff,
@@ -446,31 +453,47 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
     // without a division per step
     int ib = g / q.nkpp, ik = g - ib * q.nkpp;
     const int gb = G / q.nkpp, gk = G - gb * q.nkpp;
-    for (int p = g; p < nq; p += G) {
-      if constexpr (sizeof(T) == 4) {
-        const bool rec = a.implicit && a.jk32;
-        const PrimF32 bp = rec ? rk_rec32(a.jk32 + brec.x + ib * brec.y)
-                               : rk_pp32(a.pprims[q.bra_pp + ib], q.bsw);
-        const PrimF32 kp = rec ? rk_rec32(a.jk32 + krec.x + ik * krec.y)
-                               : rk_pp32(a.pprims[q.ket_pp + ik], q.ksw);
-        if constexpr (mode_b64(MODE)) {
-          const PrimPairJKds* bds = rec ? a.jkds + brec.x + ib * brec.y : nullptr;
-          const PrimPairJKds* kds = rec ? a.jkds + krec.x + ik * krec.y : nullptr;
-          kept += rk_prim_b64<C, mode_boys(MODE)>(a, q, bp, kp, bds, kds, q.bra_pp + ib, q.ket_pp + ik, scr, acc)
-                      ? 1
-                      : 0;
+    volatile T runs[sizeof(T) == 4 ? C::kNacc : 1];  // FP32: sums of the runs (kRunF32)
+    int end = sizeof(T) == 4 ? min(nq, kRunF32 * G) : nq;
+    for (int p = g;; end = min(nq, end + kRunF32 * G)) {
+      for (; p < end; p += G) {
+        if constexpr (sizeof(T) == 4) {
+          const bool rec = a.implicit && a.jk32;
+          const PrimF32 bp = rec ? rk_rec32(a.jk32 + brec.x + ib * brec.y)
+                                 : rk_pp32(a.pprims[q.bra_pp + ib], q.bsw);
+          const PrimF32 kp = rec ? rk_rec32(a.jk32 + krec.x + ik * krec.y)
+                                 : rk_pp32(a.pprims[q.ket_pp + ik], q.ksw);
+          if constexpr (mode_b64(MODE)) {
+            const PrimPairJKds* bds = rec ? a.jkds + brec.x + ib * brec.y : nullptr;
+            const PrimPairJKds* kds = rec ? a.jkds + krec.x + ik * krec.y : nullptr;
+            kept += rk_prim_b64<C, mode_boys(MODE)>(a, q, bp, kp, bds, kds, q.bra_pp + ib, q.ket_pp + ik, scr, acc)
+                        ? 1
+                        : 0;
+          } else {
+            kept += rk_prim<C, ATT>(a, q, bp, kp, q.bra_pp + ib, q.ket_pp + ik, scr, acc) ? 1 : 0;
+          }
         } else {
-          kept += rk_prim<C, ATT>(a, q, bp, kp, q.bra_pp + ib, q.ket_pp + ik, scr, acc) ? 1 : 0;
+          kept += rk_prim<C, ATT, MODE == kModeStore>(a, q, ib, ik, scr, acc) ? 1 : 0;
         }
-      } else {
-        kept += rk_prim<C, ATT, MODE == kModeStore>(a, q, ib, ik, scr, acc) ? 1 : 0;
+        ib += gb;
+        ik += gk;
+        if (ik >= q.nkpp) {
+          ik -= q.nkpp;
+          ++ib;
+        }
       }
-      ib += gb;
-      ik += gk;
-      if (ik >= q.nkpp) {
-        ik -= q.nkpp;
-        ++ib;
+      if constexpr (sizeof(T) == 4) {
+        if (nq > kRunF32 * G) {
+          const bool one = end <= kRunF32 * G;  // the first run
+#pragma unroll
+          for (int i = 0; i < C::kNacc; ++i) {
+            const T sum = one ? acc[i] : runs[i] + acc[i];
+            runs[i] = sum;
+            acc[i] = end < nq ? T(0) : sum;
+          }
+        }
       }
+      if (end >= nq) break;
     }
     if (G > 1) {
       for (int o = G >> 1; o > 0; o >>= 1) {
