@@ -227,10 +227,11 @@ struct lgx_context {
   cudaGraphExec_t jk_exec = nullptr;
   PassKey jk_key;
   PassRecs jk_recs;
-  // mixed passes: the FP64 and the FP32 class launches run on two streams
+  // mixed passes: the FP64 and the FP32 class launches run on streams of their own
   // forked from and joined back into `stream` (parallel branches of the
   // captured pass), so that FP32 launches use the issue slots that the
-  // FP64-pipe-bound launches leave idle; FP64 launches then hold at most
+  // FP64-pipe-bound launches leave idle; where FP32 is more than a small share of
+  // the pass (enqueue_bins), FP64 launches then hold at most
   // fp64_bps blocks per SM (0: no cap).  `launch_stream` / `scratch` are
   // the stream and the program-kernel slot scratch of the launch being
   // enqueued (the FP32 branch has its own scratch).
@@ -1712,16 +1713,24 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
   // FP32 launches run beside FP64-pipe-bound ones.
   const bool split = ctx->overlap && !ctx->noalloc && nlaunch > 1;
   pr.split = split;
-  // A pass of one precision spreads over both precisions' streams.
-  const bool two = mode32 >= 0;
+  // FP32 launches get streams of their own, and room beside the FP64 ones (the cap
+  // on those, fp64_bps), where they are more than 5% of the pass, an FP64 primitive
+  // quartet counted as eight FP32 ones; else all launches spread over all streams.
+  // Without against with, by share: (H2O)16 cc-pVDZ 29.9 and 27.8 ms (31%), 65.9 and
+  // 64.0 (6%), 73.4 and 75.9 (4%); (H2O)8 cc-pVTZ 84.9 and 82.3 (32%), 132.7 and 132.8
+  // (10%), 151.6 and 157.0 (7%), 172.4 and 180.8 (4%); one water 2.46 and 4.19 (0%).
+  double cost[2] = {0.0, 0.0};
+  for (const Job& j : jobs)
+    cost[j.fp32 ? 1 : 0] +=
+        double(C.bins[j.bi]->total[j.sp]) * C.bins[j.bi]->nq_avg * (j.fp32 ? 1.0 : 8.0);
+  const bool two = cost[1] > 0.05 * (cost[0] + cost[1]);
   const int nhalf = std::max(1, std::min(ctx->branches, lgx_context::kMaxBranches));
-  const int nbr = two ? nhalf : 2 * nhalf;
-  auto stream = [&](bool fp32, int b) {
-    return fp32 ? ctx->s32[b] : (b < nhalf ? ctx->s64[b] : ctx->s32[b - nhalf]);
-  };
+  const int nbr = two ? nhalf : 2 * nhalf;  // per pool
+  auto stream = [&](int b) { return b < nhalf ? ctx->s64[b] : ctx->s32[b - nhalf]; };
+  auto pool = [&](const Job& j) { return two && j.fp32 ? 1 : 0; };
   if (split && ctx->branch_policy == 1) {  // round-robin in bin order
     int nxt[2] = {0, 0};
-    for (auto& j : jobs) j.branch = nxt[j.fp32 ? 1 : 0]++ % nbr;
+    for (auto& j : jobs) j.branch = nxt[pool(j)]++ % nbr + pool(j) * nhalf;
   } else if (split) {  // longest first onto the least-loaded branch
     std::vector<size_t> ord(jobs.size());
     for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
@@ -1730,11 +1739,11 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
     double load[2][2 * lgx_context::kMaxBranches] = {};
     for (size_t i : ord) {
       Job& j = jobs[i];
-      double* l = load[j.fp32 ? 1 : 0];
+      double* l = load[pool(j)];
       int b = 0;
       for (int k = 1; k < nbr; ++k)
         if (l[k] < l[b]) b = k;
-      j.branch = b;
+      j.branch = b + pool(j) * nhalf;
       l[b] += j.est;
     }
     if (ctx->branch_policy == 0)  // issue longest first too (else in bin order)
@@ -1800,10 +1809,10 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
     cudaStream_t st = ctx->stream;
     if (split) {
       const int b = j.branch;
-      st = stream(fp32, b);
+      st = stream(b);
       // program-kernel slot scratch: one region per branch
-      ctx->scratch = (fp32 || b > 0) ? &ctx->gscratch_br[(fp32 ? nhalf : 0) + b] : &ctx->gscratch;
-      if (!fp32 && mode32 >= 0)
+      ctx->scratch = b > 0 ? &ctx->gscratch_br[b] : &ctx->gscratch;
+      if (!fp32 && two)
         a.max_bps = ctx->fp64_bps >= 0 ? ctx->fp64_bps
                                        : (bin.la + bin.lb + bin.lc + bin.ld <= 2 ? 1 : 2);
       if (fp32) a.max_bps = ctx->fp32_bps;
