@@ -1585,8 +1585,10 @@ void bin_args(const BinCache& C, const BinHost& bin, int sp, EriArgs& a) {
 
 // Per-class launch-shape autotuner: for every (class, precision) of the
 // pass without a tuned variant, times the candidate variants (register
-// kernel lanes per quartet; program kernel with interpreted or generated
-// post stage and its staging rows) on a sample from the middle of the bin
+// kernel lanes per quartet, from fill_group's answer up: fewer leave the GPU
+// part empty and run the serial chains that it avoids, which cost the first
+// gradient of (H2O)2 cc-pVDZ 109 ms of tuning; program kernel with interpreted or
+// generated post stage and its staging rows) on a sample from the middle of the bin
 // (its ends hold the shallowest and the deepest contractions), into scratch
 // accumulators, and keeps the fastest if it beats the default by 4%, more
 // than two runs of one shape differ.  Runs once per basis; later passes reuse
@@ -1617,8 +1619,7 @@ lgx_status tune_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int mod
       const Variant d = default_variant(ctx, B, *P, kmode, fp32, true, bin.total[sp], bin.nq_avg);
       cand.push_back(d);
       if (d.kind == 0) {
-        for (int g = 1; g <= 8 && g <= 2 * bin.nq_avg; g *= 2)
-          if (g != d.group) cand.push_back({0, g, 0});
+        for (int g = 2 * d.group; g <= 8 && g <= 2 * bin.nq_avg; g *= 2) cand.push_back({0, g, 0});
       } else {
         for (int kind = 1; kind <= d.kind; ++kind) {
           cand.push_back({kind, 1, 8});
