@@ -325,34 +325,44 @@ int fp32_kernel_mode(const lgx_context* ctx, int mode, int base_mode) {
 
 // ------------------------------------------------------- host constants
 // Boys table: F_m(k/64), m < kBoysCols, from the Maclaurin series (top m)
-// and downward recursion in long double.
-// lo: what the rounding to FP64 leaves.
-std::vector<double> make_boys_table(std::vector<double>& lo) {
-  std::vector<double> t(size_t(kBoysRows) * kBoysCols);
-  lo.resize(t.size());
-  for (int k = 0; k < kBoysRows; ++k) {
-    const long double T = (long double)k * kBoysDT;
-    const int M = kBoysCols - 1;
-    long double term = 1.0L / (2 * M + 1), sum = term;
-    for (int i = 1; i < 4000; ++i) {
-      term *= 2 * T / (2 * M + 2 * i + 1);
-      sum += term;
-      if (term < sum * 1e-22L) break;
+// and downward recursion in long double, made once per process (22 ms of the 26
+// of a context where long double is software arithmetic).
+struct BoysHost {
+  std::vector<double> f, lo;  // values, and what their rounding to FP64 leaves
+  std::vector<double> et;     // e^{-T_k}
+};
+const BoysHost& boys_host() {
+  static const BoysHost table = [] {
+    BoysHost h;
+    h.f.resize(size_t(kBoysRows) * kBoysCols);
+    h.lo.resize(h.f.size());
+    h.et.resize(kBoysRows);
+    for (int k = 0; k < kBoysRows; ++k) {
+      const long double T = (long double)k * kBoysDT;
+      const int M = kBoysCols - 1;
+      long double term = 1.0L / (2 * M + 1), sum = term;
+      for (int i = 1; i < 4000; ++i) {
+        term *= 2 * T / (2 * M + 2 * i + 1);
+        sum += term;
+        if (term < sum * 1e-22L) break;
+      }
+      const long double eT = expl(-T);
+      h.et[k] = double(eT);
+      long double f = eT * sum;
+      auto put = [&](int m) {
+        const size_t i = size_t(k) * kBoysCols + m;
+        h.f[i] = (double)f;
+        h.lo[i] = (double)(f - (long double)h.f[i]);
+      };
+      put(M);
+      for (int m = M - 1; m >= 0; --m) {
+        f = (2 * T * f + eT) / (2 * m + 1);
+        put(m);
+      }
     }
-    const long double eT = expl(-T);
-    long double f = eT * sum;
-    auto put = [&](int m) {
-      const size_t i = size_t(k) * kBoysCols + m;
-      t[i] = (double)f;
-      lo[i] = (double)(f - (long double)t[i]);
-    };
-    put(M);
-    for (int m = M - 1; m >= 0; --m) {
-      f = (2 * T * f + eT) / (2 * m + 1);
-      put(m);
-    }
-  }
-  return t;
+    return h;
+  }();
+  return table;
 }
 
 double fac(int n) {
@@ -2354,8 +2364,7 @@ lgx_status lgx_create(lgx_context** out, int device) {
     }
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     for (auto& e : c->ev_join) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    std::vector<double> boys_lo;
-    const auto boys = make_boys_table(boys_lo);
+    const std::vector<double>&boys = boys_host().f, &boys_lo = boys_host().lo;
     const auto sph = make_sph_table();
     CK(c->boys.ensure(boys.size() * sizeof(double)));
     CK(cudaMemcpy(c->boys.p, boys.data(), boys.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -2381,8 +2390,7 @@ lgx_status lgx_create(lgx_context** out, int device) {
                 boys[size_t(k) * kBoysCols + m + i] / f;
           }
           if (m == 0)
-            tay[size_t(k) * (kBoysMaxM + 1) * kBoysTaylorStride + 7] =
-                double(expl(-(long double)k * kBoysDT));
+            tay[size_t(k) * (kBoysMaxM + 1) * kBoysTaylorStride + 7] = boys_host().et[k];
         }
       CK(c->boys_tay.ensure(tay.size() * sizeof(double)));
       CK(cudaMemcpy(c->boys_tay.p, tay.data(), tay.size() * sizeof(double), cudaMemcpyHostToDevice));
