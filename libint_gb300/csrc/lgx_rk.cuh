@@ -115,7 +115,8 @@ __device__ __forceinline__ bool rk_pfac_dropped(const EriArgs& a, const RkQuarte
   return (__double_as_longlong(pfac) & 0x7fffffffffffffffll) < __double_as_longlong(scr.prec);
 }
 
-// One primitive quartet into acc (FP64).  Returns false when screened out.
+// One primitive quartet into acc (FP64).  Returns false when screened out or when
+// the attenuated operator's integrals vanish: it then enters no VRR and no count.
 // The ln-screen runs on the FP32 copies with the FP64 values inside the
 // rounding band (ln_kept).  SCR: as rk_pfac_dropped.
 template <class C, bool ATT, bool SCR>
@@ -135,7 +136,7 @@ __device__ __forceinline__ bool rk_prim(const EriArgs& a, const RkQuartet<double
   const double T = rho * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz));
   double F[C::kMmax + 1];
   if constexpr (ATT) {
-    if (!rk_boys_att<C::kMmax>(a.boys_fine, a.op, a.omega2, T, rho, pfac, F)) return true;
+    if (!rk_boys_att<C::kMmax>(a.boys_fine, a.op, a.omega2, T, rho, pfac, F)) return false;
   } else {
     rk_boys<C::kMmax>(a.boys_fine, T, pfac, F);
   }
