@@ -1538,21 +1538,22 @@ lgx_status build_bins(lgx_context* ctx, BasisDev& B, double thresh, int mode, do
 // Algorithmic FP operations of the per-primitive-quartet prologue, counted
 // from the equations of libint's primitive data (engine.impl.h:1389-1466),
 // each add, multiply, divide, square root or exponential one operation and
-// an FMA two:
-//   zeta + eta, 1/(zeta + eta), rho = zeta eta / (zeta + eta)        4
-//   P - Q, |P - Q|^2, T = rho |P - Q|^2                              9
-//   pfac = K_ab K_cd / sqrt(zeta + eta)                               3
-//   F_mmax(T) by the order-6 Taylor step, e^{-T}, 2T, and the downward
+// an FMA two.  What depends on a primitive pair alone (P - A, Q - C, 1/2zeta,
+// 1/2eta) or on the exponents (1/(zeta + eta), its square root) is formed once
+// per basis and not counted:
+//   P - Q, |P - Q|^2                                                  8
+//   eta / (zeta + eta), zeta / (zeta + eta), rho, T = rho |P - Q|^2   4
+//   pfac = K_ab K_cd / sqrt(zeta + eta)                               2
+//   F_mmax(T) by a Taylor step, e^{-T}, 2T, and the downward
 //   recursion F_m = (2T F_{m+1} + e^{-T}) / (2m + 1)          14 + 3 mmax
 //   (00|00)^(m) = pfac F_m                                      mmax + 1
-//   W - P, W - Q (eta / (zeta + eta), zeta / (zeta + eta), 6 products) 8
-//   P - A, Q - C                                                      6
-//   1/2zeta, 1/2eta, 1/2(zeta + eta), rho/zeta, rho/eta               5
-// = 50 + 4 mmax.  The mixed scheme's FP32 kernels form rho, P - Q and T a
+//   W - P, W - Q                                                      6
+//   1/2(zeta + eta)                                                   1
+// = 36 + 4 mmax.  The mixed scheme's FP32 kernels form rho, P - Q and T a
 // second time (13), in double-float arithmetic counted as one operation each;
 // they have no FP64 share.
 double prologue_flops(int mmax, bool b64) {
-  return 50.0 + 4.0 * mmax + (b64 ? 13.0 : 0.0);
+  return 36.0 + 4.0 * mmax + (b64 ? 13.0 : 0.0);
 }
 
 // FP operations of the Cartesian -> solid-harmonic transform of one set.
