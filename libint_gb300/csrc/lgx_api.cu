@@ -850,10 +850,15 @@ bool post_gen_ok(const lgx_context* ctx, const BasisDev& B, const ProgDev& P, in
 // the GPU (256 lanes per SM; every lane repeats the stages after the primitive
 // loop), else as many as fill it, up to one lane per primitive quartet.  A
 // lone water in 6-31G has 406 (ss|ss) quartets of up to 1296 primitive
-// quartets: with one lane each its pass took 2.7 ms.
+// quartets: with one lane each its pass took 2.7 ms.  4096 lanes per SM in a pass
+// over a pair subset, which runs on these shapes as they are (tune_bins): its few
+// quartets end on the chains of the deepest (every second shell pair of (H2O)8
+// cc-pVDZ 5.5 ms with 256 and 1.5 with 4096, of (H2O)16 mixed 7.0 and 2.2, of (H2O)8
+// cc-pVTZ 13.0 and 17.0).
 int fill_group(const lgx_context* ctx, long long nwork, double nq_avg) {
+  const long long lanes = ctx->pair_subset.empty() ? 256 : 4096;
   int g = 1;
-  while (g < 32 && g < nq_avg && nwork * g < 256LL * ctx->nsm) g *= 2;
+  while (g < 32 && g < nq_avg && nwork * g < lanes * ctx->nsm) g *= 2;
   return g;
 }
 
@@ -1573,9 +1578,13 @@ double sph_flops(int la, int lb, int lc, int ld, const int* pure) {
   return f;
 }
 
-int tune_key(const BinHost& bin, int deriv, int mode, bool fp32, int op) {
-  return (((class_index(bin.la, bin.lb, bin.lc, bin.ld) * 2 + deriv) * 8 + mode) * 2 +
-          (fp32 ? 1 : 0)) * 4 + op;
+// Tuned shapes hold for bins of one class and precision and, to a factor of four,
+// one size: a mixed pass's FP64 bins are smaller than the FP64 pass's, and on that
+// one's shapes the mixed pass of (H2O)8 cc-pVDZ took 12.5 ms instead of 8.
+int tune_key(const BinHost& bin, int sp, int deriv, int mode, bool fp32, int op) {
+  const int size = (63 - __builtin_clzll((unsigned long long)std::max(1LL, bin.total[sp]))) / 2;
+  return ((((class_index(bin.la, bin.lb, bin.lc, bin.ld) * 2 + deriv) * 8 + mode) * 2 +
+           (fp32 ? 1 : 0)) * 4 + op) * 32 + size;
 }
 
 // Work description of precision space sp of a class bin.
@@ -1602,8 +1611,9 @@ void bin_args(const BinCache& C, const BinHost& bin, int sp, EriArgs& a) {
 // generated post stage and its staging rows) on a sample from the middle of the bin
 // (its ends hold the shallowest and the deepest contractions), into scratch
 // accumulators, and keeps the fastest if it beats the default by 4%, more
-// than two runs of one shape differ.  Runs once per basis; later passes reuse
-// the choice.  The sample is what fills the GPU a few times over, 2^18
+// than two runs of one shape differ.  Runs once per basis and bin size; later passes
+// reuse the choice.  Passes over a pair subset run on the default shapes: a subset
+// is often used for a few passes, which the tuning would outweigh.  The sample is what fills the GPU a few times over, 2^18
 // quartets for the register and 2^14 for the program kernels: with 2^22 and
 // 2^17 the tuning of (H2O)32 cc-pVDZ took five passes' time.
 // mode32: kernel mode of the FP32 precision space (kModeJK, or kModeJKB64
@@ -1611,7 +1621,7 @@ void bin_args(const BinCache& C, const BinHost& bin, int sp, EriArgs& a) {
 // pass runs every quartet in FP64.
 lgx_status tune_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int mode32,
                      EriArgs base) {
-  if (!ctx->tune || ctx->noalloc) return LGX_OK;
+  if (!ctx->tune || ctx->noalloc || !ctx->pair_subset.empty()) return LGX_OK;
   const BinCache& C = ctx->bins;
   const size_t nn = std::max(size_t(B.nbf) * B.nbf, size_t(3 * B.natoms + 64));
   bool scratch = false;
@@ -1624,7 +1634,7 @@ lgx_status tune_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int mod
       if (bin.total[sp] == 0) continue;
       const bool fp32 = (sp == 1) && mode32 >= 0;
       const int kmode = fp32 ? mode32 : mode;
-      const int key = tune_key(bin, deriv, kmode, fp32, ctx->op);
+      const int key = tune_key(bin, sp, deriv, kmode, fp32, ctx->op);
       if (ctx->tuned.count(key)) continue;
       std::vector<Variant> cand;
       const Variant d = default_variant(ctx, B, *P, kmode, fp32, true, bin.total[sp], bin.nq_avg);
@@ -1813,8 +1823,8 @@ lgx_status enqueue_bins(lgx_context* ctx, BasisDev& B, int mode, int deriv, int 
     bin_args(C, bin, sp, a);
     a.prim_count = pr.count ? ctx->primcount.as<unsigned long long>() + 2 * j.bi + sp : nullptr;
     a.counter = counters ? counters + 2 * j.bi + sp : nullptr;
-    const auto tv = ctx->tuned.find(tune_key(bin, deriv, kmode, fp32, ctx->op));
-    const Variant v = tv != ctx->tuned.end()
+    const auto tv = ctx->tuned.find(tune_key(bin, sp, deriv, kmode, fp32, ctx->op));
+    const Variant v = tv != ctx->tuned.end() && ctx->pair_subset.empty()
                           ? tv->second
                           : default_variant(ctx, B, *P, kmode, fp32, true, bin.total[sp],
                                             bin.nq_avg);
