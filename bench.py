@@ -265,9 +265,8 @@ def kernel_roofline(launches, peaks, workload, mode):
     peak = peaks[pipe]
     bound = pipe + "-pipe"
     if r["fp32"] and f64 > 0:
-        # FP32 launch of the mixed scheme with its Boys function in FP64: the
-        # time at peak is the FP64 share at the FP64 peak plus the rest at
-        # the FP32 peak
+        # an FP32 launch with an FP64 share: the time at peak is that share at
+        # the FP64 peak plus the rest at the FP32 peak
         peak = r["flops"] / (f64 / peaks["fp64"] + (r["flops"] - f64) / peaks["fp32"])
         bound = "fp64+fp32 pipes"
     tr = NCU_TRAFFIC.get((workload, mode, name))

@@ -454,8 +454,7 @@ def main():
         d += ["  }", "  return cudaErrorNotSupported;", "}", "",
               "bool rk_%s_available(int la, int lb, int lc, int ld) {" % name,
               "  return la <= 3 && lc <= 3 && la + lb + lc + ld <= %d;" % lmax, "}"]
-    d += ["", "// One quartet over several blocks (derivative order 0 or 1); its accumulators "
-          "per block", "// in doubles, or 0 when there is no kernel.",
+    d += ["", "// One quartet over several blocks (derivative order 0 or 1).",
           "cudaError_t rk_one_launch(int deriv, int la, int lb, int lc, int ld, const EriArgs& a, "
           "int blocks,", "                          cudaStream_t st) {",
           "  switch ((((deriv * 8 + la) * 8 + lb) * 8 + lc) * 8 + ld) {"]

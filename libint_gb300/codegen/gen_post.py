@@ -211,8 +211,8 @@ def main():
     parts.append("}  // namespace lgx")
     _write_if_changed(os.path.join(GEN_DIR, "post_classes.cuh"), "\n".join(parts) + "\n")
 
-    # (precision, mode): FP64, FP32, and FP32 with the FP64 Boys function of
-    # the mixed scheme
+    # (precision, mode): FP64, FP32, and FP32 with the mixed scheme's Boys
+    # function (right to FP32 rounding)
     variants = (("double", "kModeJK"), ("float", "kModeJK"), ("float", "kModeJKB64"))
     items = [(v, c) for c in classes for v in variants]
     items.sort(key=lambda it: -_cost(it[1]))

@@ -35,8 +35,8 @@ RK_MAX_L_STORE = 4
 LMAX = 3
 # (precision, mode, class limit, attenuated operator) variants; the
 # attenuated (erf / erfc) register kernels serve the J/K passes only
-# (the kModeJKB64 / kModeStoreB64 FP32 kernels evaluate the Boys function in
-# FP64: the mixed scheme's FP32 quartets)
+# (kModeJKB64 / kModeStoreB64: the mixed scheme's FP32 quartets, whose Boys
+# function is right to FP32 rounding)
 VARIANTS = [("double", "kModeJK", RK_MAX_L, False), ("float", "kModeJK", RK_MAX_L, False),
             ("float", "kModeJKB64", RK_MAX_L, False),
             ("double", "kModeStore", RK_MAX_L_STORE, False),

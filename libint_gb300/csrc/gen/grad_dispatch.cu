@@ -118,8 +118,7 @@ bool rk_deriv_available(int la, int lb, int lc, int ld) {
   return la <= 3 && lc <= 3 && la + lb + lc + ld <= 3;
 }
 
-// One quartet over several blocks (derivative order 0 or 1); its accumulators per block
-// in doubles, or 0 when there is no kernel.
+// One quartet over several blocks (derivative order 0 or 1).
 cudaError_t rk_one_launch(int deriv, int la, int lb, int lc, int ld, const EriArgs& a, int blocks,
                           cudaStream_t st) {
   switch ((((deriv * 8 + la) * 8 + lb) * 8 + lc) * 8 + ld) {

@@ -71,6 +71,9 @@ __device__ __forceinline__ void rk_boys_core(const double* __restrict__ tay, dou
 // FP32 instructions: per m 3 FP64 operations instead of 5 on the 1/64 grid, and
 // 1 instead of 4 for the grid point.  The tables (0.8 MB for MMAX = 0, 2.5 MB
 // for 2) stay in L2.
+// Error against 128-bit values, root mean square over T <= 50, this and the
+// six-term FP64 series on the 1/64 grid: F_0 6.3e-17 and 6.3e-17 (MMAX = 0),
+// 1.63e-16 and 1.67e-16 (MMAX = 6), F_6 6.6e-17 and 6.7e-17; beyond 50 the same.
 template <int MMAX>
 __device__ __forceinline__ void rk_boys(const double* __restrict__ fine, double T, double pfac,
                                         double* F) {
@@ -197,6 +200,9 @@ __device__ __forceinline__ void rk_boys_b64(const double* __restrict__ tay, dsf 
 //   2.5e-13.
 //  T > 50: r = T^{-1/2} and u = 1/(2T) as hi + lo (boys_asym), F_0 =
 //   sqrt(pi)/2 r, F_{m+1} = (2m+1) u F_m without the e^{-T} terms.
+// Error against 128-bit values, this and rk_boys_b64 (pfac = 1): 5.92e-8 at most
+// and 2.5e-8 root mean square for both, every m <= 6, T up to 300 (the FP32
+// rounding); the product by pfac is the same rounding here, a second one there.
 // The store kernels keep rk_boys_b64: they hand out the integrals one by one,
 // and this evaluation, although as close to the exact values, rounds about
 // one F_m in a thousand (and every product by pfac) the other way.

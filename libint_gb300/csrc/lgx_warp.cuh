@@ -48,7 +48,7 @@ __device__ __forceinline__ double boys_out(double f, double pfac) { return f * p
 __device__ __forceinline__ float boys_out(double f, float pfac) { return d2f_int(f) * pfac; }
 
 // FP64 Boys F_0..F_mmax(T) * pfac into F (runtime mmax); TO = double for the
-// FP64 kernels, float for the FP32 kernels with the Boys function in FP64.
+// FP64 kernels, float for values rounded to FP32.
 template <typename TO>
 __device__ __forceinline__ void boys_to_stage(const double* __restrict__ tab,
                                               const double* __restrict__ inv_odd, double T,
@@ -86,7 +86,7 @@ __device__ __forceinline__ void boys_to_stage(const double* __restrict__ tab,
   }
 }
 
-// The mixed scheme's FP64 Boys function for the program kernels' FP32
+// The mixed scheme's FP64 Boys function for the program store kernels' FP32
 // quartets (runtime mmax <= kBoysMaxM), from the double-float argument
 // T = T.hi + T.lo (ds_boys_arg) and rounded to FP32 with integer operations,
 // times the FP32 prefactor.  T <= 50: F_mmax by the 4-term Taylor series of
