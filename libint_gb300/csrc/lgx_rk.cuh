@@ -351,6 +351,10 @@ struct RkChunks {
 // are lost), in runs of 128 1e-7, whatever the number of lanes.  The totals live in
 // local memory, touched only by quartets of more than one run.
 constexpr int kRunF32 = 128;
+// Classes of up to this many accumulators, (ss|ss) to (ps|ps) and (ss|ds), whose
+// s and p shells are the deeply contracted ones; from (ps|pp) on the totals change
+// no error measured and their code costs the mixed pass of (H2O)20 cc-pVTZ 1%.
+constexpr int kRunSums = 9;
 
 // Stores one shell set in the caller's order, the elements split between G lanes.
 template <class C, typename T>
@@ -454,8 +458,9 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
     // without a division per step
     int ib = g / q.nkpp, ik = g - ib * q.nkpp;
     const int gb = G / q.nkpp, gk = G - gb * q.nkpp;
-    volatile T runs[sizeof(T) == 4 ? C::kNacc : 1];  // FP32: sums of the runs (kRunF32)
-    int end = sizeof(T) == 4 ? min(nq, kRunF32 * G) : nq;
+    constexpr bool kRuns = sizeof(T) == 4 && C::kNacc <= kRunSums;
+    volatile T runs[kRuns ? C::kNacc : 1];  // sums of the runs (kRunF32)
+    int end = kRuns ? min(nq, kRunF32 * G) : nq;
     for (int p = g;; end = min(nq, end + kRunF32 * G)) {
       for (; p < end; p += G) {
         if constexpr (sizeof(T) == 4) {
@@ -483,7 +488,7 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
           ++ib;
         }
       }
-      if constexpr (sizeof(T) == 4) {
+      if constexpr (kRuns) {
         if (nq > kRunF32 * G) {
           const bool one = end <= kRunF32 * G;  // the first run
 #pragma unroll
@@ -494,7 +499,7 @@ __global__ void __launch_bounds__(128, (rk_min_blocks<T, LA, LB, LC, LD, MODE, A
           }
         }
       }
-      if (end >= nq) break;
+      if (!kRuns || end >= nq) break;
     }
     if (G > 1) {
       for (int o = G >> 1; o > 0; o >>= 1) {
