@@ -161,9 +161,12 @@ class Shell:
 
     def _pack(self, arr, k: int):
         """Writes the shell into entry k of an array of LgxShell."""
-        O = self.O  # any indexable sequence of numbers
+        try:
+            x, y, z = self.O.tolist()  # faster than three elements one by one
+        except (AttributeError, ValueError):  # any other indexable sequence of numbers
+            x, y, z = self.O[0], self.O[1], self.O[2]
         _lgx.SHELL_STRUCT.pack_into(arr, k * _lgx.SHELL_STRUCT.size, self.l,
-                                    1 if self.pure else 0, len(self.alpha), 0, O[0], O[1], O[2],
+                                    1 if self.pure else 0, len(self.alpha), 0, x, y, z,
                                     _lgx.address(self.alpha), _lgx.address(self.coeff))
 
     def __repr__(self):
